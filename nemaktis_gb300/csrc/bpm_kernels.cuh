@@ -38,6 +38,19 @@ enum { NDIAG = 12 };
 // F_A = alpha_i = -inf_i/beta_i (forward recurrence d_i = alpha_i d_{i-1} + b_i/beta_i),
 // F_RB = 1/beta_i, F_W = w_i, F_C = -gamma_i (backward recurrence), F_COR = corr_i.
 enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
+// Factor planes of the partitioned x-line solves (k_factor_part): every chunk of M points of a line
+// is factored by itself. F_A = -l_i (forward recurrence d_i = r_i - l_i d_{i-1}, l_i = a_i/beta_{i-1},
+// 0 at the chunk's first point), F_RB = 1/beta_i, F_C = -c_i/beta_i, F_Z = (product of F_C over the
+// points before i) * F_RB, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
+// unknown before the chunk adds to point i before the backward sweep.
+enum { F_Z = F_W, F_E = F_COR };
+// Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
+// first one): h = I_HD d_last + I_HY yf' and g = I_GD d_last + I_GY yf' from the two chunks alone,
+// I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds.
+enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, NIF };
+// Elements per line of the chunk-interleaved factor layout: CH chunks of M points, NFAC planes and
+// the NIF interface coefficients of every chunk.
+__host__ __device__ __forceinline__ size_t part_line_size(int M, int CH) { return (size_t)CH * (M * NFAC + NIF); }
 
 struct GroupParams {
 	double wavelength, k0, dX, dY, dZ;
@@ -1116,6 +1129,152 @@ __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G
 	}
 }
 
+// Pre-factorisation for the partitioned x-line solves (k_solve_xc, k_solve_xw): CH = 32 * W chunks
+// of M points per line, one thread per chunk. Every chunk is factored by itself (LU without pivoting
+// of a principal submatrix of I - mu*R_cc), so there is no scan along the line; what couples the
+// chunks is the 2x2 interface system of neighbouring chunks' border unknowns (I_* above). The line
+// scalar lsc[line][0].x receives the number of Jacobi steps K that the interface system needs to
+// reach rounding: a step multiplies the error by rho, the largest row sum of the interface couplings,
+// about the M-th power of the decay from point to point (K = 0 for 8-point chunks at the usual mesh
+// spacings in FP32, 1 in FP64). Lines with rho^KMAX above rounding (spacings far below a
+// wavelength) and lines of one chunk are factored as a single chunk by one thread and flagged -1;
+// their solve is sequential.
+// Bound: HBM and the latency of the reciprocals (M in a row). The scans over Moebius and affine maps
+// of k_factor_chunked it replaces here took 107 us per launch on the 256x256, 16-wavelength FP32 case
+// and 47 us on a 64x64 FP64 one.
+constexpr int PART_KMAX = 24;
+template <typename S>
+__global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>* __restrict__ diag,
+		cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
+	const int N = G.N, nlines = G.Ny, n = G.Nx - 1;
+	const int CH = blockDim.x, t = threadIdx.x;
+	const int line = blockIdx.x * blockDim.y + threadIdx.y;
+	const int gc = blockIdx.y, g = gc / 2, c = gc % 2;
+	const bool active = line < nlines && G.Nx > 3;
+	const int nchk = (n + M - 1) / M;
+	const cx<S>* Dg = diag + (size_t)g * NDIAG * N + (size_t)(c * 3) * N + (size_t)line * G.Nx;
+	cx<S>* Fc = fac + (size_t)gc * NFAC * plane + (size_t)line * part_line_size(M, CH);
+	cx<S>* If = Fc + (size_t)M * NFAC * CH;
+	cx<double>* ls = lsc + ((size_t)gc * nlines + line) * 2;
+	const cx<S> one = mk<S>(1, 0), zero = mk<S>(0, 0);
+	// factors of the points [i0, i0 + m) as one chunk; returns through vf, vl, wf, wl, rbl the
+	// border responses to the unknowns before (v) and after (w) the chunk and the last 1/beta
+	cx<S> vf = zero, vl = zero, wf = zero, wl = zero, rbl = zero;
+	auto chunk = [&](int i0, int m) {
+		cx<S> rb = zero, cprev = zero, ev = zero, cpz = one;
+		vf = zero;
+		for(int k = 0; k < m; k++) {
+			const int i = i0 + k;
+			const cx<S> a = -Dg[i], b = one - Dg[(size_t)N + i], cs = -Dg[2 * (size_t)N + i];
+			cx<S> al = zero;  // -l
+			if(k == 0) ev = -a;
+			else {
+				al = -(a * rb);
+				ev = al * ev;
+			}
+			const cx<S> beta = k == 0 ? b : cfma(al, cprev, b);
+			rb = crecip(beta);
+			cprev = cs;
+			const cx<S> cc = -(rb * cs), z = cpz * rb, e = rb * ev;
+			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
+			F[F_A * CH] = al;
+			F[F_RB * CH] = rb;
+			F[F_Z * CH] = z;
+			F[F_C * CH] = cc;
+			F[F_E * CH] = e;
+			vf = cfma(z, ev, vf);
+			cpz = cpz * cc;
+			vl = e;
+			wl = cc;
+		}
+		wf = cpz;
+		rbl = rb;
+	};
+	const int i0 = t * M;
+	const bool own = active && i0 < n;
+	if(own) chunk(i0, min(M, n - i0));
+	// the next chunk's responses (cyclic), through shared memory
+	__shared__ cx<S> shv[256], shw[256];
+	__shared__ S shr[8];
+	const int tid = threadIdx.y * CH + t;
+	shv[tid] = vf;
+	shw[tid] = wf;
+	__syncthreads();
+	S rho = 0;
+	if(own) {
+		const int nx = threadIdx.y * CH + (t == nchk - 1 ? 0 : t + 1);
+		const cx<S> vfn = shv[nx], wfn = shw[nx];
+		const cx<S> m = crecip(cfnma(wl, vfn, one));
+		const cx<S> mw = m * wl, mv = m * vfn;
+		const cx<S> ph = m * vl, pg = mv * vl, qh = mw * wfn, qg = m * wfn;
+		If[I_HD * CH + t] = m * rbl;
+		If[I_HY * CH + t] = mw;
+		If[I_GD * CH + t] = mv * rbl;
+		If[I_GY * CH + t] = m;
+		If[I_PH * CH + t] = ph;
+		If[I_PG * CH + t] = pg;
+		If[I_QH * CH + t] = qh;
+		If[I_QG * CH + t] = qg;
+		rho = fmax(l1abs(ph) + l1abs(qh), l1abs(pg) + l1abs(qg));
+		if(!(rho < (S)1)) rho = 1;  // NaN too
+	}
+	// largest rho of the line
+#pragma unroll
+	for(int o = 16; o > 0; o >>= 1) rho = fmax(rho, __shfl_xor_sync(0xffffffffu, rho, o));
+	if(CH > 32) {
+		if(t % 32 == 0) shr[tid / 32] = rho;
+		__syncthreads();
+		for(int w = 0; w < CH / 32; w++) rho = fmax(rho, shr[w]);
+	}
+	if(!active || t != 0) return;
+	const S lt = sizeof(S) == sizeof(float) ? (S)-18.7 : (S)-39.5;  // ln of 2^-27, 2^-57
+	int K = 0;
+	if(nchk < 2 || !(rho < (S)1)) K = -1;
+	else if(rho > (S)0 && log(rho) > lt) {
+		const S k = ceil(lt / log(rho)) - 1;
+		K = k <= (S)PART_KMAX ? (int)k : -1;
+	}
+	ls[0] = mk((double)K, 0.0);
+	if(K >= 0) return;
+	// the whole line as one chunk that is its own neighbour: h = vl h + wl g + 1/beta_last d_last,
+	// g = vf h + wf g + yf. (The block's other threads have written their chunks' factors: those of
+	// this line before the barriers above.)
+	chunk(0, n);
+	const cx<S> p = one - vl, q = one - wf;
+	const cx<S> m = crecip(cfnma(wl, vf, p * q));
+	If[I_HD * CH] = m * q * rbl;
+	If[I_HY * CH] = m * wl;
+	If[I_GD * CH] = m * vf * rbl;
+	If[I_GY * CH] = m * p;
+}
+
+// The sequential solve of a line flagged -1 by k_factor_part, by one thread: buf holds the right-hand
+// sides of KS slots (element i at (i / M) * (M + 1) + i % M) and receives the solution.
+template <typename R, int M, int KS>
+__device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n) {
+	const cx<R>* If = Fc + (size_t)M * NFAC * CH;
+#pragma unroll 1
+	for(int j = 0; j < KS; j++) {
+		cx<R>* b = buf + j * PITCH;
+		cx<R> d = mk<R>(0, 0), yf = mk<R>(0, 0);
+		for(int i = 0; i < n; i++) {
+			const cx<R>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
+			cx<R>& v = b[(i / M) * (M + 1) + i % M];
+			d = cfma(F[F_A * CH], d, v);
+			v = d;
+			yf = cfma(F[F_Z * CH], d, yf);
+		}
+		const cx<R> h = cfma(If[I_HY * CH], yf, If[I_HD * CH] * d);
+		cx<R> x = cfma(If[I_GY * CH], yf, If[I_GD * CH] * d);
+		for(int i = n - 1; i >= 0; i--) {
+			const cx<R>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
+			cx<R>& v = b[(i / M) * (M + 1) + i % M];
+			x = cfma(F[F_C * CH], x, cfma(F[F_E * CH], h, F[F_RB * CH] * v));
+			v = x;
+		}
+	}
+}
+
 // One combine of the chunk maps of a line whose chunks sit on the 32 lanes of a warp (chunk =
 // lane; lanes past the line carry identity maps). Inputs per lane: forward map (P, d0[j]),
 // sum terms (S0[j], S1), backward terms (Cp, G0[j], G1). Outputs per lane: din = the forward
@@ -1176,8 +1335,14 @@ __device__ __forceinline__ void line_combine(cx<R> P, const cx<R>* d0, const cx<
 // x-line solve fused with its right-hand side (KIND: explicit y half-step or x Woodbury term):
 // a warp per line (4 lines per block) for KS slots of one wavelength. The right-hand sides are
 // computed with coalesced loads into the warp's shared buffer in the lane-chunk layout (lane l
-// holds points [l M, l M + M)), one pass builds the chunk maps, line_combine joins them by
-// shuffles, and a last pass finishes the line, which goes back out coalesced.
+// holds points [l M, l M + M)); every lane sweeps forward through its chunk, the lanes join through
+// the border unknowns of neighbouring chunks (k_factor_part), and a backward sweep with those known
+// finishes the line, which goes back out coalesced.
+// Bound: L1 wavefronts (73 %) and load latency (issue active 50 %). Partitioning in place of forward,
+// sum and backward maps joined by shuffle scans: 20 instead of 28 multiply-adds per point and slot, 5
+// instead of 7 factor loads, and no scans (5 shuffle steps each over 3 quantities). 256x256, 16
+// wavelengths, 13 q, FP32: Woodbury solves 552 -> 490 us, explicit step 499 -> 476 us; the same mesh
+// with 3 wavelengths in FP64 (bound by the FP64 pipe) 1351 -> 962 and 1540 -> 1162 us.
 template <typename R, int M, int KIND, int KS, bool TOUT = false>
 // Resident blocks per SM requested from the compiler: 8 (64 registers) for the instances
 // whose chunk values fit, measured faster on GB300; the larger instances keep their registers.
@@ -1208,11 +1373,10 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 	const int PITCH = 32 * (M + 1);
 	cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw) + (size_t)warp * KS * PITCH;
 	if(iy < Ny) {  // always true unless TOUT (whose block writes together after a barrier)
-	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * 32 * M * NFAC;
-	const cx<double>* ls = lsc + (((size_t)g * 2 + c) * Ny + iy) * 2;
-	const cx<double> r0 = ls[0], rden = ls[1];
+	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
+	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
 	const int i0 = lane * M;
-	const cx<R> one = mk<R>(1, 0), zero = mk<R>(0, 0);
+	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s0 * 2 * N;
 	// right-hand sides, coalesced (point e = lane + 32 t), into the lane-chunk layout of buf; the
@@ -1228,62 +1392,78 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 		}
 	}
 	__syncwarp();
-	// Local pass over the lane's chunk: the right-hand sides b (written back over the stencil
-	// values in buf), the zero-carry forward values d0 and the three maps that finish the line
-	// after one combine:
-	//   forward   D_out = P * D_in + d0_end                  (P = product of a)
-	//   sum       sum_i w_i d_i = S0 + S1 * D_in
-	//   backward  x_start = Cp * X_in + G0 + G1 * D_in       (Cp = product of c)
-	// P, S1, G1 and Cp do not depend on the slot. The chunk values live in shared memory, not
-	// in registers.
-	cx<R> d0[KS], S0[KS], G0[KS];
-	cx<R> P = one, S1 = zero, G1 = zero, Cp = one;
+	if(K >= 0) {
+		// forward sweep of the lane's chunk (written back over the right-hand sides) and its first
+		// unknown yf with nothing outside the chunk
+		cx<R> d[KS], yf[KS];
+		cx<R>* vb = buf + lane * (M + 1);
 #pragma unroll
-	for(int j = 0; j < KS; j++) { d0[j] = zero; S0[j] = zero; G0[j] = zero; }
-	cx<R>* vb = buf + lane * (M + 1);
+		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
-	for(int k = 0; k < M; k++) {
-		if(i0 + k < n_unk) {
-			const cx<R> a = Fc[(k * NFAC + F_A) * 32 + lane], rb = Fc[(k * NFAC + F_RB) * 32 + lane];
-			const cx<R> w = Fc[(k * NFAC + F_W) * 32 + lane], cc = Fc[(k * NFAC + F_C) * 32 + lane];
-			P = a * P;
-			S1 = cfma(w, P, S1);
-			G1 = cfma(Cp, P, G1);
+		for(int k = 0; k < M; k++) {
+			if(i0 + k < n_unk) {
+				const cx<R> z = Fc[(k * NFAC + F_Z) * 32 + lane];
+				if(k == 0) {
 #pragma unroll
-			for(int j = 0; j < KS; j++) {
-				const cx<R> b = vb[j * PITCH + k] * rb;
-				vb[j * PITCH + k] = b;
-				d0[j] = cfma(a, d0[j], b);
-				S0[j] = cfma(w, d0[j], S0[j]);
-				G0[j] = cfma(Cp, d0[j], G0[j]);
-			}
-			Cp = Cp * cc;
-		}
-	}
-	// One combine across the chunks (lanes): forward carries, Sherman-Morrison factor,
-	// backward carries.
-	cx<R> din[KS], xin[KS], fr[KS];
-	line_combine<R, KS>(P, d0, S0, S1, G0, G1, Cp, r0, rden, lane, din, xin, fr);
-	// Finish: forward values from the carry, then the backward sweep with the correction.
+					for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
+				}
+				else {
+					const cx<R> a = Fc[(k * NFAC + F_A) * 32 + lane];
 #pragma unroll
-	for(int k = 0; k < M; k++) {
-		if(i0 + k < n_unk) {
-			const cx<R> a = Fc[(k * NFAC + F_A) * 32 + lane];
-#pragma unroll
-			for(int j = 0; j < KS; j++) { din[j] = cfma(a, din[j], vb[j * PITCH + k]); vb[j * PITCH + k] = din[j]; }
-		}
-	}
-#pragma unroll
-	for(int k = M - 1; k >= 0; k--) {
-		if(i0 + k < n_unk) {
-			const cx<R> cc = Fc[(k * NFAC + F_C) * 32 + lane], cr = Fc[(k * NFAC + F_COR) * 32 + lane];
-#pragma unroll
-			for(int j = 0; j < KS; j++) {
-				xin[j] = cfma(cc, xin[j], vb[j * PITCH + k]);
-				vb[j * PITCH + k] = cfnma(fr[j], cr, xin[j]);
+					for(int j = 0; j < KS; j++) {
+						d[j] = cfma(a, d[j], vb[j * PITCH + k]);
+						vb[j * PITCH + k] = d[j];
+						yf[j] = cfma(z, d[j], yf[j]);
+					}
+				}
 			}
 		}
+		// interface unknowns: h (the chunk's last) and g (the next chunk's first)
+		const int last = (n_unk - 1) / M;  // last chunk
+		const int left = lane == 0 ? last : lane - 1, right = lane == last ? 0 : (lane + 1) & 31;
+		const cx<R>* If = Fc + (size_t)M * NFAC * 32 + lane;
+		cx<R> h[KS], x[KS];
+		{
+			const cx<R> hd = If[I_HD * 32], hy = If[I_HY * 32], gd = If[I_GD * 32], gy = If[I_GY * 32];
+#pragma unroll
+			for(int j = 0; j < KS; j++) {
+				const cx<R> yn = shfl_idx_c(yf[j], right);
+				h[j] = cfma(hy, yn, hd * d[j]);
+				x[j] = cfma(gy, yn, gd * d[j]);
+			}
+		}
+		if(K > 0) {
+			const cx<R> ph = If[I_PH * 32], pg = If[I_PG * 32], qh = If[I_QH * 32], qg = If[I_QG * 32];
+			cx<R> bh[KS], bg[KS];
+#pragma unroll
+			for(int j = 0; j < KS; j++) { bh[j] = h[j]; bg[j] = x[j]; }
+#pragma unroll 1
+			for(int k = 0; k < K; k++) {
+#pragma unroll
+				for(int j = 0; j < KS; j++) {
+					const cx<R> hl = shfl_idx_c(h[j], left), gr = shfl_idx_c(x[j], right);
+					h[j] = cfma(qh, gr, cfma(ph, hl, bh[j]));
+					x[j] = cfma(qg, gr, cfma(pg, hl, bg[j]));
+				}
+			}
+		}
+#pragma unroll
+		for(int j = 0; j < KS; j++) h[j] = shfl_idx_c(h[j], left);
+		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
+#pragma unroll
+		for(int k = M - 1; k >= 0; k--) {
+			if(i0 + k < n_unk) {
+				const cx<R> rb = Fc[(k * NFAC + F_RB) * 32 + lane], cc = Fc[(k * NFAC + F_C) * 32 + lane];
+				const cx<R> ee = Fc[(k * NFAC + F_E) * 32 + lane];
+#pragma unroll
+				for(int j = 0; j < KS; j++) {
+					x[j] = cfma(cc, x[j], cfma(ee, h[j], rb * vb[j * PITCH + k]));
+					vb[j * PITCH + k] = x[j];
+				}
+			}
+		}
 	}
+	else if(lane == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, 32, n_unk);
 	// the explicit-step solves never accumulate; the accumulating ones load the accumulator inputs
 	// of several points before storing any (their latency would otherwise be paid point by point)
 	const bool acc = KIND != ST_EXPL_Y && acc_out;
@@ -1739,8 +1919,8 @@ __global__ void __launch_bounds__(128) k_solve_yq(Geom G, int nch, const cx<R>* 
 }
 
 // x-line solve for long lines: one block of W warps per line, 32*W chunks of M points (the
-// chunk-interleaved factor layout with 32*W chunks). Within a warp the chunk maps combine with
-// shuffles as in k_solve_xc, across the warps of the line through shared memory.
+// partitioned layout with 32*W chunks), solved as in k_solve_xc; neighbouring chunks in different
+// warps exchange their border unknowns through shared memory (2 + K barriers a line).
 // acc_in2 (may be null): a second accumulator input, acc_out = (acc_in + acc_in2) + x. TOUT: the
 // results go out transposed with the components exchanged ((c, iy, e) -> (1 - c, e, iy) of an
 // Ny x Nx plane), as in k_solve_xc.
@@ -1762,17 +1942,13 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 	const int ci = warp * 32 + lane;
 	const int PITCH = CH * (M + 1);
 	cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);  // [KS][CH][M+1]
-	cx<R>* sA = buf + KS * PITCH;                     // [KS][W]
-	cx<R>* sB = sA + KS * W;
-	cx<R>* sD = sB + KS * W;
-	cx<R>* sP = sD + KS * W;
-	cx<R>* sX = sP + KS * W;                          // [KS][2]: d at the last unknown, fr
-	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * CH * M * NFAC;
-	const cx<double>* ls = lsc + (((size_t)g * 2 + c) * Ny + iy) * 2;
-	const cx<double> r0 = ls[0], rden = ls[1];
+	cx<R>* sG = buf + KS * PITCH;                     // [2][KS][W]: g (first yf) of the warps' first chunks
+	cx<R>* sH = sG + 2 * KS * W;                      // [2][KS][W + 1]: h of the warps' last chunks, then of the line's
+	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, CH);
+	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
 	const int i0 = ci * M;
-	const int last = n_unk - 1;
-	const cx<R> one = mk<R>(1, 0), zero = mk<R>(0, 0);
+	const int last = (n_unk - 1) / M;  // last chunk
+	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s0 * 2 * N;
 	for(int e = threadIdx.x; e < n_unk; e += blockDim.x) {
@@ -1782,139 +1958,101 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
 	}
 	__syncthreads();
-	cx<R> v[KS][M];
-	cx<R> A[KS], B[KS];
+	if(K >= 0) {
+		// forward sweep of the thread's chunk and its first unknown with nothing outside the chunk
+		cx<R> d[KS], yf[KS];
+		cx<R>* vb = buf + ci * (M + 1);
 #pragma unroll
-	for(int j = 0; j < KS; j++) { A[j] = one; B[j] = zero; }
+		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
-	for(int k = 0; k < M; k++) {
-		bool ok = i0 + k < n_unk;
-		cx<R> a = zero, rb = zero;
-		if(ok) { a = Fc[(k * NFAC + F_A) * CH + ci]; rb = Fc[(k * NFAC + F_RB) * CH + ci]; }
+		for(int k = 0; k < M; k++) {
+			if(i0 + k < n_unk) {
+				const cx<R> z = Fc[(k * NFAC + F_Z) * CH + ci];
+				if(k == 0) {
 #pragma unroll
-		for(int j = 0; j < KS; j++) {
-			v[j][k] = zero;
-			if(ok) {
-				cx<R> b = buf[j * PITCH + ci * (M + 1) + k] * rb;
-				v[j][k] = b;
-				B[j] = cfma(a, B[j], b);
-				A[j] = a * A[j];
+					for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
+				}
+				else {
+					const cx<R> a = Fc[(k * NFAC + F_A) * CH + ci];
+#pragma unroll
+					for(int j = 0; j < KS; j++) {
+						d[j] = cfma(a, d[j], vb[j * PITCH + k]);
+						vb[j * PITCH + k] = d[j];
+						yf[j] = cfma(z, d[j], yf[j]);
+					}
+				}
 			}
 		}
-	}
-	// forward: inclusive scan within the warp, then the warps' totals in order
+		// interface unknowns as in k_solve_xc; neighbours in other warps through shared memory
+		const cx<R>* If = Fc + (size_t)M * NFAC * CH + ci;
+		const bool edge_r = lane == 31 || ci == last;   // the next chunk is in another warp (or the first)
+		const int wr = ci == last ? 0 : (warp + 1) % W;
+		auto next = [&](cx<R> v, const cx<R>* s, int j) {
+			const cx<R> n = shfl_down_c(v, 1);
+			return edge_r ? s[j * W + wr] : n;
+		};
+		if(lane == 0) {
 #pragma unroll
-	for(int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-		for(int j = 0; j < KS; j++) {
-			cx<R> Ap = shfl_up_c(A[j], o), Bp = shfl_up_c(B[j], o);
-			if(lane >= o) { B[j] = A[j] * Bp + B[j]; A[j] = A[j] * Ap; }
+			for(int j = 0; j < KS; j++) sG[j * W + warp] = yf[j];
 		}
-	}
-	if(lane == 31) {
-#pragma unroll
-		for(int j = 0; j < KS; j++) { sA[j * W + warp] = A[j]; sB[j * W + warp] = B[j]; }
-	}
-	__syncthreads();
-	if(threadIdx.x < KS) {
-		int j = threadIdx.x;
-		cx<R> D = zero;
-		for(int ww = 0; ww < W; ww++) {
-			sD[j * W + ww] = D;
-			D = sA[j * W + ww] * D + sB[j * W + ww];
-		}
-	}
-	__syncthreads();
-	cx<R> d[KS], acc[KS];
-#pragma unroll
-	for(int j = 0; j < KS; j++) {
-		cx<R> Ae = shfl_up_c(A[j], 1), Be = shfl_up_c(B[j], 1);
-		if(lane == 0) { Ae = one; Be = zero; }
-		d[j] = Ae * sD[j * W + warp] + Be;
-		acc[j] = zero;
-	}
-#pragma unroll
-	for(int k = 0; k < M; k++) {
-		if(i0 + k < n_unk) {
-			cx<R> a = Fc[(k * NFAC + F_A) * CH + ci], w = Fc[(k * NFAC + F_W) * CH + ci];
+		__syncthreads();
+		cx<R> h[KS], x[KS], hl[KS];
+		{
+			const cx<R> hd = If[I_HD * CH], hy = If[I_HY * CH], gd = If[I_GD * CH], gy = If[I_GY * CH];
 #pragma unroll
 			for(int j = 0; j < KS; j++) {
-				d[j] = cfma(a, d[j], v[j][k]);
-				v[j][k] = d[j];
-				acc[j] = cfma(w, d[j], acc[j]);
-			}
-			if(i0 + k == last) {
-#pragma unroll
-				for(int j = 0; j < KS; j++) sX[2 * j] = d[j];
+				const cx<R> yn = next(yf[j], sG, j);
+				h[j] = cfma(hy, yn, hd * d[j]);
+				x[j] = cfma(gy, yn, gd * d[j]);
 			}
 		}
-	}
+		cx<R> bh[KS], bg[KS];
 #pragma unroll
-	for(int j = 0; j < KS; j++) {
-#pragma unroll
-		for(int o = 16; o > 0; o >>= 1) acc[j] += shfl_xor_c(acc[j], o);
-		if(lane == 0) sP[j * W + warp] = acc[j];
-	}
-	__syncthreads();
-	if(threadIdx.x < KS) {
-		int j = threadIdx.x;
-		cx<R> tot = zero;
-		for(int ww = 0; ww < W; ww++) tot += sP[j * W + ww];
-		sX[2 * j + 1] = cvt<R>((cvt<double>(tot) - r0 * cvt<double>(sX[2 * j])) * rden);
-	}
-	// backward: chunk maps, inclusive scan from the line's end
-#pragma unroll
-	for(int j = 0; j < KS; j++) { A[j] = one; B[j] = zero; }
-#pragma unroll
-	for(int k = M - 1; k >= 0; k--) {
-		if(i0 + k < n_unk) {
-			cx<R> cc = Fc[(k * NFAC + F_C) * CH + ci];
-#pragma unroll
-			for(int j = 0; j < KS; j++) { B[j] = cfma(cc, B[j], v[j][k]); A[j] = cc * A[j]; }
-		}
-	}
-#pragma unroll
-	for(int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-		for(int j = 0; j < KS; j++) {
-			cx<R> An = shfl_down_c(A[j], o), Bn = shfl_down_c(B[j], o);
-			if(lane + o < 32) { B[j] = A[j] * Bn + B[j]; A[j] = A[j] * An; }
-		}
-	}
-	__syncthreads();  // sD of the forward pass has been read
-	if(lane == 0) {
-#pragma unroll
-		for(int j = 0; j < KS; j++) { sA[j * W + warp] = A[j]; sB[j * W + warp] = B[j]; }
-	}
-	__syncthreads();
-	if(threadIdx.x < KS) {
-		int j = threadIdx.x;
-		cx<R> D = zero;
-		for(int ww = W - 1; ww >= 0; ww--) {
-			sD[j * W + ww] = D;
-			D = sA[j * W + ww] * D + sB[j * W + ww];
-		}
-	}
-	__syncthreads();
-	cx<R> fr[KS];
-#pragma unroll
-	for(int j = 0; j < KS; j++) {
-		fr[j] = sX[2 * j + 1];
-		cx<R> An = shfl_down_c(A[j], 1), Bn = shfl_down_c(B[j], 1);
-		if(lane == 31) { An = one; Bn = zero; }
-		d[j] = An * sD[j * W + warp] + Bn;
-	}
-#pragma unroll
-	for(int k = M - 1; k >= 0; k--) {
-		if(i0 + k < n_unk) {
-			cx<R> cc = Fc[(k * NFAC + F_C) * CH + ci], cr = Fc[(k * NFAC + F_COR) * CH + ci];
+		for(int j = 0; j < KS; j++) { bh[j] = h[j]; bg[j] = x[j]; }
+#pragma unroll 1
+		for(int it = 0;; it++) {
+			// two buffers in turn: the one written here was last read two barriers ago
+			cx<R>* H = sH + (it & 1) * KS * (W + 1);
+			cx<R>* Gn = sG + ((it + 1) & 1) * KS * W;
 #pragma unroll
 			for(int j = 0; j < KS; j++) {
-				d[j] = cfma(cc, d[j], v[j][k]);
-				buf[j * PITCH + ci * (M + 1) + k] = cfnma(fr[j], cr, d[j]);
+				if(lane == 31) H[j * (W + 1) + warp] = h[j];
+				if(ci == last) H[j * (W + 1) + W] = h[j];
+			}
+			if(lane == 0) {
+#pragma unroll
+				for(int j = 0; j < KS; j++) Gn[j * W + warp] = x[j];
+			}
+			__syncthreads();
+#pragma unroll
+			for(int j = 0; j < KS; j++) {
+				const cx<R> up = shfl_up_c(h[j], 1);
+				hl[j] = lane > 0 ? up : H[j * (W + 1) + (warp > 0 ? warp - 1 : W)];
+			}
+			if(it >= K) break;
+			const cx<R> ph = If[I_PH * CH], pg = If[I_PG * CH], qh = If[I_QH * CH], qg = If[I_QG * CH];
+#pragma unroll
+			for(int j = 0; j < KS; j++) {
+				const cx<R> gr = next(x[j], Gn, j);
+				h[j] = cfma(qh, gr, cfma(ph, hl[j], bh[j]));
+				x[j] = cfma(qg, gr, cfma(pg, hl[j], bg[j]));
+			}
+		}
+		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
+#pragma unroll
+		for(int k = M - 1; k >= 0; k--) {
+			if(i0 + k < n_unk) {
+				const cx<R> rb = Fc[(k * NFAC + F_RB) * CH + ci], cc = Fc[(k * NFAC + F_C) * CH + ci];
+				const cx<R> ee = Fc[(k * NFAC + F_E) * CH + ci];
+#pragma unroll
+				for(int j = 0; j < KS; j++) {
+					x[j] = cfma(cc, x[j], cfma(ee, hl[j], rb * vb[j * PITCH + k]));
+					vb[j * PITCH + k] = x[j];
+				}
 			}
 		}
 	}
+	else if(threadIdx.x == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, CH, n_unk);
 	__syncthreads();
 	// write-out: the accumulator inputs of several points are loaded before any store
 	constexpr int U = 4;

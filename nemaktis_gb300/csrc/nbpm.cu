@@ -987,6 +987,16 @@ struct Plan : PlanBase {
 		return ps;
 	}
 
+	// Factorisation for the partitioned x-line solves: one block of 4 lines, or of one line of wpl warps.
+	void rec_factor_part(const char* name, double bytes, const Geom& Gm, int ng, int M, int wpl, const cx<R>* dg, cx<R>* fac,
+			size_t plane, cx<double>* lsc) {
+		const int LT = wpl > 1 ? 1 : 4;
+		launch(name, bytes, [&] {
+			k_factor_part<R><<<dim3((unsigned)((Gm.Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32 * wpl, LT), 0, cs>>>(
+				Gm, M, dg, fac, plane, lsc);
+		});
+	}
+
 	// Slabs [ps.iz, iz_end) of a pass. Setup of slab iz (eps plane iz+1, coefficients,
 	// factorisations) runs on streamB and overlaps the right-hand-side work of slab iz-1 on
 	// the main stream; both streams are joined again before returning.
@@ -1028,7 +1038,9 @@ struct Plan : PlanBase {
 			const double fb = (double)N * ng * 2 * (3 * sc + NFAC * sc + 4 * sc);
 			// y factorisation: 8 chunk warps per 32 columns, 16 when the grid leaves SMs idle
 			const int LT = 4, WF = ((Nx + 31) / 32) * 2 * ng < nsm && Ny - 1 >= 256 ? 16 : 8;
-			launch("factor_x", fb, [&] {
+			if(scf.Mx && !scf.xs)
+				rec_factor_part("factor_x", fb, Gm, ng, scf.Mx, scf.WPLx, ps.Dg, fx, scf.plane_x, lx);
+			else launch("factor_x", fb, [&] {
 				k_factor_chunked<R, 0><<<dim3((unsigned)((Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
 					Gm, ng, scf.Mx, 32 * scf.WPLx, 1, ps.Dg, fx, scf.plane_x, lx);
 			});
@@ -1041,10 +1053,7 @@ struct Plan : PlanBase {
 					k_coef_t<R><<<dim3((unsigned)((Nx + 31) / 32), (unsigned)((Ny + 31) / 32), (unsigned)(ng * NCT)), dim3(32, 8), 0,
 						cs>>>(Gm, C, ps.Dg, CT, W->diagT.as<cx<R>>());
 				});
-				launch("factor_y", fb, [&] {
-					k_factor_chunked<R, 0><<<dim3((unsigned)((Nx + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
-						Gt, ng, scf.Mxt, 32 * scf.WPLt, 1, W->diagT.as<cx<R>>(), fy, scf.plane_y, ly);
-				});
+				rec_factor_part("factor_y", fb, Gt, ng, scf.Mxt, scf.WPLt, W->diagT.as<cx<R>>(), fy, scf.plane_y, ly);
 			}
 			else {
 				size_t smem = (size_t)WF * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>);

@@ -91,15 +91,23 @@ struct SolveShape {
 	int cap() const { return fp32 || relax ? 32 : 16; }
 };
 
+// Elements per factor plane of `lines` partitioned lines (part_line_size in bpm_kernels.cuh: 5 factors
+// per point and 8 interface coefficients per chunk).
+inline size_t part_plane(int lines, int M, int wpl) {
+	return ((size_t)lines * 32 * wpl * (5 * M + 8) + 4) / 5;
+}
+
 inline size_t plane_x_of(const SolveCfg& c, const SolveShape& s) {
 	size_t N = (size_t)s.Nx * s.Ny;
-	return c.Mx ? std::max(N, (size_t)s.Ny * 32 * c.WPLx * c.Mx) : N;
+	if(!c.Mx) return N;
+	// k_solve_xs: chunk-interleaved factors; k_solve_xc / k_solve_xw: with the interface coefficients
+	return std::max(N, c.xs ? (size_t)s.Ny * 32 * c.Mx : part_plane(s.Ny, c.Mx, c.WPLx));
 }
 
 inline void finalize(SolveCfg& c, const SolveShape& s) {
 	c.plane_x = plane_x_of(c, s);
-	// transposed-frame y factors: the chunk-interleaved x layout of Nx lines of 32 * Mxt points
-	c.plane_y = std::max((size_t)s.Nx * s.Ny, c.Mxt ? (size_t)s.Nx * 32 * c.WPLt * c.Mxt : (size_t)0);
+	// transposed-frame y factors: the partitioned x layout of Nx lines
+	c.plane_y = std::max((size_t)s.Nx * s.Ny, c.Mxt ? part_plane(s.Nx, c.Mxt, c.WPLt) : (size_t)0);
 }
 
 inline bool xs_fits(int ks, int M, const SolveShape& s) { return (size_t)4 * ks * 32 * (M + 1) * s.csize() <= 100 * 1024; }
