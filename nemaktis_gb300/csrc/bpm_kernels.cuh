@@ -6,9 +6,10 @@
 //                                            order as the (Nl,Nq,4,Ny,Nx) user buffer
 //   eps ring  Q[2][group][NQ][iy][ix]        FP64 per-voxel derived permittivity, planes iz
 //                                            and iz+1 of every wavelength group
-//   coef      C[group][p/32][NCOEF][p%32]    cx<R>: 3 phase-operator entries and the 40
-//                                            entries of mu*R (DX, DY, DXDY stencils x 4 blocks),
-//                                            p = iy*Nx + ix, in tiles of 32 points (cidx)
+//   coef      C[group][p/32][..][p%32]      one point's operators in CSET scalars R: the stencils of
+//                                            mu*R (DX, DY, DXDY x 4 blocks) without their parts that
+//                                            are zero, and 3 complex phase-operator entries, in
+//                                            tiles of 32 points (coef_v, coef_u, coef_ph)
 //   factors   X/Y[group][comp][NFAC][p]      cx<R>: pre-factored periodic line solves
 // A "group" is one wavelength: every (q, pol) slot of the group shares eps, R, the phase
 // operator and the line-solve factorisations.
@@ -22,18 +23,57 @@ namespace nbpm {
 
 // Per-voxel derived permittivity components (PermittivityTensorField.cpp:3-99).
 enum { Q_XXTR = 0, Q_YYTR, Q_XYTR, Q_XXS, Q_YYS, Q_XYS, Q_VX, Q_VY, Q_IZZ, NQ };
-// Coefficient planes: phase operator (xx, yy, xy), then mu*R stencils.
-enum { C_PH = 0, C_DX = 3, C_DY = 15, C_DXDY = 27, NCOEF = 43 };
-// A group's coefficient set is stored in tiles of 32 points with every plane of a tile together:
-// entry (plane k, point p) at ((p / 32) * NCOEF + k) * 32 + p % 32, NCOEF * ceil(N / 32) * 32
-// entries per group. The planes a kernel reads at one point are then fixed multiples of 32
-// entries apart (compile-time offsets from one address), and 32 consecutive points of a plane
-// starting at a multiple of 32 are one contiguous segment.
-__host__ __device__ __forceinline__ size_t coef_set_size(int N) { return (size_t)NCOEF * (((size_t)N + 31) & ~(size_t)31); }
-__host__ __device__ __forceinline__ size_t cidx(int k, int p) { return ((size_t)(p >> 5) * NCOEF + k) * 32 + (p & 31); }
-// FP64 copies of the diagonal-block stencils used by the line factorisations:
-// index dir*6 + comp*3 + k (dir 0 = DX, 1 = DY; comp 0 = block 00, 1 = block 11).
-enum { NDIAG = 12 };
+// Coefficient set of one point. The entries of mu*R are i*(dZ/2)*(real), but for the walk-off terms: first
+// derivatives, which only the outer entries of DX blocks 0, 1, 2 and of DY blocks 1, 2, 3 have. So an
+// entry is one real number (its imaginary part) except those twelve, 52 numbers in place of 80, and a
+// tap with a real number costs two multiply-adds in place of four. They are kept as 12 vectors of
+// four, which a thread loads at once, and two pairs (m, c, p: the entries of the previous point, the
+// point itself and the next one; the index is the block):
+//   V_DD + b   DXDY block b: (px,py), (mx,py), (px,my), (mx,my)
+//   V_DX + i   DX block i = 0, 1, 2: m (complex), p (complex)       V_DX + 3: m3, p3, c3, c2    U_DX: c0, c1
+//   V_DY + i   DY block 3 - i = 3, 2, 1: m (complex), p (complex)   V_DY + 3: m0, p0, c0, c1    U_DY: c3, c2
+// The order of the DY blocks makes the transposed frame's DX and DY plain copies of DY and DX. Sets are
+// stored in tiles of 32 points with all of a tile together, so that what a kernel reads at one point is
+// at fixed distances from one address and 32 consecutive points of a vector are one contiguous segment.
+enum { V_DD = 0, V_DX = 4, V_DY = 8, NV = 12, U_DX = 0, U_DY = 1, NU = 2 };
+enum { CSET = 4 * NV + 2 * NU + 6 };  // scalars per point: vectors, pairs, 3 complex phase entries
+template <typename S>
+struct alignas(4 * sizeof(S)) v4 {
+	S x, y, z, w;
+};
+// complex values per group
+__host__ __device__ __forceinline__ size_t coef_set_size(int N) { return (size_t)(CSET / 2) * (((size_t)N + 31) & ~(size_t)31); }
+template <typename C>
+__device__ __forceinline__ C* coef_tile(C* coef, int p) { return coef + (size_t)(p >> 5) * (CSET / 2 * 32); }
+template <typename S>
+__device__ __forceinline__ const v4<S>& coef_v(const cx<S>* coef, int k, int p) {
+	return reinterpret_cast<const v4<S>*>(coef_tile(coef, p))[k * 32 + (p & 31)];
+}
+template <typename S>
+__device__ __forceinline__ v4<S>& coef_v(cx<S>* coef, int k, int p) {
+	return reinterpret_cast<v4<S>*>(coef_tile(coef, p))[k * 32 + (p & 31)];
+}
+// pairs and phase entries follow the vectors
+template <typename C>
+__device__ __forceinline__ C& coef_u(C* coef, int u, int p) { return coef_tile(coef, p)[2 * NV * 32 + u * 32 + (p & 31)]; }
+template <typename C>
+__device__ __forceinline__ C& coef_ph(C* coef, int i, int p) { return coef_tile(coef, p)[(2 * NV + NU) * 32 + i * 32 + (p & 31)]; }
+// Entries m, c, p of the diagonal block of component comp along direction DIRN (0: DX, 1: DY) at point p.
+template <int DIRN, typename S>
+__device__ __forceinline__ void coef_diag(const cx<S>* coef, int comp, int p, cx<S>& m, cx<S>& c, cx<S>& n) {
+	if(comp == DIRN) {  // DX block 0, DY block 3: with walk-off
+		const v4<S> v = coef_v(coef, DIRN == 0 ? V_DX : V_DY, p);
+		m = mk(v.x, v.y);
+		n = mk(v.z, v.w);
+		c = mk((S)0, coef_u(coef, DIRN == 0 ? U_DX : U_DY, p).x);
+	}
+	else {
+		const v4<S> v = coef_v(coef, DIRN == 0 ? V_DX + 3 : V_DY + 3, p);
+		m = mk((S)0, v.x);
+		n = mk((S)0, v.y);
+		c = mk((S)0, v.z);
+	}
+}
 // Line-solve factor planes.
 // F_A = alpha_i = -inf_i/beta_i (forward recurrence d_i = alpha_i d_{i-1} + b_i/beta_i),
 // F_RB = 1/beta_i, F_W = w_i, F_C = -gamma_i (backward recurrence), F_COR = corr_i.
@@ -360,7 +400,7 @@ __device__ __forceinline__ void phase_op(const T* A, const T* B, int N, int p, T
 template <typename S>
 __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		const double* __restrict__ wts, int iz, Geom G, const GroupParams* __restrict__ gps,
-		cx<S>* __restrict__ coef, cx<S>* __restrict__ diag) {
+		cx<S>* __restrict__ coef) {
 	typedef S T;  // arithmetic type of the eps planes, the phase operator and the R coefficients
 	int p = blockIdx.x * blockDim.x + threadIdx.x;
 	int g = blockIdx.y;
@@ -371,7 +411,6 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 	const T* A = QA + (size_t)g * NQ * N;
 	const T* B = QB + (size_t)g * NQ * N;
 	cx<S>* C = coef + (size_t)g * coef_set_size(N);
-	cx<S>* Dg = diag + (size_t)g * NDIAG * N + p;
 
 	// Phase operator.
 	{
@@ -379,9 +418,9 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		if(wts) { size_t vi = (size_t)iz * N + p; w0 = (T)wts[2 * vi]; w1 = (T)wts[2 * vi + 1]; }
 		cx<T> oxx, oyy, oxy;
 		phase_op<T>(A, B, N, p, w0, w1, gp, oxx, oyy, oxy);
-		C[cidx(C_PH + 0, p)] = oxx;
-		C[cidx(C_PH + 1, p)] = oyy;
-		C[cidx(C_PH + 2, p)] = oxy;
+		coef_ph(C, 0, p) = oxx;
+		coef_ph(C, 1, p) = oyy;
+		coef_ph(C, 2, p) = oxy;
 	}
 
 	CoefCtx<T> X;
@@ -397,7 +436,7 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 	int pyq = (iy == Ny - 1) ? 1 : iy + 1, myq = (iy == 0) ? Ny - 2 : iy - 1;
 	int pxs = (ix == Nx - 2) ? 0 : ix + 1, mxs = (ix == 0) ? Nx - 2 : ix - 1;
 	int pys = (iy == Ny - 2) ? 0 : iy + 1, mys = (iy == 0) ? Ny - 2 : iy - 1;
-	cx<T> r[4];
+	cx<T> r[3][4];
 	const cx<T> z = mk<T>(0, 0);
 
 	// DX: rows ix < Nx-1 when Nx > 3; k = 0 mx, 1 centre, 2 px.
@@ -413,17 +452,19 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		const T c1[3] = {cm, c0, cp};
 		const T L[3] = {(T)1 / (dX * dX), (T)-2 / (dX * dX), (T)1 / (dX * dX)};
 		const T dd[3] = {(T)-0.5 / dX, 0, (T)0.5 / dX};
+#pragma unroll
 		for(int k = 0; k < 3; k++) {
 			if(ok) {
 				int cxp = cols[k];
 				T kxx = X.avg(Q_XXTR, cxp, iy), kxy = X.avg(Q_XYTR, cxp, iy);
-				X.entry(c1[k] * kxx, c1[k] * kxy, (T)0, L[k], cxp, iy, dd[k], 0, r);
+				X.entry(c1[k] * kxx, c1[k] * kxy, (T)0, L[k], cxp, iy, dd[k], 0, r[k]);
 			}
-			else r[0] = r[1] = r[2] = r[3] = z;
-			for(int b = 0; b < 4; b++) C[cidx(C_DX + 3 * b + k, p)] = cvt<S>(r[b]);
-			Dg[(size_t)(0 * 6 + 0 * 3 + k) * N] = r[0];
-			Dg[(size_t)(0 * 6 + 1 * 3 + k) * N] = r[3];
+			else r[k][0] = r[k][1] = r[k][2] = r[k][3] = z;
 		}
+#pragma unroll
+		for(int b = 0; b < 3; b++) coef_v(C, V_DX + b, p) = v4<S>{r[0][b].x, r[0][b].y, r[2][b].x, r[2][b].y};
+		coef_v(C, V_DX + 3, p) = v4<S>{r[0][3].y, r[2][3].y, r[1][3].y, r[1][2].y};
+		coef_u(C, U_DX, p) = mk(r[1][0].y, r[1][1].y);
 	}
 	// DY: rows iy < Ny-1 when Ny > 3; k = 0 my, 1 centre, 2 py.
 	{
@@ -438,17 +479,19 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		const T c1[3] = {cm, c0, cp};
 		const T L[3] = {(T)1 / (dY * dY), (T)-2 / (dY * dY), (T)1 / (dY * dY)};
 		const T dd[3] = {(T)-0.5 / dY, 0, (T)0.5 / dY};
+#pragma unroll
 		for(int k = 0; k < 3; k++) {
 			if(ok) {
 				int cyp = rows[k];
 				T kyy = X.avg(Q_YYTR, ix, cyp), kxy = X.avg(Q_XYTR, ix, cyp);
-				X.entry(L[k], (T)0, c1[k] * kxy, c1[k] * kyy, ix, cyp, dd[k], 1, r);
+				X.entry(L[k], (T)0, c1[k] * kxy, c1[k] * kyy, ix, cyp, dd[k], 1, r[k]);
 			}
-			else r[0] = r[1] = r[2] = r[3] = z;
-			for(int b = 0; b < 4; b++) C[cidx(C_DY + 3 * b + k, p)] = cvt<S>(r[b]);
-			Dg[(size_t)(1 * 6 + 0 * 3 + k) * N] = r[0];
-			Dg[(size_t)(1 * 6 + 1 * 3 + k) * N] = r[3];
+			else r[k][0] = r[k][1] = r[k][2] = r[k][3] = z;
 		}
+#pragma unroll
+		for(int b = 3; b > 0; b--) coef_v(C, V_DY + 3 - b, p) = v4<S>{r[0][b].x, r[0][b].y, r[2][b].x, r[2][b].y};
+		coef_v(C, V_DY + 3, p) = v4<S>{r[0][0].y, r[2][0].y, r[1][0].y, r[1][1].y};
+		coef_u(C, U_DY, p) = mk(r[1][3].y, r[1][2].y);
 	}
 	// DXDY: rows ix < Nx-1, iy < Ny-1 when Nx > 3 and Ny > 3; k = pxpy, mxpy, pxmy, mxmy.
 	{
@@ -464,16 +507,21 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		const T d10[4] = {a2, -a2, -c2, c2};
 		const int cxs[4] = {pxs, mxs, pxs, mxs};
 		const int cys[4] = {pys, pys, mys, mys};
+		S dq[4][4];
+#pragma unroll
 		for(int k = 0; k < 4; k++) {
 			if(ok) {
 				T kxx = X.avg(Q_XXTR, cxs[k], cys[k]), kyy = X.avg(Q_YYTR, cxs[k], cys[k]);
 				T kxy = X.avg(Q_XYTR, cxs[k], cys[k]);
 				X.entry(d01[k] * kxy, g0[k] + d01[k] * kyy, g0[k] + d10[k] * kxx, d10[k] * kxy,
-					cxs[k], cys[k], (T)0, 0, r);
+					cxs[k], cys[k], (T)0, 0, r[0]);
 			}
-			else r[0] = r[1] = r[2] = r[3] = z;
-			for(int b = 0; b < 4; b++) C[cidx(C_DXDY + 4 * b + k, p)] = cvt<S>(r[b]);
+			else r[0][0] = r[0][1] = r[0][2] = r[0][3] = z;
+#pragma unroll
+			for(int b = 0; b < 4; b++) dq[b][k] = r[0][b].y;
 		}
+#pragma unroll
+		for(int b = 0; b < 4; b++) coef_v(C, V_DD + b, p) = v4<S>{dq[b][0], dq[b][1], dq[b][2], dq[b][3]};
 	}
 }
 
@@ -484,202 +532,122 @@ template <typename R>
 struct Stencil {
 	const cx<R>* C;
 	int N, Nx, Ny;
-	__device__ __forceinline__ cx<R> c(int plane, int p) const { return C[cidx(plane, p)]; }
-	// DX block b at row (x, y): columns mx, x, px with period Nx-1.
-	__device__ __forceinline__ cx<R> dx(int b, int x, int y, const cx<R>* s) const {
-		int p = x + Nx * y;
-		int mx = x == 0 ? Nx - 2 : x - 1, px = x == Nx - 2 ? 0 : x + 1;
-		int base = C_DX + 3 * b;
-		return c(base, p) * s[mx + Nx * y] + c(base + 1, p) * s[p] + c(base + 2, p) * s[px + Nx * y];
-	}
-	__device__ __forceinline__ cx<R> dy(int b, int x, int y, const cx<R>* s) const {
-		int p = x + Nx * y;
-		int my = y == 0 ? Ny - 2 : y - 1, py = y == Ny - 2 ? 0 : y + 1;
-		int base = C_DY + 3 * b;
-		return c(base, p) * s[x + Nx * my] + c(base + 1, p) * s[p] + c(base + 2, p) * s[x + Nx * py];
-	}
-	__device__ __forceinline__ cx<R> dxdy(int b, int x, int y, const cx<R>* s) const {
-		int p = x + Nx * y;
-		int mx = x == 0 ? Nx - 2 : x - 1, px = x == Nx - 2 ? 0 : x + 1;
-		int my = y == 0 ? Ny - 2 : y - 1, py = y == Ny - 2 ? 0 : y + 1;
-		int base = C_DXDY + 4 * b;
-		return c(base, p) * s[px + Nx * py] + c(base + 1, p) * s[mx + Nx * py] +
-			c(base + 2, p) * s[px + Nx * my] + c(base + 3, p) * s[mx + Nx * my];
-	}
-	// Multi-slot forms: the same stencil coefficients applied to KS fields (slot planes
-	// ss apart), accumulated into out[].
-	template <int KS>
-	__device__ __forceinline__ void dx_m(int b, int x, int y, const cx<R>* s, size_t ss, cx<R>* out) const {
-		int p = x + Nx * y;
-		int mx = x == 0 ? Nx - 2 : x - 1, px = x == Nx - 2 ? 0 : x + 1;
-		int base = C_DX + 3 * b;
-		cx<R> c0 = c(base, p), c1 = c(base + 1, p), c2 = c(base + 2, p);
-#pragma unroll
-		for(int j = 0; j < KS; j++) {
-			const cx<R>* f = s + j * ss;
-			out[j] = cfma(c2, f[px + Nx * y], cfma(c1, f[p], cfma(c0, f[mx + Nx * y], out[j])));
-		}
-	}
-	template <int KS>
-	__device__ __forceinline__ void dy_m(int b, int x, int y, const cx<R>* s, size_t ss, cx<R>* out) const {
-		int p = x + Nx * y;
-		int my = y == 0 ? Ny - 2 : y - 1, py = y == Ny - 2 ? 0 : y + 1;
-		int base = C_DY + 3 * b;
-		cx<R> c0 = c(base, p), c1 = c(base + 1, p), c2 = c(base + 2, p);
-#pragma unroll
-		for(int j = 0; j < KS; j++) {
-			const cx<R>* f = s + j * ss;
-			out[j] = cfma(c2, f[x + Nx * py], cfma(c1, f[p], cfma(c0, f[x + Nx * my], out[j])));
-		}
-	}
-	template <int KS>
-	__device__ __forceinline__ void dxdy_m(int b, int x, int y, const cx<R>* s, size_t ss, cx<R>* out) const {
-		int p = x + Nx * y;
-		int mx = x == 0 ? Nx - 2 : x - 1, px = x == Nx - 2 ? 0 : x + 1;
-		int my = y == 0 ? Ny - 2 : y - 1, py = y == Ny - 2 ? 0 : y + 1;
-		int base = C_DXDY + 4 * b;
-		cx<R> c0 = c(base, p), c1 = c(base + 1, p), c2 = c(base + 2, p), c3 = c(base + 3, p);
-#pragma unroll
-		for(int j = 0; j < KS; j++) {
-			const cx<R>* f = s + j * ss;
-			out[j] = cfma(c3, f[mx + Nx * my], cfma(c2, f[px + Nx * my], cfma(c1, f[mx + Nx * py], cfma(c0, f[px + Nx * py], out[j]))));
-		}
-	}
 };
+
+// out += (i*a) f for a real entry a of an imaginary coefficient.
+template <typename R>
+__device__ __forceinline__ cx<R> ifma(R a, cx<R> f, cx<R> out) { return mk<R>(fmar(-a, f.y, out.x), fmar(a, f.x, out.y)); }
 
 // Step kinds of the composite stencil kernel (ParaxialPrimaryEvolutionOperator.cpp:153-207
 // with the duplicate-row/column fix-ups of BlockSparseMatrix.cpp folded in analytically).
 enum { ST_EXPL_Y = 0, ST_EXPL_X = 1, ST_WOOD_X = 2, ST_WOOD_Y = 3 };
 
-// One component of a composite stencil step at point (ix, iy). EXPL kinds return
-// f + mu*R f (explicit half-step), WOOD kinds return mu*R_offdiag t (Woodbury right-hand side).
-// (xx, yy) are the indices with the duplicate column / row folded onto column / row 0, which
-// is where the reference's fix-ups copy their values from.
-template <typename R, int KIND>
-__device__ __forceinline__ cx<R> composite(const Stencil<R>& st, int comp, int ix, int iy,
-		const cx<R>* f0, const cx<R>* f1) {
-	const int Nx = st.Nx, Ny = st.Ny;
-	const int xx = ix == Nx - 1 ? 0 : ix, yy = iy == Ny - 1 ? 0 : iy;
-	const bool ax = Nx > 3, ay = Ny > 3;
-	cx<R> T = mk<R>(0, 0);
-	if(KIND == ST_EXPL_Y) {
-		if(comp == 0) {
-			if(ay) T = st.dy(0, ix, yy, f0) + st.dy(1, ix, yy, f1);
-			return f0[ix + Nx * iy] + T;
-		}
-		if(ay) {
-			if(ax) T = st.dy(3, xx, yy, f1) + st.dxdy(3, xx, yy, f1) + st.dy(2, xx, yy, f0) + st.dxdy(2, xx, yy, f0);
-			else T = st.dy(3, ix, yy, f1) + st.dy(2, ix, yy, f0);
-		}
-		return f1[ix + Nx * iy] + T;
-	}
-	if(KIND == ST_EXPL_X) {
-		if(comp == 0) {
-			if(ax) {
-				if(ay) T = st.dx(0, xx, yy, f0) + st.dxdy(0, xx, yy, f0) + st.dx(1, xx, yy, f1) + st.dxdy(1, xx, yy, f1);
-				else T = st.dx(0, xx, iy, f0) + st.dx(1, xx, iy, f1);
-			}
-			return f0[ix + Nx * iy] + T;
-		}
-		if(ax) T = st.dx(3, xx, iy, f1) + st.dx(2, xx, iy, f0);
-		return f1[ix + Nx * iy] + T;
-	}
-	if(KIND == ST_WOOD_X) {
-		if(comp == 0) {
-			if(ax) {
-				if(ay) T = st.dx(1, xx, yy, f1) + st.dxdy(1, xx, yy, f1) + st.dxdy(0, xx, yy, f0);
-				else T = st.dx(1, xx, iy, f1);
-			}
-			return T;
-		}
-		if(ax) T = st.dx(2, xx, iy, f0);
-		return T;
-	}
-	// ST_WOOD_Y
-	if(comp == 0) {
-		if(ay) T = st.dy(1, ix, yy, f1);
-		return T;
-	}
-	if(ay) {
-		if(ax) T = st.dy(2, xx, yy, f0) + st.dxdy(2, xx, yy, f0) + st.dxdy(3, xx, yy, f1);
-		else T = st.dy(2, ix, yy, f0);
-	}
-	return T;
+// A value at a byte offset from a field plane: the plane's address is the same for the whole block and
+// the offset 32 bits wide (a plane pair of one slot is below 4 GB), so that an access costs one add at most.
+template <typename R>
+__device__ __forceinline__ cx<R> at_off(const cx<R>* f, unsigned o) {
+	return *reinterpret_cast<const cx<R>*>(reinterpret_cast<const char*>(f) + o);
 }
 
-// composite() for KS consecutive slots at once (f0: comp-0 plane of the first slot, slot
-// planes 2N apart, comp-1 plane at +N); every stencil coefficient is loaded once.
+// One component of a composite stencil step at point (ix, iy) for KS consecutive slots at once (f0: comp-0
+// plane of the first slot, slot planes 2N apart, comp-1 plane at +N); every stencil coefficient is loaded
+// once. EXPL kinds return f + mu*R f (explicit half-step), WOOD kinds mu*R_offdiag t (Woodbury
+// right-hand side). (xx, yy) are the indices with the duplicate column / row folded onto column / row
+// 0, which is where the reference's fix-ups copy their values from. The neighbours wrap with period
+// N - 1; directions of three points or fewer have no derivatives.
 template <typename R, int KIND, int KS>
 __device__ __forceinline__ void composite_m(const Stencil<R>& st, int comp, int ix, int iy, const cx<R>* f0,
 		cx<R>* out) {
 	const int Nx = st.Nx, Ny = st.Ny;
-	const size_t N = st.N, ss = 2 * N;
-	const cx<R>* f1 = f0 + N;
-	const int xx = ix == Nx - 1 ? 0 : ix, yy = iy == Ny - 1 ? 0 : iy;
+	const size_t N = st.N;
+	constexpr unsigned SZ = sizeof(cx<R>);
 	const bool ax = Nx > 3, ay = Ny > 3;
-	const int p = ix + Nx * iy;
+	const cx<R>* C = st.C;
+	constexpr bool XDIR = KIND == ST_EXPL_X || KIND == ST_WOOD_X;  // derivatives along x (else along y)
+	constexpr bool EXPL = KIND == ST_EXPL_X || KIND == ST_EXPL_Y;
+	// the component that also takes the mixed derivatives: 0 along x, 1 along y
+	const bool mixed = XDIR ? comp == 0 : comp == 1;
 #pragma unroll
 	for(int j = 0; j < KS; j++) out[j] = mk<R>(0, 0);
-	if(KIND == ST_EXPL_Y) {
-		if(comp == 0) {
-			if(ay) { st.template dy_m<KS>(0, ix, yy, f0, ss, out); st.template dy_m<KS>(1, ix, yy, f1, ss, out); }
+	const unsigned own = ((unsigned)iy * (unsigned)Nx + (unsigned)ix) * SZ;
+	if(XDIR ? ax : ay) {
+		const bool both = mixed && ax && ay;
+		// the row point of the taps: folded along both directions where the mixed derivatives take part
+		// (or would, without the other direction: only along this one)
+		const int xx = (XDIR || both) && ix == Nx - 1 ? 0 : ix;
+		const int yy = (!XDIR || both) && iy == Ny - 1 ? 0 : iy;
+		const int p = xx + Nx * yy;
+		const unsigned o = (unsigned)p * SZ;
+		const unsigned om = XDIR ? (xx == 0 ? o + (unsigned)(Nx - 2) * SZ : o - SZ)
+			: (yy == 0 ? o + (unsigned)(Ny - 2) * (unsigned)Nx * SZ : o - (unsigned)Nx * SZ);
+		const unsigned op = XDIR ? (xx == Nx - 2 ? o - (unsigned)(Nx - 2) * SZ : o + SZ)
+			: (yy == Ny - 2 ? o - (unsigned)(Ny - 2) * (unsigned)Nx * SZ : o + (unsigned)Nx * SZ);
+		// entries (m, c, p) applied to component plane f of every slot
+		auto taps = [&](v4<R> v, R c, const cx<R>* f) {
 #pragma unroll
-			for(int j = 0; j < KS; j++) out[j] += f0[j * ss + p];
-			return;
-		}
-		if(ay) {
-			if(ax) {
-				st.template dy_m<KS>(3, xx, yy, f1, ss, out); st.template dxdy_m<KS>(3, xx, yy, f1, ss, out);
-				st.template dy_m<KS>(2, xx, yy, f0, ss, out); st.template dxdy_m<KS>(2, xx, yy, f0, ss, out);
+			for(int j = 0; j < KS; j++) {
+				const cx<R>* fj = f + 2 * N * j;
+				out[j] = cfma(mk(v.z, v.w), at_off(fj, op), ifma(c, at_off(fj, o), cfma(mk(v.x, v.y), at_off(fj, om), out[j])));
 			}
-			else { st.template dy_m<KS>(3, ix, yy, f1, ss, out); st.template dy_m<KS>(2, ix, yy, f0, ss, out); }
-		}
+		};
+		auto itaps = [&](R m, R c, R n, const cx<R>* f) {  // without walk-off
 #pragma unroll
-		for(int j = 0; j < KS; j++) out[j] += f1[j * ss + p];
-		return;
-	}
-	if(KIND == ST_EXPL_X) {
-		if(comp == 0) {
-			if(ax) {
-				if(ay) {
-					st.template dx_m<KS>(0, xx, yy, f0, ss, out); st.template dxdy_m<KS>(0, xx, yy, f0, ss, out);
-					st.template dx_m<KS>(1, xx, yy, f1, ss, out); st.template dxdy_m<KS>(1, xx, yy, f1, ss, out);
+			for(int j = 0; j < KS; j++) {
+				const cx<R>* fj = f + 2 * N * j;
+				out[j] = ifma(n, at_off(fj, op), ifma(c, at_off(fj, o), ifma(m, at_off(fj, om), out[j])));
+			}
+		};
+		const cx<R>* f1 = f0 + N;
+		// DX and DY blocks by their place in the set: D + 3 holds (m, p, c) of the block without walk-off and a
+		// centre, U the centres of the two other blocks
+		constexpr int D = XDIR ? V_DX : V_DY, U = XDIR ? U_DX : U_DY;
+		if(XDIR) {
+			if(comp == 0) {
+				const cx<R> u = coef_u(C, U, p);
+				if(EXPL) taps(coef_v(C, D, p), u.x, f0);
+				taps(coef_v(C, D + 1, p), u.y, f1);
+			}
+			else {
+				const v4<R> w = coef_v(C, D + 3, p);
+				if(EXPL) itaps(w.x, w.z, w.y, f1);
+				taps(coef_v(C, D + 2, p), w.w, f0);
+			}
+		}
+		else {
+			if(comp == 0) {
+				const v4<R> w = coef_v(C, D + 3, p);
+				if(EXPL) itaps(w.x, w.z, w.y, f0);
+				taps(coef_v(C, D + 2, p), w.w, f1);
+			}
+			else {
+				const cx<R> u = coef_u(C, U, p);
+				if(EXPL) taps(coef_v(C, D, p), u.x, f1);
+				taps(coef_v(C, D + 1, p), u.y, f0);
+			}
+		}
+		if(both) {
+			// corners: the offsets along the other direction, relative to the tap along this one
+			const unsigned dm = XDIR ? (yy == 0 ? (unsigned)(Ny - 2) * (unsigned)Nx * SZ : 0u - (unsigned)Nx * SZ)
+				: (xx == 0 ? (unsigned)(Nx - 2) * SZ : 0u - SZ);
+			const unsigned dp = XDIR ? (yy == Ny - 2 ? 0u - (unsigned)(Ny - 2) * (unsigned)Nx * SZ : (unsigned)Nx * SZ)
+				: (xx == Nx - 2 ? 0u - (unsigned)(Nx - 2) * SZ : SZ);
+			const unsigned opp = op + dp, omm = om + dm, opm = XDIR ? op + dm : om + dp, omp = XDIR ? om + dp : op + dm;
+			// opm: (px, my), omp: (mx, py)
+			auto corners = [&](v4<R> v, const cx<R>* f) {
+#pragma unroll
+				for(int j = 0; j < KS; j++) {
+					const cx<R>* fj = f + 2 * N * j;
+					out[j] = ifma(v.w, at_off(fj, omm), ifma(v.z, at_off(fj, opm), ifma(v.y, at_off(fj, omp), ifma(v.x, at_off(fj, opp), out[j]))));
 				}
-				else { st.template dx_m<KS>(0, xx, iy, f0, ss, out); st.template dx_m<KS>(1, xx, iy, f1, ss, out); }
-			}
+			};
+			if(XDIR) { corners(coef_v(C, V_DD + 0, p), f0); corners(coef_v(C, V_DD + 1, p), f1); }
+			else { corners(coef_v(C, V_DD + 3, p), f1); corners(coef_v(C, V_DD + 2, p), f0); }
+		}
+	}
+	if(EXPL) {
+		const cx<R>* f = f0 + (comp == 0 ? 0 : N);
 #pragma unroll
-			for(int j = 0; j < KS; j++) out[j] += f0[j * ss + p];
-			return;
-		}
-		if(ax) { st.template dx_m<KS>(3, xx, iy, f1, ss, out); st.template dx_m<KS>(2, xx, iy, f0, ss, out); }
-#pragma unroll
-		for(int j = 0; j < KS; j++) out[j] += f1[j * ss + p];
-		return;
-	}
-	if(KIND == ST_WOOD_X) {
-		if(comp == 0) {
-			if(ax) {
-				if(ay) {
-					st.template dx_m<KS>(1, xx, yy, f1, ss, out); st.template dxdy_m<KS>(1, xx, yy, f1, ss, out);
-					st.template dxdy_m<KS>(0, xx, yy, f0, ss, out);
-				}
-				else st.template dx_m<KS>(1, xx, iy, f1, ss, out);
-			}
-			return;
-		}
-		if(ax) st.template dx_m<KS>(2, xx, iy, f0, ss, out);
-		return;
-	}
-	if(comp == 0) {
-		if(ay) st.template dy_m<KS>(1, ix, yy, f1, ss, out);
-		return;
-	}
-	if(ay) {
-		if(ax) {
-			st.template dy_m<KS>(2, xx, yy, f0, ss, out); st.template dxdy_m<KS>(2, xx, yy, f0, ss, out);
-			st.template dxdy_m<KS>(3, xx, yy, f1, ss, out);
-		}
-		else st.template dy_m<KS>(2, ix, yy, f0, ss, out);
+		for(int j = 0; j < KS; j++) out[j] += at_off(f + 2 * N * j, own);
 	}
 }
 
@@ -693,10 +661,13 @@ __global__ void k_stencil(Geom G, int slot0, const cx<R>* __restrict__ coef, con
 	int g = (slot0 + s) / G.spg - slot0 / G.spg;
 	Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s * 2 * N;
-	const cx<R>* f1 = f0 + N;
 	int ix = p % Nx, iy = p / Nx;
-	dst[(size_t)s * 2 * N + p] = composite<R, KIND>(st, 0, ix, iy, f0, f1);
-	dst[(size_t)s * 2 * N + N + p] = composite<R, KIND>(st, 1, ix, iy, f0, f1);
+#pragma unroll
+	for(int c = 0; c < 2; c++) {
+		cx<R> r;
+		composite_m<R, KIND, 1>(st, c, ix, iy, f0, &r);
+		dst[(size_t)s * 2 * N + (size_t)c * N + p] = r;
+	}
 }
 
 // Periodic line solve with the pre-factored Thomas/Sherman-Morrison data, sequential form:
@@ -790,40 +761,47 @@ __device__ __forceinline__ cx<R> shfl_xor_c(cx<R> v, int m) {
 // exchanged): the stencil blocks b become 3 - b (00 <-> 11, 01 <-> 10), the DX and DY stencils
 // exchange, the DXDY corners (px,py), (mx,py), (px,my), (mx,my) become corners 0, 2, 1, 3, and the
 // duplicate-row/column folding and the period-(N-1) wraps map onto themselves. This kernel
-// writes, per wavelength group, the transposed planes those solves read: DY' (every block) from
-// DX, DX' (blocks 1 and 2) from DY, every DXDY' block from DXDY, and the diagonal stencils of the
-// transposed x-lines (diag' direction 0, component c') from the y diagonals of component 1 - c'.
-// Each block moves one 32x32 tile of one plane through shared memory (coalesced reads and writes).
-constexpr int NCT = 12 + 6 + 16 + 6;  // planes per group: DY', DX' (blocks 1, 2), DXDY', diag'
+// writes, per wavelength group, the transposed sets those solves read (their phase entries are not
+// used): with the set's order of blocks DY' is DX, DX' is DY and DXDY' block b is DXDY block 3 - b with
+// its two middle corners exchanged. Each block moves a 32x32 tile of one vector (or of the two pairs)
+// through shared memory, coalesced on both sides.
+// Bound: HBM (setup stream).
+constexpr int NCT = NV + 1;  // moves per group: the vectors, and the two pairs together
 template <typename S>
-__global__ void __launch_bounds__(256) k_coef_t(Geom G, const cx<S>* __restrict__ coef, const cx<S>* __restrict__ diag,
-		cx<S>* __restrict__ coefT, cx<S>* __restrict__ diagT) {
-	__shared__ cx<S> tile[32][33];
+__global__ void __launch_bounds__(256) k_coef_t(Geom G, const cx<S>* __restrict__ coef, cx<S>* __restrict__ coefT) {
+	__shared__ v4<S> tile[32][33];
 	const int Nx = G.Nx, Ny = G.Ny, N = G.N;
 	const int g = blockIdx.z / NCT, k = blockIdx.z % NCT;
-	int sp, dp;  // source / destination plane
-	bool dg = false;
-	if(k < 12) { const int b = k / 3, kk = k % 3; dp = C_DY + 3 * b + kk; sp = C_DX + 3 * (3 - b) + kk; }
-	else if(k < 18) { const int b = 1 + (k - 12) / 3, kk = (k - 12) % 3; dp = C_DX + 3 * b + kk; sp = C_DY + 3 * (3 - b) + kk; }
-	else if(k < 34) {
-		const int b = (k - 18) / 4, kk = (k - 18) % 4;
-		const int sk = kk == 1 ? 2 : kk == 2 ? 1 : kk;
-		dp = C_DXDY + 4 * b + kk; sp = C_DXDY + 4 * (3 - b) + sk;
-	}
-	else { const int cp = (k - 34) / 3, kk = (k - 34) % 3; dp = 0 * 6 + cp * 3 + kk; sp = 1 * 6 + (1 - cp) * 3 + kk; dg = true; }
-	// diagonal stencils: plain planes; coefficient planes: the tiled layout (cidx)
-	const cx<S>* src = dg ? diag + (size_t)g * NDIAG * N : coef + (size_t)g * coef_set_size(N);
-	cx<S>* dst = dg ? diagT + (size_t)g * NDIAG * N : coefT + (size_t)g * coef_set_size(N);
-	auto at = [&](int plane, int q) { return dg ? (size_t)plane * N + q : cidx(plane, q); };
+	const cx<S>* src = coef + (size_t)g * coef_set_size(N);
+	cx<S>* dst = coefT + (size_t)g * coef_set_size(N);
+	const int sv = k < V_DX ? 3 - k : k < V_DY ? k + 4 : k - 4;  // source vector of destination vector k
 	const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
 	for(int r = threadIdx.y; r < 32; r += blockDim.y) {
 		const int x = x0 + threadIdx.x, y = y0 + r;
-		if(x < Nx && y < Ny) tile[r][threadIdx.x] = src[at(sp, y * Nx + x)];
+		if(x < Nx && y < Ny) {
+			const int q = y * Nx + x;
+			v4<S> v;
+			if(k == NV) {
+				const cx<S> a = coef_u(src, U_DY, q), b = coef_u(src, U_DX, q);
+				v = v4<S>{a.x, a.y, b.x, b.y};
+			}
+			else v = coef_v(src, sv, q);
+			if(k < V_DX) v = v4<S>{v.x, v.z, v.y, v.w};
+			tile[r][threadIdx.x] = v;
+		}
 	}
 	__syncthreads();
 	for(int r = threadIdx.y; r < 32; r += blockDim.y) {
 		const int y = y0 + threadIdx.x, x = x0 + r;  // destination row x, column y
-		if(x < Nx && y < Ny) dst[at(dp, x * Ny + y)] = tile[threadIdx.x][r];
+		if(x < Nx && y < Ny) {
+			const int q = x * Ny + y;
+			const v4<S> v = tile[threadIdx.x][r];
+			if(k == NV) {
+				coef_u(dst, U_DX, q) = mk(v.x, v.y);
+				coef_u(dst, U_DY, q) = mk(v.z, v.w);
+			}
+			else coef_v(dst, k, q) = v;
+		}
 	}
 }
 
@@ -888,7 +866,7 @@ __device__ __forceinline__ Aff<T> shfl_down_a(const Aff<T>& X, int o) { return A
 
 template <typename S, int DIRN>
 __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G, int ngroups, int chunkMx, int chunksX, int W,
-		const cx<S>* __restrict__ diag, cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
+		const cx<S>* __restrict__ coef, cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
 	typedef S T;
 	const int Nx = G.Nx, Ny = G.Ny, N = G.N;
 	const int L = DIRN == 0 ? Nx : Ny;
@@ -913,7 +891,7 @@ __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G
 	const bool active = line < nlines && L > 3;
 	const int g = gc / 2, c = gc % 2;
 	const int i0 = chunk * M, i1 = min(i0 + M, n);
-	const cx<T>* Dg = diag + (size_t)g * NDIAG * N + (size_t)(DIRN * 6 + c * 3) * N;
+	const cx<T>* Cg = coef + (size_t)g * coef_set_size(N);
 	cx<S>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane;
 	const int stride = DIRN == 0 ? 1 : Nx;
 	const int base = DIRN == 0 ? Nx * line : line;
@@ -927,9 +905,9 @@ __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G
 		return (((size_t)line * chunkMx + i % chunkMx) * NFAC + f) * chunksX + (i / chunkMx);
 	};
 	const cx<T> one = mk<T>(1, 0), zero = mk<T>(0, 0);
-	auto sup = [&](int i) { return -Dg[2 * (size_t)N + P(i)]; };
-	auto mid = [&](int i) { return one - Dg[1 * (size_t)N + P(i)]; };
-	auto inf = [&](int i) { return -Dg[P(i)]; };
+	auto sup = [&](int i) { cx<T> m, cc, n; coef_diag<DIRN>(Cg, c, P(i), m, cc, n); return -n; };
+	auto mid = [&](int i) { cx<T> m, cc, n; coef_diag<DIRN>(Cg, c, P(i), m, cc, n); return one - cc; };
+	auto inf = [&](int i) { cx<T> m, cc, n; coef_diag<DIRN>(Cg, c, P(i), m, cc, n); return -m; };
 	cx<T> m0 = zero, a0 = zero, corner = zero;
 	if(active) {
 		m0 = mid(0);
@@ -1144,7 +1122,7 @@ __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G
 // and 47 us on a 64x64 FP64 one.
 constexpr int PART_KMAX = 24;
 template <typename S>
-__global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>* __restrict__ diag,
+__global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>* __restrict__ coef,
 		cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
 	const int N = G.N, nlines = G.Ny, n = G.Nx - 1;
 	const int CH = blockDim.x, t = threadIdx.x;
@@ -1152,7 +1130,8 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	const int gc = blockIdx.y, g = gc / 2, c = gc % 2;
 	const bool active = line < nlines && G.Nx > 3;
 	const int nchk = (n + M - 1) / M;
-	const cx<S>* Dg = diag + (size_t)g * NDIAG * N + (size_t)(c * 3) * N + (size_t)line * G.Nx;
+	const cx<S>* Cg = coef + (size_t)g * coef_set_size(N);
+	const int p0 = line * G.Nx;
 	cx<S>* Fc = fac + (size_t)gc * NFAC * plane + (size_t)line * part_line_size(M, CH);
 	cx<S>* If = Fc + (size_t)M * NFAC * CH;
 	cx<double>* ls = lsc + ((size_t)gc * nlines + line) * 2;
@@ -1165,7 +1144,9 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		vf = zero;
 		for(int k = 0; k < m; k++) {
 			const int i = i0 + k;
-			const cx<S> a = -Dg[i], b = one - Dg[(size_t)N + i], cs = -Dg[2 * (size_t)N + i];
+			cx<S> em, ec, en;
+			coef_diag<0>(Cg, c, p0 + i, em, ec, en);
+			const cx<S> a = -em, b = one - ec, cs = -en;
 			cx<S> al = zero;  // -l
 			if(k == 0) ev = -a;
 			else {
@@ -1342,7 +1323,9 @@ __device__ __forceinline__ void line_combine(cx<R> P, const cx<R>* d0, const cx<
 // sum and backward maps joined by shuffle scans: 20 instead of 28 multiply-adds per point and slot, 5
 // instead of 7 factor loads, and no scans (5 shuffle steps each over 3 quantities). 256x256, 16
 // wavelengths, 13 q, FP32: Woodbury solves 552 -> 490 us, explicit step 499 -> 476 us; the same mesh
-// with 3 wavelengths in FP64 (bound by the FP64 pipe) 1351 -> 962 and 1540 -> 1162 us.
+// with 3 wavelengths in FP64 (bound by the FP64 pipe) 1351 -> 962 and 1540 -> 1162 us. With the real
+// entries of the coefficient set (4 x-taps and 10 with one real number each in place of 14 complex
+// ones for the Woodbury term): FP32 490 -> 477 and 476 -> 491 us, FP64 962 -> 785 and 1162 -> 923 us.
 template <typename R, int M, int KIND, int KS, bool TOUT = false>
 // Resident blocks per SM requested from the compiler: 8 (64 registers) for the instances
 // whose chunk values fit, measured faster on GB300; the larger instances keep their registers.
@@ -2372,7 +2355,7 @@ __global__ void k_phase(Geom G, int slot0, const cx<R>* __restrict__ coef, cx<R>
 	int N = G.N;
 	int g = (slot0 + s) / G.spg - slot0 / G.spg;
 	const cx<R>* C = coef + (size_t)g * coef_set_size(N);
-	cx<R> oxx = C[cidx(C_PH + 0, p)], oyy = C[cidx(C_PH + 1, p)], oxy = C[cidx(C_PH + 2, p)];
+	cx<R> oxx = coef_ph(C, 0, p), oyy = coef_ph(C, 1, p), oxy = coef_ph(C, 2, p);
 	cx<R>* f = F + (size_t)s * 2 * N + p;
 	cx<R> a = f[0], b = f[N];
 	f[0] = oxx * a + oxy * b;
@@ -2389,7 +2372,7 @@ __device__ __forceinline__ int ref_wrap(int i, int n) {
 
 template <typename R>
 __device__ __forceinline__ void phase_apply(const cx<R>* C, size_t N, int p, cx<R>& a, cx<R>& b) {
-	cx<R> oxx = C[cidx(C_PH + 0, p)], oyy = C[cidx(C_PH + 1, p)], oxy = C[cidx(C_PH + 2, p)];
+	cx<R> oxx = coef_ph(C, 0, p), oyy = coef_ph(C, 1, p), oxy = coef_ph(C, 2, p);
 	cx<R> u = cfma(oxy, b, oxx * a), v = cfma(oyy, b, oxy * a);
 	a = u;
 	b = v;

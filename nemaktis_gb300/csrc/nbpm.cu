@@ -162,9 +162,9 @@ struct SampleHost {
 		// workspace: field-sized iterates T, T2 (T3 for the scratch-chunk y solve), eps and
 		// coefficient rings, diagonal stencils, double-buffered factor planes / line scalars
 		// (slab iz uses half iz & 1), screen and widening buffers
-		DevBuf T, T2, T3, Qring, coef, diag, facx, facy, lscx, lscy, scr, stage;
-		// transposed-frame y solves: transposed coefficient ring (two slabs) and diagonal stencils
-		DevBuf coefT, diagT;
+		DevBuf T, T2, T3, Qring, coef, facx, facy, lscx, lscy, scr, stage;
+		// transposed-frame y solves: transposed coefficient ring (two slabs)
+		DevBuf coefT;
 		size_t facx_half = 0, facy_half = 0, lsc_half = 0;
 		std::vector<cudaEvent_t*> events() {
 			return {&eFork, &eJoin, &eCoef, &eFac, &eTrans, &eAdi[0], &eAdi[1], &eNref, &eNrefFork, &eEnd};
@@ -555,11 +555,7 @@ struct Plan : PlanBase {
 				if(need_t3) dalloc(L.T3, sizeof(cx<R>) * nT);
 				dalloc(L.Qring, sizeof(R) * (size_t)2 * ng * NQ * N);
 				dalloc(L.coef, sizeof(cx<R>) * (size_t)2 * ng * coef_set_size((int)N));  // two slabs (transition kernels)
-				dalloc(L.diag, sizeof(cx<R>) * (size_t)ng * NDIAG * N);
-				if(need_t) {
-					dalloc(L.coefT, sizeof(cx<R>) * (size_t)2 * ng * coef_set_size((int)N));
-					dalloc(L.diagT, sizeof(cx<R>) * (size_t)ng * NDIAG * N);
-				}
+				if(need_t) dalloc(L.coefT, sizeof(cx<R>) * (size_t)2 * ng * coef_set_size((int)N));
 				L.facx_half = L.facy_half = nFx;
 				L.lsc_half = nL;
 				dalloc(L.facx, sizeof(cx<R>) * nFx * 2);
@@ -568,8 +564,8 @@ struct Plan : PlanBase {
 				dalloc(L.lscy, sizeof(cx<double>) * nL * 2);
 				dalloc(L.scr, sizeof(cx<R>) * (size_t)2 * ng * 2 * 2 * N);  // x and y halves
 				if(sizeof(R) != sizeof(double)) dalloc(L.stage, sizeof(cx<double>) * (size_t)h.slots * 2 * N);
-				for(DevBuf* b : {&L.T, &L.T2, &L.T3, &L.Qring, &L.coef, &L.diag, &L.facx, &L.facy, &L.lscx, &L.lscy,
-						&L.scr, &L.stage, &L.coefT, &L.diagT})
+				for(DevBuf* b : {&L.T, &L.T2, &L.T3, &L.Qring, &L.coef, &L.facx, &L.facy, &L.lscx, &L.lscy,
+						&L.scr, &L.stage, &L.coefT})
 					dev_bytes += b->bytes;
 			}
 			// per-sample buffers
@@ -678,7 +674,7 @@ struct Plan : PlanBase {
 			auto& L = hp->lane;
 			auto drop = [&](DevBuf& b) { dev_bytes -= (long long)b.bytes; b.alloc(0); };
 			if(!scfg[hp->index].ys && L.T3.p) drop(L.T3);
-			if(!scfg[hp->index].Mxt && L.coefT.p) { drop(L.coefT); drop(L.diagT); }
+			if(!scfg[hp->index].Mxt && L.coefT.p) drop(L.coefT);
 		}
 		select(*S[0]);
 	}
@@ -700,7 +696,7 @@ struct Plan : PlanBase {
 	void zero_workspace() {
 		for(auto& hp : S) {
 			auto& L = hp->lane;
-			for(DevBuf* b : {&L.T, &L.T2, &L.T3, &L.coef, &L.facx, &L.facy, &L.lscx, &L.lscy, &L.coefT, &L.diagT, &hp->F})
+			for(DevBuf* b : {&L.T, &L.T2, &L.T3, &L.coef, &L.facx, &L.facy, &L.lscx, &L.lscy, &L.coefT, &hp->F})
 				if(b->p) CK(cudaMemsetAsync(b->p, 0, b->bytes, stream0));
 		}
 		CK(cudaStreamSynchronize(stream0));
@@ -914,7 +910,6 @@ struct Plan : PlanBase {
 		cx<R>* T2b = nullptr;
 		R* Qr[2] = {nullptr, nullptr};
 		cx<R>* Cring[2] = {nullptr, nullptr};
-		cx<R>* Dg = nullptr;
 		const cx<R>* Cprev = nullptr;
 		double eps_bytes = 0, field_pts = 0;
 	};
@@ -963,7 +958,6 @@ struct Plan : PlanBase {
 		ps.Qr[1] = ps.Qr[0] + (size_t)ps.ng * NQ * N;
 		ps.Cring[0] = W->coef.as<cx<R>>();
 		ps.Cring[1] = W->coef.as<cx<R>>() + (size_t)ps.ng * coef_set_size(N);
-		ps.Dg = W->diag.as<cx<R>>();
 		ps.eps_bytes = (double)N * ps.ng * (h.fd * 8 + (mk_ ? 1 : 0) + NQ * sizeof(R));
 		ps.field_pts = (double)N * ps.nsl;
 		const int ng = ps.ng, nsl = ps.nsl, slot0 = ps.slot0;
@@ -988,12 +982,12 @@ struct Plan : PlanBase {
 	}
 
 	// Factorisation for the partitioned x-line solves: one block of 4 lines, or of one line of wpl warps.
-	void rec_factor_part(const char* name, double bytes, const Geom& Gm, int ng, int M, int wpl, const cx<R>* dg, cx<R>* fac,
+	void rec_factor_part(const char* name, double bytes, const Geom& Gm, int ng, int M, int wpl, const cx<R>* C, cx<R>* fac,
 			size_t plane, cx<double>* lsc) {
 		const int LT = wpl > 1 ? 1 : 4;
 		launch(name, bytes, [&] {
 			k_factor_part<R><<<dim3((unsigned)((Gm.Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32 * wpl, LT), 0, cs>>>(
-				Gm, M, dg, fac, plane, lsc);
+				Gm, M, C, fac, plane, lsc);
 		});
 	}
 
@@ -1029,37 +1023,37 @@ struct Plan : PlanBase {
 			});
 			// coef(iz) overwrites the set the transition of slab iz-1 read (slab iz-2)
 			if(iz >= 1) CK(cudaStreamWaitEvent(streamB, eTrans, 0));
-			launch("coef", (double)N * ng * (2 * NQ * sizeof(R) + NCOEF * sc + NDIAG * sc + (wts ? 16 : 0)), [&] {
-				k_coef<R><<<pgrid(N, ng, 128), 128, 0, cs>>>(QA, QB, wts, iz, Gm, gps, C, ps.Dg);
+			launch("coef", (double)N * ng * (2 * NQ * sizeof(R) + CSET * sizeof(R) + (wts ? 16 : 0)), [&] {
+				k_coef<R><<<pgrid(N, ng, 128), 128, 0, cs>>>(QA, QB, wts, iz, Gm, gps, C);
 			});
 			CK(cudaEventRecord(eCoef, streamB));
 			// factor(iz) overwrites the half the line solves of slab iz-2 used
 			if(iz >= 2) CK(cudaStreamWaitEvent(streamB, eAdi[iz & 1], 0));
-			const double fb = (double)N * ng * 2 * (3 * sc + NFAC * sc + 4 * sc);
+			const double fb = (double)N * ng * 2 * (2 * sc + NFAC * sc);  // 4 scalars of the set read per component
 			// y factorisation: 8 chunk warps per 32 columns, 16 when the grid leaves SMs idle
 			const int LT = 4, WF = ((Nx + 31) / 32) * 2 * ng < nsm && Ny - 1 >= 256 ? 16 : 8;
 			if(scf.Mx && !scf.xs)
-				rec_factor_part("factor_x", fb, Gm, ng, scf.Mx, scf.WPLx, ps.Dg, fx, scf.plane_x, lx);
+				rec_factor_part("factor_x", fb, Gm, ng, scf.Mx, scf.WPLx, C, fx, scf.plane_x, lx);
 			else launch("factor_x", fb, [&] {
 				k_factor_chunked<R, 0><<<dim3((unsigned)((Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
-					Gm, ng, scf.Mx, 32 * scf.WPLx, 1, ps.Dg, fx, scf.plane_x, lx);
+					Gm, ng, scf.Mx, 32 * scf.WPLx, 1, C, fx, scf.plane_x, lx);
 			});
 			cx<R>* CT = scf.Mxt ? W->coefT.as<cx<R>>() + (size_t)(iz & 1) * ng * coef_set_size(N) : nullptr;
 			if(scf.Mxt) {
 				// y-lines as x-lines of the transposed frame: transposed coefficients and diagonals,
 				// then the x-line factorisation of that frame
 				const Geom Gt = transposed(Gm);
-				launch("coef_t", 2.0 * N * ng * NCT * sc, [&] {
+				launch("coef_t", 2.0 * N * ng * (CSET - 6) * sizeof(R), [&] {
 					k_coef_t<R><<<dim3((unsigned)((Nx + 31) / 32), (unsigned)((Ny + 31) / 32), (unsigned)(ng * NCT)), dim3(32, 8), 0,
-						cs>>>(Gm, C, ps.Dg, CT, W->diagT.as<cx<R>>());
+						cs>>>(Gm, C, CT);
 				});
-				rec_factor_part("factor_y", fb, Gt, ng, scf.Mxt, scf.WPLt, W->diagT.as<cx<R>>(), fy, scf.plane_y, ly);
+				rec_factor_part("factor_y", fb, Gt, ng, scf.Mxt, scf.WPLt, CT, fy, scf.plane_y, ly);
 			}
 			else {
 				size_t smem = (size_t)WF * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>);
 				launch("factor_y", fb, [&] {
 					k_factor_chunked<R, 1><<<dim3((unsigned)((Nx + 31) / 32), (unsigned)(ng * 2)), dim3(32, WF), smem, cs>>>(
-						Gm, ng, 0, 32, WF, ps.Dg, fy, scf.plane_y, ly);
+						Gm, ng, 0, 32, WF, C, fy, scf.plane_y, ly);
 				});
 			}
 			CK(cudaEventRecord(eFac, streamB));
@@ -1268,7 +1262,7 @@ struct Plan : PlanBase {
 		// once per wavelength
 		const int reads = 1 + (acc_in && acc_in != src ? 1 : 0) + (acc_in2 && acc_in2 != src && acc_in2 != acc_in ? 1 : 0);
 		const int writes = (dst ? 1 : 0) + (acc_out ? 1 : 0);
-		double bytes = fp * (reads + writes) + (double)Gm.N * ng * (2 * NFAC + (wood ? 14 : 20)) * sz;
+		double bytes = fp * (reads + writes) + (double)Gm.N * ng * (2 * NFAC * sz + (wood ? 18 : 26) * sizeof(R));
 		SolveLaunch L;
 		L.stream = cs;
 		if(dirn == 0) {
