@@ -23,6 +23,38 @@ namespace nbpm {
 
 // Per-voxel derived permittivity components (PermittivityTensorField.cpp:3-99).
 enum { Q_XXTR = 0, Q_YYTR, Q_XYTR, Q_XXS, Q_YYS, Q_XYS, Q_VX, Q_VY, Q_IZZ, NQ };
+// Line-solve factor planes.
+// F_A = alpha_i = -inf_i/beta_i (forward recurrence d_i = alpha_i d_{i-1} + b_i/beta_i),
+// F_RB = 1/beta_i, F_W = w_i, F_C = -gamma_i (backward recurrence), F_COR = corr_i.
+enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
+// Factor planes of the partitioned x-line solves (k_factor_part): every chunk of M points of a line
+// is factored by itself. F_A = -l_i (forward recurrence d_i = r_i - l_i d_{i-1}, l_i = a_i/beta_{i-1},
+// 0 at the chunk's first point), F_RB = 1/beta_i, F_C = -c_i/beta_i, F_Z = (product of F_C over the
+// points before i) * F_RB, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
+// unknown before the chunk adds to point i before the backward sweep.
+enum { F_Z = F_W, F_E = F_COR };
+// Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
+// first one): h = I_HD d_last + I_HY yf' and g = I_GD d_last + I_GY yf' from the two chunks alone,
+// I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds.
+enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, NIF };
+// Layout of a line's factors: for each point k of a chunk the vectors {F_A, F_Z} of the CH chunks, then
+// {F_RB, F_C}, then F_E; after the M points the NIF interface coefficients of the chunks.
+__host__ __device__ __forceinline__ size_t part_line_size(int M, int CH) { return (size_t)CH * (M * NFAC + NIF); }
+template <typename S>
+struct alignas(4 * sizeof(S)) v4 {
+	S x, y, z, w;
+};
+template <typename S>
+__device__ __forceinline__ const v4<S>& part_az(const cx<S>* Fc, int k, int CH, int ci) {
+	return reinterpret_cast<const v4<S>*>(Fc + (size_t)k * NFAC * CH)[ci];
+}
+template <typename S>
+__device__ __forceinline__ const v4<S>& part_rc(const cx<S>* Fc, int k, int CH, int ci) {
+	return reinterpret_cast<const v4<S>*>(Fc + (size_t)k * NFAC * CH + 2 * CH)[ci];
+}
+template <typename S>
+__device__ __forceinline__ const cx<S>& part_e(const cx<S>* Fc, int k, int CH, int ci) { return Fc[(size_t)k * NFAC * CH + 4 * CH + ci]; }
+
 // Coefficient set of one point. The entries of mu*R are i*(dZ/2)*(real), but for the walk-off terms: first
 // derivatives, which only the outer entries of DX blocks 0, 1, 2 and of DY blocks 1, 2, 3 have. So an
 // entry is one real number (its imaginary part) except those twelve, 52 numbers in place of 80, and a
@@ -37,10 +69,6 @@ enum { Q_XXTR = 0, Q_YYTR, Q_XYTR, Q_XXS, Q_YYS, Q_XYS, Q_VX, Q_VY, Q_IZZ, NQ };
 // at fixed distances from one address and 32 consecutive points of a vector are one contiguous segment.
 enum { V_DD = 0, V_DX = 4, V_DY = 8, NV = 12, U_DX = 0, U_DY = 1, NU = 2 };
 enum { CSET = 4 * NV + 2 * NU + 6 };  // scalars per point: vectors, pairs, 3 complex phase entries
-template <typename S>
-struct alignas(4 * sizeof(S)) v4 {
-	S x, y, z, w;
-};
 // complex values per group
 __host__ __device__ __forceinline__ size_t coef_set_size(int N) { return (size_t)(CSET / 2) * (((size_t)N + 31) & ~(size_t)31); }
 template <typename C>
@@ -74,24 +102,6 @@ __device__ __forceinline__ void coef_diag(const cx<S>* coef, int comp, int p, cx
 		c = mk((S)0, v.z);
 	}
 }
-// Line-solve factor planes.
-// F_A = alpha_i = -inf_i/beta_i (forward recurrence d_i = alpha_i d_{i-1} + b_i/beta_i),
-// F_RB = 1/beta_i, F_W = w_i, F_C = -gamma_i (backward recurrence), F_COR = corr_i.
-enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
-// Factor planes of the partitioned x-line solves (k_factor_part): every chunk of M points of a line
-// is factored by itself. F_A = -l_i (forward recurrence d_i = r_i - l_i d_{i-1}, l_i = a_i/beta_{i-1},
-// 0 at the chunk's first point), F_RB = 1/beta_i, F_C = -c_i/beta_i, F_Z = (product of F_C over the
-// points before i) * F_RB, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
-// unknown before the chunk adds to point i before the backward sweep.
-enum { F_Z = F_W, F_E = F_COR };
-// Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
-// first one): h = I_HD d_last + I_HY yf' and g = I_GD d_last + I_GY yf' from the two chunks alone,
-// I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds.
-enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, NIF };
-// Elements per line of the chunk-interleaved factor layout: CH chunks of M points, NFAC planes and
-// the NIF interface coefficients of every chunk.
-__host__ __device__ __forceinline__ size_t part_line_size(int M, int CH) { return (size_t)CH * (M * NFAC + NIF); }
-
 struct GroupParams {
 	double wavelength, k0, dX, dY, dZ;
 	double no, ne, ne_imag, nhost, nin, nout_fresnel;
@@ -1157,12 +1167,10 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 			rb = crecip(beta);
 			cprev = cs;
 			const cx<S> cc = -(rb * cs), z = cpz * rb, e = rb * ev;
-			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
-			F[F_A * CH] = al;
-			F[F_RB * CH] = rb;
-			F[F_Z * CH] = z;
-			F[F_C * CH] = cc;
-			F[F_E * CH] = e;
+			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH;
+			reinterpret_cast<v4<S>*>(F)[i / M] = v4<S>{al.x, al.y, z.x, z.y};
+			reinterpret_cast<v4<S>*>(F + 2 * CH)[i / M] = v4<S>{rb.x, rb.y, cc.x, cc.y};
+			F[4 * CH + i / M] = e;
 			vf = cfma(z, ev, vf);
 			cpz = cpz * cc;
 			vl = e;
@@ -1174,6 +1182,16 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	const int i0 = t * M;
 	const bool own = active && i0 < n;
 	if(own) chunk(i0, min(M, n - i0));
+	if(active) {
+		// past the line's end: entries that leave the sweeps' values as they are, so that the solves need no
+		// condition at every point (a branch there makes each point wait for its own factors)
+		for(int k = max(0, min(M, n - i0)); k < M; k++) {
+			cx<S>* F = Fc + (size_t)k * NFAC * CH;
+			reinterpret_cast<v4<S>*>(F)[t] = v4<S>{1, 0, 0, 0};
+			reinterpret_cast<v4<S>*>(F + 2 * CH)[t] = v4<S>{0, 0, 1, 0};
+			F[4 * CH + t] = zero;
+		}
+	}
 	// the next chunk's responses (cyclic), through shared memory
 	__shared__ cx<S> shv[256], shw[256];
 	__shared__ S shr[8];
@@ -1230,8 +1248,9 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 }
 
 // The sequential solve of a line flagged -1 by k_factor_part, by one thread: buf holds the right-hand
-// sides of KS slots (element i at (i / M) * (M + 1) + i % M) and receives the solution.
-template <typename R, int M, int KS>
+// sides of KS slots (element i of slot j at ((i / M) * (M + 1) + i % M) * ES + j * PITCH) and receives the
+// solution.
+template <typename R, int M, int KS, int ES = 1>
 __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n) {
 	const cx<R>* If = Fc + (size_t)M * NFAC * CH;
 #pragma unroll 1
@@ -1239,18 +1258,18 @@ __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* 
 		cx<R>* b = buf + j * PITCH;
 		cx<R> d = mk<R>(0, 0), yf = mk<R>(0, 0);
 		for(int i = 0; i < n; i++) {
-			const cx<R>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
-			cx<R>& v = b[(i / M) * (M + 1) + i % M];
-			d = cfma(F[F_A * CH], d, v);
+			const v4<R> az = part_az(Fc, i % M, CH, i / M);
+			cx<R>& v = b[((i / M) * (M + 1) + i % M) * ES];
+			d = cfma(mk(az.x, az.y), d, v);
 			v = d;
-			yf = cfma(F[F_Z * CH], d, yf);
+			yf = cfma(mk(az.z, az.w), d, yf);
 		}
 		const cx<R> h = cfma(If[I_HY * CH], yf, If[I_HD * CH] * d);
 		cx<R> x = cfma(If[I_GY * CH], yf, If[I_GD * CH] * d);
 		for(int i = n - 1; i >= 0; i--) {
-			const cx<R>* F = Fc + (size_t)(i % M) * NFAC * CH + i / M;
-			cx<R>& v = b[(i / M) * (M + 1) + i % M];
-			x = cfma(F[F_C * CH], x, cfma(F[F_E * CH], h, F[F_RB * CH] * v));
+			const v4<R> rc = part_rc(Fc, i % M, CH, i / M);
+			cx<R>& v = b[((i / M) * (M + 1) + i % M) * ES];
+			x = cfma(mk(rc.z, rc.w), x, cfma(part_e(Fc, i % M, CH, i / M), h, mk(rc.x, rc.y) * v));
 			v = x;
 		}
 	}
@@ -1358,7 +1377,6 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 	if(iy < Ny) {  // always true unless TOUT (whose block writes together after a barrier)
 	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
 	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
-	const int i0 = lane * M;
 	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s0 * 2 * N;
@@ -1367,12 +1385,14 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 #pragma unroll 1
 	for(int t = 0; t < M; t++) {
 		const int e = lane + 32 * t;
-		if(e < n_unk) {
-			cx<R> r[KS];
-			composite_m<R, KIND, KS>(st, c, e, iy, f0, r);
+		cx<R> r[KS];
+		if(e < n_unk) composite_m<R, KIND, KS>(st, c, e, iy, f0, r);
+		else {
 #pragma unroll
-			for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
+			for(int j = 0; j < KS; j++) r[j] = zero;
 		}
+#pragma unroll
+		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
 	}
 	__syncwarp();
 	if(K >= 0) {
@@ -1384,20 +1404,19 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
 		for(int k = 0; k < M; k++) {
-			if(i0 + k < n_unk) {
-				const cx<R> z = Fc[(k * NFAC + F_Z) * 32 + lane];
-				if(k == 0) {
+			const v4<R> az = part_az(Fc, k, 32, lane);
+			const cx<R> z = mk(az.z, az.w);
+			if(k == 0) {
 #pragma unroll
-					for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
-				}
-				else {
-					const cx<R> a = Fc[(k * NFAC + F_A) * 32 + lane];
+				for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
+			}
+			else {
+				const cx<R> a = mk(az.x, az.y);
 #pragma unroll
-					for(int j = 0; j < KS; j++) {
-						d[j] = cfma(a, d[j], vb[j * PITCH + k]);
-						vb[j * PITCH + k] = d[j];
-						yf[j] = cfma(z, d[j], yf[j]);
-					}
+				for(int j = 0; j < KS; j++) {
+					d[j] = cfma(a, d[j], vb[j * PITCH + k]);
+					vb[j * PITCH + k] = d[j];
+					yf[j] = cfma(z, d[j], yf[j]);
 				}
 			}
 		}
@@ -1435,9 +1454,9 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
 #pragma unroll
 		for(int k = M - 1; k >= 0; k--) {
-			if(i0 + k < n_unk) {
-				const cx<R> rb = Fc[(k * NFAC + F_RB) * 32 + lane], cc = Fc[(k * NFAC + F_C) * 32 + lane];
-				const cx<R> ee = Fc[(k * NFAC + F_E) * 32 + lane];
+			{
+				const v4<R> rc = part_rc(Fc, k, 32, lane);
+				const cx<R> rb = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, 32, lane);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
 					x[j] = cfma(cc, x[j], cfma(ee, h[j], rb * vb[j * PITCH + k]));
@@ -1929,14 +1948,19 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 	cx<R>* sH = sG + 2 * KS * W;                      // [2][KS][W + 1]: h of the warps' last chunks, then of the line's
 	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, CH);
 	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
-	const int i0 = ci * M;
 	const int last = (n_unk - 1) / M;  // last chunk
 	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s0 * 2 * N;
-	for(int e = threadIdx.x; e < n_unk; e += blockDim.x) {
+#pragma unroll 1
+	for(int t = 0; t < M; t++) {
+		const int e = threadIdx.x + CH * t;
 		cx<R> r[KS];
-		composite_m<R, KIND, KS>(st, c, e, iy, f0, r);
+		if(e < n_unk) composite_m<R, KIND, KS>(st, c, e, iy, f0, r);
+		else {
+#pragma unroll
+			for(int j = 0; j < KS; j++) r[j] = zero;
+		}
 #pragma unroll
 		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
 	}
@@ -1949,20 +1973,19 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
 		for(int k = 0; k < M; k++) {
-			if(i0 + k < n_unk) {
-				const cx<R> z = Fc[(k * NFAC + F_Z) * CH + ci];
-				if(k == 0) {
+			const v4<R> az = part_az(Fc, k, CH, ci);
+			const cx<R> z = mk(az.z, az.w);
+			if(k == 0) {
 #pragma unroll
-					for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
-				}
-				else {
-					const cx<R> a = Fc[(k * NFAC + F_A) * CH + ci];
+				for(int j = 0; j < KS; j++) { d[j] = vb[j * PITCH]; yf[j] = z * d[j]; }
+			}
+			else {
+				const cx<R> a = mk(az.x, az.y);
 #pragma unroll
-					for(int j = 0; j < KS; j++) {
-						d[j] = cfma(a, d[j], vb[j * PITCH + k]);
-						vb[j * PITCH + k] = d[j];
-						yf[j] = cfma(z, d[j], yf[j]);
-					}
+				for(int j = 0; j < KS; j++) {
+					d[j] = cfma(a, d[j], vb[j * PITCH + k]);
+					vb[j * PITCH + k] = d[j];
+					yf[j] = cfma(z, d[j], yf[j]);
 				}
 			}
 		}
@@ -2024,9 +2047,9 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
 #pragma unroll
 		for(int k = M - 1; k >= 0; k--) {
-			if(i0 + k < n_unk) {
-				const cx<R> rb = Fc[(k * NFAC + F_RB) * CH + ci], cc = Fc[(k * NFAC + F_C) * CH + ci];
-				const cx<R> ee = Fc[(k * NFAC + F_E) * CH + ci];
+			{
+				const v4<R> rc = part_rc(Fc, k, CH, ci);
+				const cx<R> rb = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, CH, ci);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
 					x[j] = cfma(cc, x[j], cfma(ee, hl[j], rb * vb[j * PITCH + k]));
@@ -2692,6 +2715,178 @@ __global__ void k_phase_sync(Geom G, int slot0, const cx<R>* __restrict__ CA, co
 		if(Cb) phase_apply(Cb, N, d, a, b);
 		f[d] = a;
 		f[N + d] = b;
+	};
+	put(p);
+	if(ax && ix == 0) put((Nx - 1) + Nx * iy);
+	if(ay && iy == 0) put(ix + Nx * (Ny - 1));
+	if(ax && ay && ix == 0 && iy == 0) put((Nx - 1) + Nx * (Ny - 1));
+}
+
+// k_shift_fused for the two slots of a (wavelength, q) (FP32): the same window passes, one slot after the
+// other through the same shared memory, the results written as pairs (pair_kernels.cuh). The phase entries
+// and the window's indices are the same for both. blockIdx.z: pair of the pass; pair0: the pass's first one.
+static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0, const ShiftParams* __restrict__ sp,
+		const cx<float>* __restrict__ CA, const cx<float>* __restrict__ CB, int nsh, const cx<float>* __restrict__ F,
+		v4<float>* __restrict__ Fo) {
+	typedef float R;
+	extern __shared__ unsigned char smem_raw[];
+	const int z = blockIdx.z, g = z / G.Nq;
+	const ShiftParams& P = sp[pair0 + z];
+	const ShiftW<R> W(P);
+	const size_t N = G.N;
+	const int Nx = G.Nx, Ny = G.Ny;
+	const bool ax = Nx > 3, ay = Ny > 3;
+	const int x0 = blockIdx.x * SHT, y0 = blockIdx.y * SHT;
+	const int tid = threadIdx.x;
+	const cx<R>* f = F + (size_t)z * 4 * N;
+	v4<float>* fo = Fo + (size_t)z * 2 * N;
+	const cx<R>* Ca = CA ? CA + (size_t)g * coef_set_size(N) : nullptr;
+	const cx<R>* Cb = CB + (size_t)g * coef_set_size(N);
+	const int Px = Nx - 1, Py = Ny - 1;
+	const int bx = ax ? nsh * (P.msx - 1) : 0, by = ay ? nsh * (P.msy - 1) : 0;
+	const int wx = ax ? SHT + 3 * nsh : SHT, wy = ay ? SHT + 3 * nsh : SHT;
+	cx<R> ph = W.ph;
+	if(nsh == 2) ph = ph * ph;
+	const bool regular = (!ax || P.msx - 1 > -Px) && (!ay || P.msy - 1 > -Py);  // see k_shift_fused
+	if(!regular) {
+		for(int e = tid; e < SHT * SHT; e += blockDim.x) {
+			int ix = x0 + e % SHT, iy = y0 + e / SHT;
+			if(ix >= Nx || iy >= Ny) continue;
+			cx<R> o[2][2];
+			for(int pol = 0; pol < 2; pol++) {
+				shift_point_exact(G, P, f + pol * 2 * N, Ca, nsh, ix, iy, o[pol][0], o[pol][1]);
+				o[pol][0] = o[pol][0] * ph;
+				o[pol][1] = o[pol][1] * ph;
+				phase_apply(Cb, N, ix + Nx * iy, o[pol][0], o[pol][1]);
+			}
+			for(int c = 0; c < 2; c++) fo[c * N + ix + Nx * iy] = v4<float>{o[0][c].x, o[0][c].y, o[1][c].x, o[1][c].y};
+		}
+		return;
+	}
+	constexpr int PA = SHT + 7, PB = SHT + 1;
+	cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);  // [2][wy][PA]: the window
+	cx<R>* B = A + 2 * (SHT + 6) * PA;             // [2][wy][PB]: the window after the x-passes
+	const int lane = tid % 32, warp = tid / 32, nwarp = blockDim.x / 32;
+	int xc[2];
+#pragma unroll
+	for(int h = 0; h < 2; h++) {
+		const int u = lane + 32 * h;
+		xc[h] = u >= wx ? -1 : ax ? pmod(x0 + bx + u, Px) : (x0 + u < Nx ? x0 + u : -1);
+	}
+	// the thread's outputs: 4 rows of one column (SHT * SHT / 4 threads)
+	const int ix = x0 + tid % SHT, iy0 = y0 + tid / SHT * 4;
+	cx<R> keep[2][4];
+	for(int pol = 0; pol < 2; pol++) {
+		const cx<R>* fp = f + pol * 2 * N;
+		if(pol) __syncthreads();  // the first slot's window has been read
+		for(int v = warp; v < wy; v += nwarp) {
+			const int yi = ay ? pmod(y0 + by + v, Py) : (y0 + v < Ny ? y0 + v : -1);
+#pragma unroll
+			for(int h = 0; h < 2; h++) {
+				const int u = lane + 32 * h;
+				if(u < wx) {
+					cx<R> a = mk<R>(0, 0), b = mk<R>(0, 0);
+					if(xc[h] >= 0 && yi >= 0) tap_in(fp, Ca, N, xc[h] + Nx * yi, a, b);
+					A[v * PA + u] = a;
+					A[(SHT + 6) * PA + v * PA + u] = b;
+				}
+			}
+		}
+		__syncthreads();
+		const cx<R>* Y = A;
+		int PY = PA;
+		if(ax) {
+			const int nin = 8 + 3 * nsh;
+			for(int t = tid; t < 2 * 4 * wy; t += blockDim.x) {
+				const int v = t % wy, r = t / wy, seg = r % 4, c = r / 4;
+				const cx<R>* in = A + c * (SHT + 6) * PA + v * PA + seg * 8;
+				cx<R> w[14];
+#pragma unroll
+				for(int k = 0; k < 14; k++) w[k] = k < nin ? in[k] : mk<R>(0, 0);
+#pragma unroll
+				for(int k = 0; k < 11; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
+				if(nsh == 2) {
+#pragma unroll
+					for(int k = 0; k < 8; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
+				}
+				cx<R>* out = B + c * (SHT + 6) * PB + v * PB + seg * 8;
+#pragma unroll
+				for(int k = 0; k < 8; k++) out[k] = w[k];
+			}
+			__syncthreads();
+			Y = B;
+			PY = PB;
+		}
+		cx<R> o[2][4];
+#pragma unroll
+		for(int c = 0; c < 2; c++) {
+			const cx<R>* in = Y + c * (SHT + 6) * PY + (tid / SHT) * 4 * PY + tid % SHT;
+			if(ay) {
+				const int nin = 4 + 3 * nsh;
+				cx<R> w[10];
+#pragma unroll
+				for(int k = 0; k < 10; k++) w[k] = k < nin ? in[k * PY] : mk<R>(0, 0);
+#pragma unroll
+				for(int k = 0; k < 7; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
+				if(nsh == 2) {
+#pragma unroll
+					for(int k = 0; k < 4; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
+				}
+#pragma unroll
+				for(int k = 0; k < 4; k++) o[c][k] = w[k];
+			}
+			else {
+#pragma unroll
+				for(int k = 0; k < 4; k++) o[c][k] = in[k * PY];
+			}
+		}
+		if(pol == 0) {
+#pragma unroll
+			for(int k = 0; k < 4; k++) { keep[0][k] = o[0][k]; keep[1][k] = o[1][k]; }
+		}
+		else if(ix < Nx) {
+#pragma unroll
+			for(int k = 0; k < 4; k++) {
+				const int iy = iy0 + k;
+				if(iy < Ny) {
+					cx<R> a0 = keep[0][k] * ph, a1 = keep[1][k] * ph, b0 = o[0][k] * ph, b1 = o[1][k] * ph;
+					const int p = ix + Nx * iy;
+					phase_apply(Cb, N, p, a0, a1);
+					phase_apply(Cb, N, p, b0, b1);
+					fo[p] = v4<float>{a0.x, a0.y, b0.x, b0.y};
+					fo[N + p] = v4<float>{a1.x, a1.y, b1.x, b1.y};
+				}
+			}
+		}
+	}
+}
+
+// k_phase_sync for the two slots of a (wavelength, q) (FP32), out of place: plain planes in, pairs out.
+static __global__ void k_phase_sync_pair(Geom G, const cx<float>* __restrict__ CA, const cx<float>* __restrict__ CB,
+		const cx<float>* __restrict__ F, v4<float>* __restrict__ Fo) {
+	int p = blockIdx.x * blockDim.x + threadIdx.x;
+	if(p >= G.N) return;
+	const int z = blockIdx.y, g = z / G.Nq;
+	const size_t N = G.N;
+	const int Nx = G.Nx, Ny = G.Ny;
+	const bool ax = Nx > 3, ay = Ny > 3;
+	int ix = p % Nx, iy = p / Nx;
+	if((ax && ix == Nx - 1) || (ay && iy == Ny - 1)) return;
+	const cx<float>* f = F + (size_t)z * 4 * N + p;
+	v4<float>* fo = Fo + (size_t)z * 2 * N;
+	const cx<float>* Cb = CB + (size_t)g * coef_set_size(N);
+	cx<float> u0 = f[0], u1 = f[N], v0 = f[2 * N], v1 = f[3 * N];
+	if(CA) {
+		const cx<float>* Ca = CA + (size_t)g * coef_set_size(N);
+		phase_apply(Ca, N, p, u0, u1);
+		phase_apply(Ca, N, p, v0, v1);
+	}
+	auto put = [&](int d) {
+		cx<float> a = u0, b = u1, c = v0, e = v1;
+		phase_apply(Cb, N, d, a, b);
+		phase_apply(Cb, N, d, c, e);
+		fo[d] = v4<float>{a.x, a.y, c.x, c.y};
+		fo[N + d] = v4<float>{b.x, b.y, e.x, e.y};
 	};
 	put(p);
 	if(ax && ix == 0) put((Nx - 1) + Nx * iy);

@@ -26,6 +26,7 @@
 #include "../../include/nbpm.h"
 #include "bpm_kernels.cuh"
 #include "fft_kernels.cuh"
+#include "pair_kernels.cuh"
 #include "plan_iface.h"
 #include "vti_writer.h"
 #include "host_settings.h"
@@ -487,9 +488,11 @@ struct Plan : PlanBase {
 			(int)((size_t)16 * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>))));
 		CK(cudaFuncSetAttribute(k_shift_fused<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)((size_t)4 * (SHT + 6) * (SHT + 6) * sizeof(cx<R>))));
+		CK(cudaFuncSetAttribute(k_shift_pair, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			(int)((size_t)4 * (SHT + 6) * (SHT + 6) * sizeof(cx<float>))));
 		if(sizeof(R) == sizeof(float)) {
 			set_solve_smem_x_f32((int)smem_limit); set_solve_smem_y_f32((int)smem_limit); set_solve_smem_yt_f32((int)smem_limit);
-			set_solve_smem_xs_f32((int)smem_limit); set_solve_smem_xw_f32((int)smem_limit);
+			set_solve_smem_xs_f32((int)smem_limit); set_solve_smem_xw_f32((int)smem_limit); set_solve_smem_pair((int)smem_limit);
 		}
 		else {
 			set_solve_smem_x_f64((int)smem_limit); set_solve_smem_y_f64((int)smem_limit); set_solve_smem_yt_f64((int)smem_limit);
@@ -631,6 +634,9 @@ struct Plan : PlanBase {
 			if(!zeroed) { zero_workspace(); zeroed = true; }
 			const std::string key = tune_key(h);
 			std::string note;
+			double best_sum = 0;
+			int timed = 0;
+			no_pairs = true;
 			for(int dirn = 0; dirn < 2; dirn++) {
 				if(!forced.empty() && (dirn == 0 ? forced.substr(0, forced.find(';')) != "auto"
 						: (forced.find(';') != std::string::npos && forced.substr(forced.find(';') + 1) != "auto")))
@@ -663,6 +669,44 @@ struct Plan : PlanBase {
 				const std::string ws = dirn == 0 ? win.xstr() : win.ystr();
 				tune_cache_put((dirn == 0 ? "x|" : "y|") + key, ws);
 				note += std::string(dirn == 0 ? "x" : "y") + " tuned " + ws + " [" + times + "]; ";
+				best_sum += best;
+				timed++;
+			}
+			no_pairs = false;
+			// the pair kernels need both directions: their best x and y together against the best of each
+			if(timed == 2 && sizeof(R) == sizeof(float)) {
+				const SolveCfg keep = sc;
+				SolveCfg win = sc;
+				double sum = 0;
+				std::string times;
+				for(int dirn = 0; dirn < 2; dirn++) {
+					const auto& cands = dirn == 0 ? xc : yc;
+					double best = 1e300;
+					for(auto& c : cands) {
+						if(!(dirn == 0 ? c.pair_x() : c.pair_y())) continue;
+						SolveCfg t = win;
+						if(dirn == 0) {
+							t.set_x(c);
+							for(auto& d : yc) if(d.pair_y()) { t.set_y(d); break; }
+						}
+						else t.set_y(c);
+						t.plane_x = pmax;
+						if(!t.pairs()) continue;
+						sc = t;
+						const double ms = time_direction(h, dirn);
+						char b[96];
+						std::snprintf(b, sizeof b, "%s %.3f ms", (dirn == 0 ? c.xstr() : c.ystr()).c_str(), ms);
+						times += (times.empty() ? "" : ", ") + std::string(b);
+						if(ms < best) { best = ms; win = t; }
+					}
+					sum += best;
+				}
+				sc = sum < best_sum ? win : keep;
+				if(sum < best_sum) {
+					tune_cache_put("x|" + key, win.xstr());
+					tune_cache_put("y|" + key, win.ystr());
+				}
+				note += "pairs " + std::string(sum < best_sum ? win.str() : "slower") + " [" + times + "]; ";
 			}
 			sc.plane_x = pmax;
 			tune_notes[h.index] = (tune_notes[h.index].empty() ? "" : tune_notes[h.index] + ", ") + note;
@@ -1187,6 +1231,24 @@ struct Plan : PlanBase {
 		const double sc = sizeof(cx<R>);
 		const double fpb = (double)Gm.N * nsl * 4 * sc;
 		const ShiftParams* sp = h.shiftd.as<ShiftParams>();
+		if(CB && on_pairs(h)) {
+			// to T2b as pairs of slots, which the line solves of the slab work on
+			auto* F = reinterpret_cast<const cx<float>*>(Fp);
+			auto* A = reinterpret_cast<const cx<float>*>(CA);
+			auto* B = reinterpret_cast<const cx<float>*>(CB);
+			auto* T = reinterpret_cast<v4<float>*>(T2b);
+			if(!h.any_shift)
+				launch("phase_sync", fpb, [&] { k_phase_sync_pair<<<pgrid(Gm.N, nsl / 2), 256, 0, cs>>>(Gm, A, B, F, T); });
+			else {
+				const int nsh = two_shifts ? 2 : 1;
+				dim3 grid((unsigned)((Gm.Nx + SHT - 1) / SHT), (unsigned)((Gm.Ny + SHT - 1) / SHT), (unsigned)(nsl / 2));
+				size_t smem = (size_t)4 * (SHT + 6) * (SHT + 6) * sizeof(cx<float>);
+				launch("shift_fused", fpb + (double)Gm.N * (nsl / Gm.spg) * 6 * sc, [&] {
+					k_shift_pair<<<grid, 256, smem, cs>>>(Gm, slot0 / 2, sp, A, B, nsh, F, T);
+				});
+			}
+			return T2b;
+		}
 		if(!h.any_shift) {
 			launch("phase_sync", fpb, [&] {
 				k_phase_sync<R><<<pgrid(Gm.N, nsl), 256, 0, cs>>>(Gm, slot0, CA, CB, Fp);
@@ -1390,6 +1452,40 @@ struct Plan : PlanBase {
 		}
 	}
 
+	// Whether a sample's slabs run on pairs of slots (FP32).
+	bool no_pairs = false;  // the tuner's timings of the general kernels
+	bool on_pairs(const SampleHost& h) const { return sizeof(R) == sizeof(float) && !no_pairs && scfg[h.index].pairs(); }
+
+	// The line solves of a slab on pairs: x frame, then the transposed frame, two Woodbury iterates each.
+	void rec_adi_pairs(SampleHost& h, const Geom& Gm, int nsl, int ng, const cx<R>* C, cx<R>* Fp, cx<R>* Tb, cx<R>* T2b,
+			const cx<R>* xsrc, int only_dirn) {
+		typedef cx<float> cf;
+		const SolveCfg& c = scfg[h.index];
+		const double fp = (double)Gm.N * nsl * 2 * sizeof(cx<R>);
+		for(int dirn = 0; dirn < 2; dirn++) {
+			if(only_dirn >= 0 && dirn != only_dirn) continue;
+			const Geom G = dirn == 0 ? Gm : transposed(Gm);
+			const int M = dirn == 0 ? c.Mx : c.Mxt, W = dirn == 0 ? c.WPLx : c.WPLt;
+			const cf* co = reinterpret_cast<const cf*>(dirn == 0 ? C : ct_cur);
+			const cf* fa = reinterpret_cast<const cf*>(dirn == 0 ? fx_cur : fy_cur);
+			const cx<double>* ls = dirn == 0 ? lx_cur : ly_cur;
+			const size_t plane = dirn == 0 ? c.plane_x : c.plane_y;
+			auto solve = [&](const char* name, int passes, int kind, int out, const cx<R>* src, cx<R>* dst, const cx<R>* acc0, cx<R>* plain) {
+				const double bytes = fp * passes + (double)Gm.N * ng * (2 * NFAC * sizeof(cx<R>) + (kind == ST_WOOD_X ? 18 : 26) * sizeof(R));
+				launch(name, bytes, [&] {
+					if(!launch_solve_pair(cs, M, W, kind, out, G, ng, co, fa, plane, ls, reinterpret_cast<const cf*>(src),
+							reinterpret_cast<cf*>(dst), reinterpret_cast<const cf*>(acc0), reinterpret_cast<cf*>(plain)))
+						throw BackendError(E_INTERNAL, "no pair-solve instance");
+				});
+			};
+			const char* we = dirn == 0 ? "expl_solve_x" : "expl_solve_y";
+			const char* ww = dirn == 0 ? "wood_solve_x" : "wood_solve_y";
+			solve(we, 2, ST_EXPL_Y, PO_SAME, dirn == 0 ? xsrc : Fp, Tb, nullptr, nullptr);
+			solve(ww, 2, ST_WOOD_X, PO_SAME, Tb, T2b, nullptr, nullptr);
+			solve(ww, 3, ST_WOOD_X, dirn == 0 ? PO_TRANS : PO_PLAIN, T2b, Fp, Tb, Fp);
+		}
+	}
+
 	// ParaxialPrimaryEvolutionOperator::apply (ParaxialPrimaryEvolutionOperator.cpp:153-209).
 	// only_dirn >= 0: that direction's solves alone (the tuner's timing runs).
 	void rec_adi(SampleHost& h, const Geom& Gm, int slot0, int nsl, int ng, int Nw, const cx<R>* C, cx<R>* Fp,
@@ -1399,6 +1495,10 @@ struct Plan : PlanBase {
 		dim3 gr = pgrid(N, nsl);
 		const double fp = (double)N * nsl;
 		const SolveCfg& cfg = scfg[h.index];
+		if(on_pairs(h)) {
+			rec_adi_pairs(h, Gm, nsl, ng, C, Fp, Tb, T2b, xsrc, only_dirn);
+			return;
+		}
 		for(int dirn = 0; dirn < 2; dirn++) {
 			if(only_dirn >= 0 && dirn != only_dirn) continue;
 			bool fused = dirn == 0 ? cfg.Mx > 0 : (cfg.My > 0 || cfg.ys || cfg.yq > 0 || cfg.Mt > 0 || cfg.Mxt > 0);

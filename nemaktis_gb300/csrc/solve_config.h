@@ -74,6 +74,11 @@ struct SolveCfg {
 	// x on k_solve_xc or k_solve_xw: the kernels whose last Woodbury solve can hand the fields over
 	// to the transposed frame
 	bool x_hands_over() const { return Mx > 0 && !xs; }
+	// Both directions partitioned with two slots per thread: in FP32 they run on pairs of slots
+	// (pair_kernels.cuh).
+	bool pair_x() const { return x_hands_over() && KSx == 2 && Mx <= 8; }
+	bool pair_y() const { return Mxt > 0 && KSy == 2 && Mxt <= 8; }
+	bool pairs() const { return pair_x() && pair_y(); }
 };
 
 // What the choice depends on.
@@ -94,7 +99,7 @@ struct SolveShape {
 // Elements per factor plane of `lines` partitioned lines (part_line_size in bpm_kernels.cuh: 5 factors
 // per point and 8 interface coefficients per chunk).
 inline size_t part_plane(int lines, int M, int wpl) {
-	return ((size_t)lines * 32 * wpl * (5 * M + 8) + 4) / 5;
+	return ((size_t)lines * 32 * wpl * (5 * M + 8) + 4) / 5 + 1;
 }
 
 inline size_t plane_x_of(const SolveCfg& c, const SolveShape& s) {
@@ -105,9 +110,11 @@ inline size_t plane_x_of(const SolveCfg& c, const SolveShape& s) {
 }
 
 inline void finalize(SolveCfg& c, const SolveShape& s) {
-	c.plane_x = plane_x_of(c, s);
+	// even: the factors are read as 2-complex vectors
+	c.plane_x = (plane_x_of(c, s) + 1) & ~(size_t)1;
 	// transposed-frame y factors: the partitioned x layout of Nx lines
 	c.plane_y = std::max((size_t)s.Nx * s.Ny, c.Mxt ? part_plane(s.Nx, c.Mxt, c.WPLt) : (size_t)0);
+	c.plane_y = (c.plane_y + 1) & ~(size_t)1;
 }
 
 inline bool xs_fits(int ks, int M, const SolveShape& s) { return (size_t)4 * ks * 32 * (M + 1) * s.csize() <= 100 * 1024; }

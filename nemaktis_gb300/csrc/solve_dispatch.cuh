@@ -32,6 +32,12 @@ bool launch_solve_xw(const SolveLaunch& L, Geom G, int slot0, int nch, const cx<
 	size_t plane, const cx<double>* lsc, const cx<R>* src, cx<R>* dst, const cx<R>* ai, cx<R>* ao, const cx<R>* ai2 = nullptr);
 void set_solve_smem_xw_f32(int bytes);
 void set_solve_smem_xw_f64(int bytes);
+// FP32 pair solves (pair_kernels.cuh), M and warps per line W: kind ST_EXPL_Y (out PO_SAME) or ST_WOOD_X; src,
+// dst, acc0: pairs; plain: the plain planes of PO_PLAIN. Returns false if there is no instance.
+bool launch_solve_pair(cudaStream_t st, int M, int W, int kind, int out, Geom G, int ng, const cx<float>* coef,
+	const cx<float>* fac, size_t plane, const cx<double>* lsc, const cx<float>* src, cx<float>* dst, const cx<float>* acc0,
+	cx<float>* plain);
+void set_solve_smem_pair(int bytes);
 template <typename R>
 bool launch_solve_xs(const SolveLaunch& L, Geom G, int slot0, int nch, const cx<R>* coef, const cx<R>* fac,
 	size_t plane, const cx<double>* lsc, const cx<R>* src, cx<R>* dst, const cx<R>* ai, cx<R>* ao);
