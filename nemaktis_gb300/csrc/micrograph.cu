@@ -16,7 +16,11 @@
 //   filt      (Nl, Nq, Ny, Nx) complex  mask * filter^|zf| / (Nx Ny) for the current focus
 //   spectrum  (Ny, Nx, Nl) double
 // Focalisation = x-line FFT (vals -> focused), one fused kernel per y-line doing the forward
-// FFT, the filter product and the inverse FFT, then the inverse x-line FFT.
+// FFT, the filter product and the inverse FFT, then the inverse x-line FFT. Fourier columns that the
+// aperture excludes altogether (63 % of them at NA 0.41 and spacings of half a wavelength) are skipped by
+// the second and taken as zero by the third. Bound: the FP64 pipe (28 operations per point and pass). 256x256,
+// 4 wavelengths x 19 q: refocus and spectrum 6.5 ms with every column and 72 operations per wavevector in the
+// spectrum, 4.4 ms so.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -129,17 +133,37 @@ __global__ void k_focus_filter(long long N, int Nl, int Nq, double NA, double a,
 	filt[t] = f * scale;
 }
 
+// Which Fourier columns of a (wavelength, q) reach the aperture: (kx + px)^2 < (k0 NA)^2, rounded as in
+// k_objective_table, whose |k+p|^2 is not below (kx + px)^2 then either.
+__global__ void k_focus_keep(int Nx, int Nq, double dx, double NA, const double* __restrict__ wl,
+		const double* __restrict__ qv, unsigned char* __restrict__ keep) {
+	const int ix = blockIdx.x * blockDim.x + threadIdx.x, lq = blockIdx.y;
+	if(ix >= Nx) return;
+	double tx = __dsub_rn(fmod(__dadd_rn((double)ix, __dmul_rn(0.5, (double)Nx)), (double)Nx), __dmul_rn(0.5, (double)Nx));
+	double kx = __ddiv_rn(__dmul_rn(__dmul_rn(tx, 2.0), PI_NP), __dmul_rn((double)Nx, dx));
+	double k0 = __ddiv_rn(2.0 * PI_NP, wl[lq / Nq]);
+	double ax = __dadd_rn(kx, __dmul_rn(k0, qv[2 * (lq % Nq)]));
+	double kna = __dmul_rn(k0, NA);
+	keep[(size_t)lq * Nx + ix] = __dmul_rn(ax, ax) < __dmul_rn(kna, kna);
+}
+
 // One block transforms `lpb` y-lines (adjacent columns x of one plane (l, q, comp)): forward
 // FFT, product with the focus filter of (l, q), inverse FFT (unscaled; the scale is in filt).
 __global__ void k_focus_cols(cx<double>* F, FftPlan1D P, int nlines, int Nx, long long N, int lpb,
-		const cx<double>* __restrict__ tw, const cx<double>* __restrict__ filt) {
+		const cx<double>* __restrict__ tw, const cx<double>* __restrict__ filt, const unsigned char* __restrict__ keep) {
 	extern __shared__ unsigned char smem_raw[];
 	cx<double>* sA = reinterpret_cast<cx<double>*>(smem_raw);
 	const int n = P.n, pitch = n + 1;
 	cx<double>* sB = sA + (size_t)lpb * pitch;
+	cx<double>* wp = sB + (size_t)lpb * pitch;
 	int l0 = blockIdx.x * lpb;
 	int nl = min(lpb, nlines - l0);
 	if(nl <= 0) return;
+	// columns outside the objective's aperture: their filter is zero, and the backward row transforms take
+	// them as zero (keep null: every column)
+	bool any = !keep;
+	for(int i = 0; i < nl && !any; i++) any = keep[(size_t)((l0 + i) / Nx / 4) * Nx + (l0 + i) % Nx] != 0;
+	if(!any) return;
 	auto addr = [&](int line, int i) {
 		return (long long)(line / Nx) * N + (long long)i * Nx + (line % Nx);
 	};
@@ -149,7 +173,7 @@ __global__ void k_focus_cols(cx<double>* F, FftPlan1D P, int nlines, int Nx, lon
 		sA[li * pitch + i] = F[addr(l0 + li, i)];
 	}
 	__syncthreads();
-	cx<double>* res = fft_stages<double>(sA, sB, P, nl, tw, -1);
+	cx<double>* res = fft_stages<double>(sA, sB, P, nl, tw, -1, wp);
 	for(int e = threadIdx.x; e < tot; e += blockDim.x) {
 		int li = e % nl, i = e / nl;
 		int line = l0 + li;
@@ -157,7 +181,7 @@ __global__ void k_focus_cols(cx<double>* F, FftPlan1D P, int nlines, int Nx, lon
 		res[li * pitch + i] = res[li * pitch + i] * filt[lq * N + (long long)i * Nx + (line % Nx)];
 	}
 	__syncthreads();
-	cx<double>* res2 = fft_stages<double>(res, res == sA ? sB : sA, P, nl, tw, +1);
+	cx<double>* res2 = fft_stages<double>(res, res == sA ? sB : sA, P, nl, tw, +1, wp);
 	for(int e = threadIdx.x; e < tot; e += blockDim.x) {
 		int li = e % nl, i = e / nl;
 		F[addr(l0 + li, i)] = res2[li * pitch + i];
@@ -173,8 +197,13 @@ __global__ void k_spectrum(const cx<double>* __restrict__ F, long long N, int Nl
 	long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	int l = blockIdx.y;
 	if(p >= N) return;
-	cx<double> A[4], B[4];
-	for(int i = 0; i < 4; i++) { A[i] = pre[4 * l + i]; B[i] = post[4 * l + i]; }
+	// || B T A ||^2 = sum_ab P_ab t_a^H G t_b over the columns t_0 = (v0, v1), t_1 = (v2, v3) of T, with the
+	// Hermitian G = B^H B and P = A A^H: 48 instead of 72 FP64 operations per wavevector
+	const cx<double>*A = pre + 4 * l, *B = post + 4 * l;
+	const double G00 = norm2(B[0]) + norm2(B[2]), G11 = norm2(B[1]) + norm2(B[3]);
+	const cx<double> G01 = conj(B[0]) * B[1] + conj(B[2]) * B[3];
+	const double P00 = norm2(A[0]) + norm2(A[1]), P11 = norm2(A[2]) + norm2(A[3]);
+	const cx<double> P10 = A[2] * conj(A[0]) + A[3] * conj(A[1]);
 	double acc = 0;
 	for(int k = 0; k < nw; k++) {
 		const cx<double>* f = F + ((long long)(l * Nq + q_start + k) * 4) * N + p;
@@ -182,12 +211,12 @@ __global__ void k_spectrum(const cx<double>* __restrict__ F, long long N, int Nl
 		double s;
 		if(plain) s = norm2(v0) + norm2(v1) + norm2(v2) + norm2(v3);
 		else {
-			// T = [[v0, v2], [v1, v3]]; X = T . pre; Y = post . X
-			cx<double> x00 = v0 * A[0] + v2 * A[2], x01 = v0 * A[1] + v2 * A[3];
-			cx<double> x10 = v1 * A[0] + v3 * A[2], x11 = v1 * A[1] + v3 * A[3];
-			cx<double> y00 = B[0] * x00 + B[1] * x10, y01 = B[0] * x01 + B[1] * x11;
-			cx<double> y10 = B[2] * x00 + B[3] * x10, y11 = B[2] * x01 + B[3] * x11;
-			s = norm2(y00) + norm2(y01) + norm2(y10) + norm2(y11);
+			const cx<double> u0 = cfma(G01, v1, G00 * v0), u1 = cfma(conj(G01), v0, G11 * v1);  // G t_0
+			const cx<double> w0 = cfma(G01, v3, G00 * v2), w1 = cfma(conj(G01), v2, G11 * v3);  // G t_1
+			const double s0 = v0.x * u0.x + v0.y * u0.y + v1.x * u1.x + v1.y * u1.y;
+			const double s1 = v2.x * w0.x + v2.y * w0.y + v3.x * w1.x + v3.y * w1.y;
+			const cx<double> x = cfma(conj(v1), w1, conj(v0) * w0);  // t_0^H G t_1
+			s = P00 * s0 + P11 * s1 + 2 * (P10.x * x.x - P10.y * x.y);
 		}
 		acc += w[k] * (0.5 * s);
 	}
@@ -304,7 +333,7 @@ struct Microscope {
 	size_t smem_limit = 0;
 	cudaStream_t st = nullptr;
 	cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-	Buf dwl, dnout, dqv, tab, filt, vals, foc, spec, dw, dpre, dpost, twx, twy;
+	Buf dwl, dnout, dqv, tab, filt, keep, vals, foc, spec, dw, dpre, dpost, twx, twy;
 	size_t nw_cap = 0;
 	float focus_ms = 0, spectrum_ms = 0;
 	long long bytes = 0;
@@ -392,6 +421,7 @@ struct Microscope {
 		dqv.alloc(sizeof(double) * qv.size());
 		tab.alloc(sizeof(double2) * nlq);
 		filt.alloc(sizeof(cx<double>) * nlq);
+		keep.alloc((size_t)Nl * Nq * Nx);
 		vals.alloc(sizeof(cx<double>) * nvals());
 		foc.alloc(sizeof(cx<double>) * nvals());
 		spec.alloc(sizeof(double) * N * Nl);
@@ -414,17 +444,19 @@ struct Microscope {
 	}
 
 	// x-line FFT of every plane, from src (null: in place) into foc.
-	void fft_rows(const cx<double>* src, int sign) {
+	void fft_rows(const cx<double>* src, int sign, const unsigned char* kp = nullptr) {
 		FftPlan1D px;
 		fft_plan_1d(Nx, px);
+		fft_fit<double>(px, smem_limit);
 		size_t per_line = 2 * (size_t)(Nx + 1) * sizeof(cx<double>);
+		const size_t limit = smem_limit - fft_smem<double>(px, 0);
 		int lpb = (int)std::max<size_t>(1, std::min<size_t>(64, (size_t)(48 * 1024) / per_line));
-		lpb = std::max(1, std::min(lpb, (int)(smem_limit / per_line)));
+		lpb = std::max(1, std::min(lpb, (int)(limit / per_line)));
 		int nlines = Nl * Nq * 4 * Ny;
 		int blocks = (nlines + lpb - 1) / lpb;
 		int threads = std::min(256, std::max(32, ((lpb * Nx / 2) + 31) / 32 * 32));
-		k_fft_lines<double><<<blocks, threads, per_line * lpb, st>>>(foc.as<cx<double>>(), src, px, nlines, Ny, N,
-			Nx, 1, lpb, twx.as<cx<double>>(), sign);
+		k_fft_lines<double><<<blocks, threads, fft_smem<double>(px, lpb), st>>>(foc.as<cx<double>>(), src, px, nlines, Ny, N,
+			Nx, 1, lpb, twx.as<cx<double>>(), sign, kp);
 	}
 
 	void focus(double z_focus, double NA_obj) {
@@ -442,14 +474,18 @@ struct Microscope {
 		else MCK(cudaMemcpyAsync(foc.p, vals.p, sizeof(cx<double>) * nvals(), cudaMemcpyDeviceToDevice, st));
 		FftPlan1D py;
 		fft_plan_1d(Ny, py);
+		fft_fit<double>(py, smem_limit);
 		size_t per_line = 2 * (size_t)(Ny + 1) * sizeof(cx<double>);
-		int lpb = (int)std::max<size_t>(1, std::min<size_t>(16, smem_limit / per_line));
+		int lpb = (int)std::max<size_t>(1, std::min<size_t>(16, (smem_limit - fft_smem<double>(py, 0)) / per_line));
+		unsigned char* kp = Nx > 1 ? keep.as<unsigned char>() : nullptr;  // one column: no row transforms
+		if(kp) k_focus_keep<<<dim3((unsigned)((Nx + 127) / 128), (unsigned)(Nl * Nq)), 128, 0, st>>>(Nx, Nq, dx, NA, dwl.as<double>(),
+			dqv.as<double>(), kp);
 		int nlines = Nl * Nq * 4 * Nx;
 		int blocks = (nlines + lpb - 1) / lpb;
 		int threads = std::min(256, std::max(32, ((lpb * Ny / 2) + 31) / 32 * 32));
-		k_focus_cols<<<blocks, threads, per_line * lpb, st>>>(foc.as<cx<double>>(), py, nlines, Nx, N, lpb,
-			twy.as<cx<double>>(), filt.as<cx<double>>());
-		if(Nx > 1) fft_rows(nullptr, +1);
+		k_focus_cols<<<blocks, threads, fft_smem<double>(py, lpb), st>>>(foc.as<cx<double>>(), py, nlines, Nx, N, lpb,
+			twy.as<cx<double>>(), filt.as<cx<double>>(), kp);
+		if(Nx > 1) fft_rows(nullptr, +1, kp);
 		MCK(cudaGetLastError());
 		MCK(cudaEventRecord(ev[1], st));
 		MCK(cudaEventSynchronize(ev[1]));

@@ -151,7 +151,7 @@ struct SampleHost {
 	std::vector<double> bulk_data;
 	cx<double>* hstage = nullptr;  // pinned host staging of one pass's plane
 	// device
-	DevBuf dir, dmask, dwts, F, E0, gpsd, shiftd, partial, wl, nout, qv, bstage;
+	DevBuf dir, dmask, dwts, F, E0, gpsd, shiftd, partial, wl, nout, qv, keep, bstage;
 	// The sample's lane: its own streams (sample 0 uses the plan's), events and workspace, so that
 	// the samples of a batch run side by side on the device, each in its own branch of the graph.
 	struct Lane {
@@ -484,6 +484,7 @@ struct Plan : PlanBase {
 		smem_limit = (size_t)optin;
 		CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
 		CK(cudaFuncSetAttribute(k_fft_lines<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit));
+		CK(cudaFuncSetAttribute(k_screen_cols<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit));
 		CK(cudaFuncSetAttribute(k_factor_chunked<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)((size_t)16 * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>))));
 		CK(cudaFuncSetAttribute(k_shift_fused<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -583,6 +584,7 @@ struct Plan : PlanBase {
 			dalloc(h.wl, sizeof(double) * h.G);
 			dalloc(h.nout, sizeof(double) * h.G);
 			dalloc(h.qv, sizeof(double) * 2 * h.Nq);
+			dalloc(h.keep, (size_t)h.G * h.Nq * h.s.Nx);
 			if(h.bulk) {
 				size_t nb = sizeof(cx<double>) * (size_t)ng * h.spg * 2 * N;
 				dalloc(h.bstage, nb);
@@ -897,20 +899,24 @@ struct Plan : PlanBase {
 	// ---- launch helpers (count launches while recording) ----
 	dim3 pgrid(int N, int ny, int threads = 256) { return dim3((unsigned)((N + threads - 1) / threads), (unsigned)ny); }
 
-	void fft2(SampleHost& h, cx<R>* F, int nplanes, int sign) {
+	// passes: bit 0 rows, bit 1 columns; keep: see k_fft_lines (rows)
+	void fft2(SampleHost& h, cx<R>* F, int nplanes, int sign, int passes = 3, const unsigned char* keep = nullptr) {
 		int Nx = h.s.Nx, Ny = h.s.Ny;
 		for(int pass = 0; pass < 2; pass++) {
+			if(!(passes >> pass & 1)) continue;
 			int n = pass == 0 ? Nx : Ny;
 			if(n == 1) continue;
 			FftPlan1D P;
 			if(!fft_plan_1d(n, P)) throw BackendError(E_INTERNAL, "FFT plan too deep");
+			fft_fit<R>(P, smem_limit);
 			size_t per_line = 2 * (size_t)(n + 1) * sizeof(cx<R>);
+			const size_t table = fft_smem<R>(P, 0), limit = smem_limit - table;
 			if(per_line > smem_limit)
 				throw BackendError(E_SETTINGS, "FFT line length " + std::to_string(n) + " exceeds shared memory");
 			int lpb = (int)std::max<size_t>(1, std::min<size_t>(64, (size_t)(48 * 1024) / per_line));
-			if(pass == 1) lpb = std::max(lpb, std::min(16, (int)(smem_limit / per_line)));
-			lpb = std::max(1, std::min(lpb, (int)(smem_limit / per_line)));
-			size_t smem = per_line * lpb;
+			if(pass == 1) lpb = std::max(lpb, std::min(16, (int)(limit / per_line)));
+			lpb = std::max(1, std::min(lpb, (int)(limit / per_line)));
+			size_t smem = fft_smem<R>(P, lpb);
 			int nlines, lpp;
 			long long ps = (long long)Nx * Ny, ls, es;
 			if(pass == 0) { nlines = nplanes * Ny; lpp = Ny; ls = Nx; es = 1; }
@@ -920,7 +926,8 @@ struct Plan : PlanBase {
 			cx<R>* tw = twiddles(n);
 			double bytes = 2.0 * sizeof(cx<R>) * (double)nplanes * Nx * Ny;
 			launch(pass == 0 ? "fft_rows" : "fft_cols", bytes, [&] {
-				k_fft_lines<R><<<blocks, threads, smem, cs>>>(F, nullptr, P, nlines, lpp, ps, ls, es, lpb, tw, sign);
+				k_fft_lines<R><<<blocks, threads, smem, cs>>>(F, nullptr, P, nlines, lpp, ps, ls, es, lpb, tw, sign,
+					pass == 0 ? keep : nullptr);
 			});
 		}
 	}
@@ -1142,6 +1149,33 @@ struct Plan : PlanBase {
 		const double sc = sizeof(cx<R>);
 		cx<R>* F = h.F.as<cx<R>>();
 		int nplanes = h.slots * 2;
+		// the y half in one pass where the two components of at least one 32-byte segment of columns fit in
+		// shared memory (up to about 3500 rows)
+		FftPlan1D P;
+		if(h.s.Nx > 1 && h.s.Ny > 1 && fft_plan_1d(h.s.Ny, P)) {
+			const int least = (int)(32 / sc);
+			int nc = 4 * least;  // 128-byte segments while two blocks share an SM
+			auto bytes = [&](int c) { return fft_smem<R>(P, 2 * c) + sizeof(cx<R>) + sizeof(double) * (size_t)(h.s.Ny + c); };
+			while(nc > least && 2 * bytes(nc) > smem_limit) nc /= 2;
+			const size_t smem = bytes(nc);
+			if(smem <= smem_limit) {
+				const int Nx = h.s.Nx, Ny = h.s.Ny, gq = h.G * h.Nq;
+				unsigned char* keep = h.keep.template as<unsigned char>();
+				launch("screen_keep", (double)Nx * gq, [&] {
+					k_screen_keep<<<dim3((unsigned)((Nx + 127) / 128), (unsigned)gq), 128, 0, cs>>>(h.sp, h.wl.template as<double>(),
+						h.qv.template as<double>(), keep);
+				});
+				fft2(h, F, nplanes, -1, 1);
+				cx<R>* tw = twiddles(Ny);
+				const int threads = std::min(512, std::max(64, (2 * nc * Ny / 4 + 31) / 32 * 32));
+				launch("screen_cols", (double)N * h.slots * 4 * sc, [&] {
+					k_screen_cols<R><<<dim3((unsigned)((Nx + nc - 1) / nc), (unsigned)h.slots), threads, smem, cs>>>(F, h.sp, P, nc, tw,
+						h.wl.template as<double>(), h.nout.template as<double>(), h.qv.template as<double>(), keep);
+				});
+				fft2(h, F, nplanes, +1, 1, keep);
+				return;
+			}
+		}
 		fft2(h, F, nplanes, -1);
 		launch("screen_filter", (double)N * h.slots * 4 * sc, [&] {
 			k_screen_filter<R><<<pgrid(N, h.G * h.Nq, 128), 128, 0, cs>>>(F, h.sp, 0, h.wl.as<double>(),
