@@ -1361,6 +1361,7 @@ struct Plan : PlanBase {
 		double bytes = fp * (reads + writes) + (double)Gm.N * ng * (2 * NFAC * sz + (wood ? 18 : 26) * sizeof(R));
 		SolveLaunch L;
 		L.stream = cs;
+		L.dep = dirn == 1 || wood;  // a slab's first solve also waits for the factorisation
 		if(dirn == 0) {
 			L.M = sc.Mx; L.kind = wood ? ST_WOOD_X : ST_EXPL_Y;
 			const int LT = 4;
@@ -1504,10 +1505,11 @@ struct Plan : PlanBase {
 			const cf* fa = reinterpret_cast<const cf*>(dirn == 0 ? fx_cur : fy_cur);
 			const cx<double>* ls = dirn == 0 ? lx_cur : ly_cur;
 			const size_t plane = dirn == 0 ? c.plane_x : c.plane_y;
+			// every solve but a slab's first (which also waits for the factorisation) depends on the one before alone
 			auto solve = [&](const char* name, int passes, int kind, int out, const cx<R>* src, cx<R>* dst, const cx<R>* acc0, cx<R>* plain) {
 				const double bytes = fp * passes + (double)Gm.N * ng * (2 * NFAC * sizeof(cx<R>) + (kind == ST_WOOD_X ? 18 : 26) * sizeof(R));
 				launch(name, bytes, [&] {
-					if(!launch_solve_pair(cs, M, W, kind, out, G, ng, co, fa, plane, ls, reinterpret_cast<const cf*>(src),
+					if(!launch_solve_pair(cs, dirn == 1 || kind == ST_WOOD_X, M, W, kind, out, G, ng, co, fa, plane, ls, reinterpret_cast<const cf*>(src),
 							reinterpret_cast<cf*>(dst), reinterpret_cast<const cf*>(acc0), reinterpret_cast<cf*>(plain)))
 						throw BackendError(E_INTERNAL, "no pair-solve instance");
 				});

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 		const cx<float>* __restrict__ fac, size_t plane, const cx<double>* __restrict__ lsc, const pr* __restrict__ src,
 		pr* __restrict__ dst, const pr* __restrict__ acc0, cx<float>* __restrict__ plain) {
 	extern __shared__ unsigned char smem_raw[];
+	wait_predecessor();
 	constexpr int LT = 4;
 	// 16-byte entries per warp; the warps' buffers 2 entries apart modulo 8: no bank conflicts when the
 	// block reads one point of its 4 lines
@@ -245,6 +246,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 		const cx<float>* __restrict__ fac, size_t plane, const cx<double>* __restrict__ lsc, const pr* __restrict__ src,
 		pr* __restrict__ dst, const pr* __restrict__ acc0, cx<float>* __restrict__ plain) {
 	extern __shared__ unsigned char smem_raw[];
+	wait_predecessor();
 	constexpr int LT = 2;
 	const int CH = 32 * W, WS = CH * (M + 1) + 4;  // the two lines' buffers 4 entries apart modulo 8
 	pr* const bufs = reinterpret_cast<pr*>(smem_raw);

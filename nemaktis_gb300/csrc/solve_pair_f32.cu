@@ -12,7 +12,7 @@ namespace nbpm {
 #define NBPM_XWP_ALL(F) \
 	F(8, ST_EXPL_Y, PO_SAME) F(8, ST_WOOD_X, PO_SAME) F(8, ST_WOOD_X, PO_TRANS) F(8, ST_WOOD_X, PO_PLAIN)
 
-bool launch_solve_pair(cudaStream_t st, int M, int W, int kind, int out, Geom G, int ng, const cx<float>* coef,
+bool launch_solve_pair(cudaStream_t st, bool dep, int M, int W, int kind, int out, Geom G, int ng, const cx<float>* coef,
 		const cx<float>* fac, size_t plane, const cx<double>* lsc, const cx<float>* src, cx<float>* dst, const cx<float>* acc0,
 		cx<float>* plain) {
 	const pr* s = reinterpret_cast<const pr*>(src);
@@ -23,7 +23,7 @@ bool launch_solve_pair(cudaStream_t st, int M, int W, int kind, int out, Geom G,
 		const size_t smem = (size_t)4 * (32 * (M + 1) + 2) * sizeof(pr);
 #define NBPM_XP(MM, KD, OO) \
 		if(M == MM && kind == KD && out == OO) { \
-			k_solve_xp<MM, KD, OO><<<grid, 128, smem, st>>>(G, coef, fac, plane, lsc, s, d, a, plain); \
+			launch_dep(dep, k_solve_xp<MM, KD, OO>, grid, dim3(128), smem, st, G, coef, fac, plane, lsc, s, d, a, plain); \
 			return true; \
 		}
 		NBPM_XP_ALL(NBPM_XP)
@@ -38,7 +38,7 @@ bool launch_solve_pair(cudaStream_t st, int M, int W, int kind, int out, Geom G,
 	const int regs = W > 2 ? 64 : (size_t)grid.x * grid.y * 4 <= (size_t)152 * 20 ? 96 : 72;
 #define NBPM_XWP_R(MM, KD, OO, RR) \
 	if(M == MM && kind == KD && out == OO && regs == RR) { \
-		k_solve_xwp<MM, KD, OO, RR><<<grid, 64 * W, smem, st>>>(G, W, coef, fac, plane, lsc, s, d, a, plain); \
+		launch_dep(dep, k_solve_xwp<MM, KD, OO, RR>, grid, dim3((unsigned)(64 * W)), smem, st, G, W, coef, fac, plane, lsc, s, d, a, plain); \
 		return true; \
 	}
 #define NBPM_XWP(MM, KD, OO) NBPM_XWP_R(MM, KD, OO, 64) NBPM_XWP_R(MM, KD, OO, 72) NBPM_XWP_R(MM, KD, OO, 96)

@@ -5,12 +5,12 @@ namespace nbpm {
 
 #define NBPM_XC(MM, KK, KD) \
 	if(L.M == MM && L.KS == KK && L.kind == KD && !L.tout) { \
-		k_solve_xc<float, MM, KD, KK><<<L.grid, L.block, L.smem, L.stream>>>(G, slot0, nch, coef, fac, plane, lsc, \
+		launch_dep(L.dep, k_solve_xc<float, MM, KD, KK>, L.grid, L.block, L.smem, L.stream, G, slot0, nch, coef, fac, plane, lsc, \
 			src, dst, ai, ao, ai2); \
 		return true; \
 	} \
 	if(L.M == MM && L.KS == KK && L.kind == KD && L.tout && KD == ST_WOOD_X) { \
-		k_solve_xc<float, MM, ST_WOOD_X, KK, true><<<L.grid, L.block, L.smem, L.stream>>>(G, slot0, nch, coef, fac, plane, \
+		launch_dep(L.dep, k_solve_xc<float, MM, ST_WOOD_X, KK, true>, L.grid, L.block, L.smem, L.stream, G, slot0, nch, coef, fac, plane, \
 			lsc, src, dst, ai, ao, ai2); \
 		return true; \
 	}
@@ -67,12 +67,12 @@ void set_solve_smem_xs_f32(int bytes) {
 
 #define NBPM_XW(KK, KD) \
 	if(L.M == 8 && L.KS == KK && L.kind == KD && !L.tout) { \
-		k_solve_xw<float, 8, KD, KK><<<L.grid, L.block, L.smem, L.stream>>>(G, slot0, nch, coef, fac, plane, lsc, \
+		launch_dep(L.dep, k_solve_xw<float, 8, KD, KK>, L.grid, L.block, L.smem, L.stream, G, slot0, nch, coef, fac, plane, lsc, \
 			src, dst, ai, ao, ai2); \
 		return true; \
 	} \
 	if(L.M == 8 && L.KS == KK && L.kind == KD && L.tout && KD == ST_WOOD_X) { \
-		k_solve_xw<float, 8, ST_WOOD_X, KK, true><<<L.grid, L.block, L.smem, L.stream>>>(G, slot0, nch, coef, fac, plane, \
+		launch_dep(L.dep, k_solve_xw<float, 8, ST_WOOD_X, KK, true>, L.grid, L.block, L.smem, L.stream, G, slot0, nch, coef, fac, plane, \
 			lsc, src, dst, ai, ao, ai2); \
 		return true; \
 	}
