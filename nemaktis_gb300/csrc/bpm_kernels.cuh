@@ -107,6 +107,7 @@ struct GroupParams {
 	double no, ne, ne_imag, nhost, nin, nout_fresnel;
 	double absorp_im;  // imaginary part of 1 + i*ne_imag/(ne-no)
 	double nref;
+	double rX, rY, rXX, rYY, rXY;  // 1/dX, 1/dY, 1/dX^2, 1/dY^2, 1/(dX dY)
 };
 
 struct ShiftParams {
@@ -243,36 +244,41 @@ static __global__ void k_eps_plane(const double* __restrict__ dir, int fd, const
 			e0 = ei + a * (float)d[0]; e1 = ei + a * (float)d[1]; e2 = ei + a * (float)d[2];
 			e3 = a * (float)d[3]; e4 = a * (float)d[4]; e5 = a * (float)d[5];
 		}
-		float xx = e0 - (e4 * e4) / e2, yy = e1 - (e5 * e5) / e2, xy = e3 - e4 * e5 / e2;
+		const float rz = 1.f / e2, vx = e4 * rz, vy = e5 * rz;
+		float xx = e0 - e4 * vx, yy = e1 - e5 * vy, xy = e3 - e4 * vy;
 		float det = xx * yy - xy * xy, tr = 0.5f * (xx + yy), ne;
 		if(tr * tr - det < 1e-8f) ne = sqrtf(tr);
 		else { float r = sqrtf(tr * tr - det); ne = (sqrtf(tr + r) + sqrtf(tr - r)) / 2.f; }
+		const float rn = 0.25f / ne;
 		o[Q_XXTR * N] = (Q)xx;
 		o[Q_YYTR * N] = (Q)yy;
 		o[Q_XYTR * N] = (Q)xy;
-		o[Q_XXS * N] = (Q)(ne + (xx - yy) / (4 * ne));
-		o[Q_YYS * N] = (Q)(ne + (yy - xx) / (4 * ne));
-		o[Q_XYS * N] = (Q)(xy / (2 * ne));
-		o[Q_VX * N] = (Q)(e4 / e2);
-		o[Q_VY * N] = (Q)(e5 / e2);
-		o[Q_IZZ * N] = (Q)(1.f / e2);
+		o[Q_XXS * N] = (Q)(ne + (xx - yy) * rn);
+		o[Q_YYS * N] = (Q)(ne + (yy - xx) * rn);
+		o[Q_XYS * N] = (Q)(xy * (2 * rn));
+		o[Q_VX * N] = (Q)vx;
+		o[Q_VY * N] = (Q)vy;
+		o[Q_IZZ * N] = (Q)rz;
 		return;
 	}
 	double e[6];
 	eps_voxel(dir + v * fd, fd, m, gp, e);
-	double xxtr = e[0] - (e[4] * e[4]) / e[2];
-	double yytr = e[1] - (e[5] * e[5]) / e[2];
-	double xytr = e[3] - e[4] * e[5] / e[2];
+	// one division by eps_zz and one by neff: an FP64 division costs about ten multiplications
+	const double rz = 1. / e[2], vx = e[4] * rz, vy = e[5] * rz;
+	double xxtr = e[0] - e[4] * vx;
+	double yytr = e[1] - e[5] * vy;
+	double xytr = e[3] - e[4] * vy;
 	double neff = neff_of(xxtr, yytr, xytr);
+	const double rn = 0.25 / neff;
 	o[Q_XXTR * N] = (Q)xxtr;
 	o[Q_YYTR * N] = (Q)yytr;
 	o[Q_XYTR * N] = (Q)xytr;
-	o[Q_XXS * N] = (Q)(neff + (xxtr - yytr) / (4 * neff));
-	o[Q_YYS * N] = (Q)(neff + (yytr - xxtr) / (4 * neff));
-	o[Q_XYS * N] = (Q)(xytr / (2 * neff));
-	o[Q_VX * N] = (Q)(e[4] / e[2]);
-	o[Q_VY * N] = (Q)(e[5] / e[2]);
-	o[Q_IZZ * N] = (Q)(1. / e[2]);
+	o[Q_XXS * N] = (Q)(neff + (xxtr - yytr) * rn);
+	o[Q_YYS * N] = (Q)(neff + (yytr - xxtr) * rn);
+	o[Q_XYS * N] = (Q)(xytr * (2 * rn));
+	o[Q_VX * N] = (Q)vx;
+	o[Q_VY * N] = (Q)vy;
+	o[Q_IZZ * N] = (Q)rz;
 }
 
 // Partial sums of neff over the volume for nref (PermittivityTensorField.cpp:183-211),
@@ -293,9 +299,10 @@ static __global__ void k_neff_partial(const double* __restrict__ dir, int fd, co
 		}
 		double e[6];
 		eps_voxel(dir + v * fd, fd, mask ? mask[v] != 0 : true, gp, e);
-		double xxtr = e[0] - (e[4] * e[4]) / e[2];
-		double yytr = e[1] - (e[5] * e[5]) / e[2];
-		double xytr = e[3] - e[4] * e[5] / e[2];
+		const double rz = 1. / e[2];
+		double xxtr = e[0] - (e[4] * e[4]) * rz;
+		double yytr = e[1] - (e[5] * e[5]) * rz;
+		double xytr = e[3] - e[4] * e[5] * rz;
 		acc += neff_of(xxtr, yytr, xytr);
 	}
 	sh[threadIdx.x] = acc;
@@ -334,7 +341,8 @@ struct CoefCtx {
 	__device__ __forceinline__ void sinv(int x, int y, T& ixx, T& iyy, T& ixy) const {
 		T exx = avg(Q_XXS, x, y), eyy = avg(Q_YYS, x, y), exy = avg(Q_XYS, x, y);
 		T det = exx * eyy - exy * exy;
-		ixx = eyy / det; iyy = exx / det; ixy = -exy / det;
+		const T r = (T)1 / det;
+		ixx = eyy * r; iyy = exx * r; ixy = -exy * r;
 	}
 	// One stencil entry of mu*R for the 4 blocks (00, 01, 10, 11). D is the real 2x2 entry
 	// of D at this (row, column) pair; dd is the first-derivative weight of the walk-off
@@ -383,7 +391,16 @@ __device__ __forceinline__ void phase_op(const T* A, const T* B, int N, int p, T
 	cx<T> a = mk<T>((T)1, (T)gp.absorp_im);
 	cx<T> sinc = mk<T>((T)1, (T)0);
 	cx<T> e, c;
-	if(sizeof(T) == sizeof(double)) {
+	if(gp.absorp_im == 0) {
+		// no absorption: the imaginary parts vanish (sinh 0, cosh 0 below)
+		T s, co, se, ce;
+		if(sizeof(T) == sizeof(double)) { double a_, b_; sincos((double)det, &a_, &b_); s = (T)a_; co = (T)b_; sincos((double)tr, &a_, &b_); se = (T)a_; ce = (T)b_; }
+		else { float a_, b_; sincosf((float)det, &a_, &b_); s = (T)a_; co = (T)b_; sincosf((float)tr, &a_, &b_); se = (T)a_; ce = (T)b_; }
+		if(!(fabs(det) < (T)1e-8)) sinc = mk<T>(s / det, (T)0);
+		e = mk<T>(ce, se);
+		c = mk<T>(co, (T)0);
+	}
+	else if(sizeof(T) == sizeof(double)) {
 		cx<double> ad = cvt<double>(a);
 		if(!(fabs((double)det) < 1e-8)) {
 			cx<double> sn = csin_d((double)det * ad);
@@ -439,7 +456,7 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 	X.sinv(ix, iy, X.rxx, X.ryy, X.rxy);
 	X.va0 = X.vsum(0, ix, iy);
 	X.va1 = X.vsum(1, ix, iy);
-	const T dX = (T)gp.dX, dY = (T)gp.dY;
+	const T rX = (T)gp.rX, rY = (T)gp.rY, rXX = (T)gp.rXX, rYY = (T)gp.rYY, rXY = (T)gp.rXY;
 	auto ezz = [&](int x, int y) { int i = x + Nx * y; return (A[Q_IZZ * N + i] + B[Q_IZZ * N + i]) / (T)2; };
 	T e0 = ezz(ix, iy);
 	int pxq = (ix == Nx - 1) ? 1 : ix + 1, mxq = (ix == 0) ? Nx - 2 : ix - 1;
@@ -454,14 +471,14 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		bool ok = Nx > 3 && ix < Nx - 1;
 		T cm = 0, cp = 0, c0 = 0;
 		if(ok) {
-			cm = (T)0.5 * (ezz(mxq, iy) + e0) / (dX * dX);
-			cp = (T)0.5 * (ezz(pxq, iy) + e0) / (dX * dX);
+			cm = (T)0.5 * (ezz(mxq, iy) + e0) * rXX;
+			cp = (T)0.5 * (ezz(pxq, iy) + e0) * rXX;
 			c0 = -cm - cp;
 		}
 		const int cols[3] = {mxs, ix, pxs};
 		const T c1[3] = {cm, c0, cp};
-		const T L[3] = {(T)1 / (dX * dX), (T)-2 / (dX * dX), (T)1 / (dX * dX)};
-		const T dd[3] = {(T)-0.5 / dX, 0, (T)0.5 / dX};
+		const T L[3] = {rXX, (T)-2 * rXX, rXX};
+		const T dd[3] = {(T)-0.5 * rX, 0, (T)0.5 * rX};
 #pragma unroll
 		for(int k = 0; k < 3; k++) {
 			if(ok) {
@@ -481,14 +498,14 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		bool ok = Ny > 3 && iy < Ny - 1;
 		T cm = 0, cp = 0, c0 = 0;
 		if(ok) {
-			cp = (T)0.5 * (ezz(ix, pyq) + e0) / (dY * dY);
-			cm = (T)0.5 * (ezz(ix, myq) + e0) / (dY * dY);
+			cp = (T)0.5 * (ezz(ix, pyq) + e0) * rYY;
+			cm = (T)0.5 * (ezz(ix, myq) + e0) * rYY;
 			c0 = -cm - cp;
 		}
 		const int rows[3] = {mys, iy, pys};
 		const T c1[3] = {cm, c0, cp};
-		const T L[3] = {(T)1 / (dY * dY), (T)-2 / (dY * dY), (T)1 / (dY * dY)};
-		const T dd[3] = {(T)-0.5 / dY, 0, (T)0.5 / dY};
+		const T L[3] = {rYY, (T)-2 * rYY, rYY};
+		const T dd[3] = {(T)-0.5 * rY, 0, (T)0.5 * rY};
 #pragma unroll
 		for(int k = 0; k < 3; k++) {
 			if(ok) {
@@ -509,10 +526,10 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		T a1 = 0, c1 = 0, a2 = 0, c2 = 0;
 		const T q4 = (T)0.25;
 		if(ok) {
-			a1 = q4 * ezz(pxq, iy) / (dX * dY); c1 = q4 * ezz(mxq, iy) / (dX * dY);
-			a2 = q4 * ezz(ix, pyq) / (dX * dY); c2 = q4 * ezz(ix, myq) / (dX * dY);
+			a1 = q4 * ezz(pxq, iy) * rXY; c1 = q4 * ezz(mxq, iy) * rXY;
+			a2 = q4 * ezz(ix, pyq) * rXY; c2 = q4 * ezz(ix, myq) * rXY;
 		}
-		const T g0[4] = {-q4 / (dX * dY), q4 / (dX * dY), q4 / (dX * dY), -q4 / (dX * dY)};
+		const T g0[4] = {-q4 * rXY, q4 * rXY, q4 * rXY, -q4 * rXY};
 		const T d01[4] = {a1, -c1, -a1, c1};
 		const T d10[4] = {a2, -a2, -c2, c2};
 		const int cxs[4] = {pxs, mxs, pxs, mxs};
@@ -1149,6 +1166,11 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	// factors of the points [i0, i0 + m) as one chunk; returns through vf, vl, wf, wl, rbl the
 	// border responses to the unknowns before (v) and after (w) the chunk and the last 1/beta
 	cx<S> vf = zero, vl = zero, wf = zero, wl = zero, rbl = zero;
+	// 1 / b with one division: the pivots are 1 + O(dz / (k0 n dx^2)), far from the ends of the range
+	auto recip = [](cx<S> b) {
+		const S r = (S)1 / (b.x * b.x + b.y * b.y);
+		return mk(b.x * r, -b.y * r);
+	};
 	auto chunk = [&](int i0, int m) {
 		cx<S> rb = zero, cprev = zero, ev = zero, cpz = one;
 		vf = zero;
@@ -1164,7 +1186,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 				ev = al * ev;
 			}
 			const cx<S> beta = k == 0 ? b : cfma(al, cprev, b);
-			rb = crecip(beta);
+			rb = recip(beta);
 			cprev = cs;
 			const cx<S> cc = -(rb * cs), z = cpz * rb, e = rb * ev;
 			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH;
@@ -1203,7 +1225,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	if(own) {
 		const int nx = threadIdx.y * CH + (t == nchk - 1 ? 0 : t + 1);
 		const cx<S> vfn = shv[nx], wfn = shw[nx];
-		const cx<S> m = crecip(cfnma(wl, vfn, one));
+		const cx<S> m = recip(cfnma(wl, vfn, one));
 		const cx<S> mw = m * wl, mv = m * vfn;
 		const cx<S> ph = m * vl, pg = mv * vl, qh = mw * wfn, qg = m * wfn;
 		If[I_HD * CH + t] = m * rbl;

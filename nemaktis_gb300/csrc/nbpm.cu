@@ -415,6 +415,8 @@ struct Plan : PlanBase {
 				gp.wavelength = s.wavelengths[g];
 				gp.k0 = 2 * PI_REF / gp.wavelength;
 				gp.dX = gp.k0 * s.dx; gp.dY = gp.k0 * s.dy; gp.dZ = gp.k0 * s.dz;
+				gp.rX = 1 / gp.dX; gp.rY = 1 / gp.dY;
+				gp.rXX = 1 / (gp.dX * gp.dX); gp.rYY = 1 / (gp.dY * gp.dY); gp.rXY = 1 / (gp.dX * gp.dY);
 				gp.no = s.no[g]; gp.ne = s.ne[g]; gp.ne_imag = s.ne_imag[g];
 				gp.nhost = s.nhost[g]; gp.nin = s.nin[g];
 				gp.nout_fresnel = s.iso_index.size() > 0 ? s.iso_index[0] : s.nout[g];
