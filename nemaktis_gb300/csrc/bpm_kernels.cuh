@@ -44,6 +44,8 @@ template <typename S>
 struct alignas(4 * sizeof(S)) v4 {
 	S x, y, z, w;
 };
+// Shared-memory pitch of a chunk of M points: odd, so that accesses in chunk order have no bank conflicts.
+__host__ __device__ constexpr int part_pitch(int M) { return M | 1; }
 template <typename S>
 __device__ __forceinline__ const v4<S>& part_az(const cx<S>* Fc, int k, int CH, int ci) {
 	return reinterpret_cast<const v4<S>*>(Fc + (size_t)k * NFAC * CH)[ci];
@@ -1270,7 +1272,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 }
 
 // The sequential solve of a line flagged -1 by k_factor_part, by one thread: buf holds the right-hand
-// sides of KS slots (element i of slot j at ((i / M) * (M + 1) + i % M) * ES + j * PITCH) and receives the
+// sides of KS slots (element i of slot j at ((i / M) * part_pitch(M) + i % M) * ES + j * PITCH) and receives the
 // solution.
 template <typename R, int M, int KS, int ES = 1>
 __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n) {
@@ -1281,7 +1283,7 @@ __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* 
 		cx<R> d = mk<R>(0, 0), yf = mk<R>(0, 0);
 		for(int i = 0; i < n; i++) {
 			const v4<R> az = part_az(Fc, i % M, CH, i / M);
-			cx<R>& v = b[((i / M) * (M + 1) + i % M) * ES];
+			cx<R>& v = b[((i / M) * part_pitch(M) + i % M) * ES];
 			d = cfma(mk(az.x, az.y), d, v);
 			v = d;
 			yf = cfma(mk(az.z, az.w), d, yf);
@@ -1290,7 +1292,7 @@ __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* 
 		cx<R> x = cfma(If[I_GY * CH], yf, If[I_GD * CH] * d);
 		for(int i = n - 1; i >= 0; i--) {
 			const v4<R> rc = part_rc(Fc, i % M, CH, i / M);
-			cx<R>& v = b[((i / M) * (M + 1) + i % M) * ES];
+			cx<R>& v = b[((i / M) * part_pitch(M) + i % M) * ES];
 			x = cfma(mk(rc.z, rc.w), x, cfma(part_e(Fc, i % M, CH, i / M), h, mk(rc.x, rc.y) * v));
 			v = x;
 		}
@@ -1404,7 +1406,7 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 	const int g = bc / nch, ch = bc % nch;
 	const int s0 = g * G.spg + ch * KS;  // first slot (pass-relative)
 	const int n_unk = Nx - 1;
-	const int PITCH = 32 * (M + 1);
+	const int PITCH = 32 * part_pitch(M);
 	cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw) + (size_t)warp * KS * PITCH;
 	if(iy < Ny) {  // always true unless TOUT (whose block writes together after a barrier)
 	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
@@ -1424,14 +1426,14 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 			for(int j = 0; j < KS; j++) r[j] = zero;
 		}
 #pragma unroll
-		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
+		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * part_pitch(M) + e % M] = r[j];
 	}
 	__syncwarp();
 	if(K >= 0) {
 		// forward sweep of the lane's chunk (written back over the right-hand sides) and its first
 		// unknown yf with nothing outside the chunk
 		cx<R> d[KS], yf[KS];
-		cx<R>* vb = buf + lane * (M + 1);
+		cx<R>* vb = buf + lane * part_pitch(M);
 #pragma unroll
 		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
@@ -1527,7 +1529,7 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
 					const size_t o = (size_t)(s0 + j) * 2 * N + (size_t)c * N + (size_t)iy * Nx + e;
-					const cx<R> x = buf[j * PITCH + (ee / M) * (M + 1) + ee % M];
+					const cx<R> x = buf[j * PITCH + (ee / M) * part_pitch(M) + ee % M];
 					if(dst) dst[o] = x;
 					if(acc) acc_out[o] = a[u][j] + x;
 				}
@@ -1560,7 +1562,7 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 				const int t = t0 + u * BT, e = t / LT, w = t % LT, line = blockIdx.x * LT + w;
 				if(t < Nx * LT && line < Ny) {
 					const int ee = e == Nx - 1 ? 0 : e;
-					const cx<R>* bw = bufs + (size_t)w * KS * PITCH + (ee / M) * (M + 1) + ee % M;
+					const cx<R>* bw = bufs + (size_t)w * KS * PITCH + (ee / M) * part_pitch(M) + ee % M;
 #pragma unroll
 					for(int j = 0; j < KS; j++) {
 						const size_t out = (size_t)(s0 + j) * 2 * N + (size_t)(1 - c) * N + (size_t)e * Ny + line;
@@ -1975,7 +1977,7 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 	const int n_unk = Nx - 1;
 	const int CH = 32 * W;
 	const int ci = warp * 32 + lane;
-	const int PITCH = CH * (M + 1);
+	const int PITCH = CH * part_pitch(M);
 	cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);  // [KS][CH][M+1]
 	cx<R>* sG = buf + KS * PITCH;                     // [2][KS][W]: g (first yf) of the warps' first chunks
 	cx<R>* sH = sG + 2 * KS * W;                      // [2][KS][W + 1]: h of the warps' last chunks, then of the line's
@@ -1995,13 +1997,13 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 			for(int j = 0; j < KS; j++) r[j] = zero;
 		}
 #pragma unroll
-		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * (M + 1) + e % M] = r[j];
+		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * part_pitch(M) + e % M] = r[j];
 	}
 	__syncthreads();
 	if(K >= 0) {
 		// forward sweep of the thread's chunk and its first unknown with nothing outside the chunk
 		cx<R> d[KS], yf[KS];
-		cx<R>* vb = buf + ci * (M + 1);
+		cx<R>* vb = buf + ci * part_pitch(M);
 #pragma unroll
 		for(int j = 0; j < KS; j++) d[j] = yf[j] = zero;
 #pragma unroll
@@ -2116,7 +2118,7 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 				const int ee = e == Nx - 1 ? 0 : e;
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
-					const cx<R> x = buf[j * PITCH + (ee / M) * (M + 1) + ee % M];
+					const cx<R> x = buf[j * PITCH + (ee / M) * part_pitch(M) + ee % M];
 					const size_t o = TOUT ? (size_t)(s0 + j) * 2 * N + (size_t)(1 - c) * N + iy + (size_t)e * Ny
 						: (size_t)(s0 + j) * 2 * N + (size_t)c * N + (size_t)iy * Nx + e;
 					if(dst) dst[o] = x;

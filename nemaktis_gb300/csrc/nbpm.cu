@@ -209,6 +209,12 @@ static void CUDART_CB bulk_host_fn(void* p) {
 	}
 }
 
+// The step count of k_factor_part's line scalars, for the tuner's timing runs.
+__global__ void k_fill_steps(int lines, int K, cx<double>* lsc) {
+	int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < lines) lsc[2 * (size_t)i] = mk((double)K, 0.0);
+}
+
 // Nearest-index divisions used by the shift operator are computed on the device from nref;
 // this kernel restates the SimpleShiftOperator constructor (SimpleShiftOperator.cpp:3-50).
 __global__ void k_nref_final(int ngroups, int nblocks, size_t nvox, const double* __restrict__ partial,
@@ -750,6 +756,19 @@ struct Plan : PlanBase {
 		CK(cudaStreamSynchronize(stream0));
 	}
 
+	// Jacobi steps K (k_factor_part) that the partitioned lines of direction dirn take at the sample's longest
+	// wavelength with chunks of M points: the decay from point to point is about a / |1 + 2 i a| for the
+	// coupling a = dz / (4 n k0 d^2). The workspace of the timing runs holds no factors, and K is part of a
+	// configuration's cost (64x64 FP64: 7 steps for chunks of 2 points, 3 for 4).
+	int usual_steps(const SampleHost& h, int dirn, int M) const {
+		double lam = 0, ne = 1;
+		for(size_t g = 0; g < h.s.wavelengths.size(); g++) { lam = std::max(lam, h.s.wavelengths[g]); ne = std::max(ne, std::abs(h.s.no[g])); }
+		const double d = dirn == 0 ? h.s.dx : h.s.dy, a = h.s.dz / (4 * ne * (2 * 3.14159265 / lam) * d * d);
+		const double rho = 2 * std::pow(a / std::sqrt(1 + 4 * a * a), M), lt = sizeof(R) == sizeof(float) ? -18.7 : -39.5;
+		if(!(rho < 1)) return PART_KMAX;
+		return std::min((int)PART_KMAX, std::max(0, (int)std::ceil(lt / std::log(rho)) - 1));
+	}
+
 	// Device time of one slab's solves of one direction with the current configuration of
 	// sample h (explicit step + Woodbury iterates, eager launches on the main stream): the best of
 	// three runs after one warm-up.
@@ -761,6 +780,13 @@ struct Plan : PlanBase {
 		fx_cur = W->facx.as<cx<R>>(); fy_cur = W->facy.as<cx<R>>();
 		lx_cur = W->lscx.as<cx<double>>(); ly_cur = W->lscy.as<cx<double>>();
 		ct_cur = W->coefT.as<cx<R>>();
+		{
+			const SolveCfg& c = scfg[h.index];
+			const int M = dirn == 0 ? (c.xs ? 0 : c.Mx) : c.Mxt;
+			const int lines = (dirn == 0 ? Gm.Ny : Gm.Nx) * 2 * ng;
+			k_fill_steps<<<(lines + 255) / 256, 256, 0, stream>>>(lines, M ? usual_steps(h, dirn, M) : 0, dirn == 0 ? lx_cur : ly_cur);
+			CK(cudaGetLastError());
+		}
 		float best = 1e30f;
 		for(int r = 0; r < 4; r++) {
 			CK(cudaEventRecord(ev[2], stream));
@@ -1392,7 +1418,7 @@ struct Plan : PlanBase {
 			}
 			L.grid = dim3((unsigned)((Gm.Ny + LT - 1) / LT), (unsigned)(ng * nch * 2));
 			L.block = dim3(32 * LT);
-			L.smem = (size_t)LT * L.KS * 32 * (L.M + 1) * sizeof(cx<R>);
+			L.smem = (size_t)LT * L.KS * 32 * part_pitch(L.M) * sizeof(cx<R>);
 			L.tout = tout;
 			launch(wood ? "wood_solve_x" : "expl_solve_x", bytes, [&] {
 				if(!launch_solve_xc<R>(L, Gm, slot0, nch, C, fx_cur, sc.plane_x, lx_cur, src,
@@ -1422,7 +1448,7 @@ struct Plan : PlanBase {
 			const int nch = h.spg / L.KS;
 			L.grid = dim3((unsigned)((Gt.Ny + LT - 1) / LT), (unsigned)(ng * nch * 2));
 			L.block = dim3(32 * LT);
-			L.smem = (size_t)LT * L.KS * 32 * (L.M + 1) * sizeof(cx<R>);
+			L.smem = (size_t)LT * L.KS * 32 * part_pitch(L.M) * sizeof(cx<R>);
 			L.tout = tout;
 			launch(wood ? "wood_solve_y" : "expl_solve_y", bytes, [&] {
 				if(!launch_solve_xc<R>(L, Gt, slot0, nch, ct_cur, fy_cur, sc.plane_y, ly_cur, src, dst, acc_in, acc_out,

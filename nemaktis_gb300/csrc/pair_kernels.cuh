@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 	constexpr int LT = 4;
 	// 16-byte entries per warp; the warps' buffers 2 entries apart modulo 8: no bank conflicts when the
 	// block reads one point of its 4 lines
-	constexpr int WS = 32 * (M + 1) + 2;
+	constexpr int PM = part_pitch(M), WS = 32 * PM + 2;
 	pr* const bufs = reinterpret_cast<pr*>(smem_raw);
 	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 	const int Nx = G.Nx, Ny = G.Ny, N = G.N, nch = G.Nq;
@@ -160,11 +160,11 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 #pragma unroll 1
 		for(int t = 0; t < M; t++) {
 			const int e = lane + 32 * t;
-			buf[e + e / M] = e < n ? rhs(e) : pr{0, 0, 0, 0};  // chunk e / M at pitch M + 1
+			buf[e / M * PM + e % M] = e < n ? rhs(e) : pr{0, 0, 0, 0};  // chunk e / M
 		}
 		__syncwarp();
 		if(K >= 0) {
-			pr* vb = buf + lane * (M + 1);
+			pr* vb = buf + lane * PM;
 			pr d, yf;
 			pair_forward<M>(vb, Fc, 32, lane, d, yf);
 			const int last = (n - 1) / M;
@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 			for(int u = 0; u < U; u++) {
 				const int e = lane + 32 * (t0 + u);
 				if(t0 + u <= M && e < Nx) {
-					pr x = e == n ? first : buf[e + e / M];
+					pr x = e == n ? first : buf[e / M * PM + e % M];
 					if(KIND == ST_WOOD_X) x = padd(a[u], x);
 					if(OUT == PO_SAME) o[e] = x;
-					else buf[e + e / M] = x;
+					else buf[e / M * PM + e % M] = x;
 				}
 			}
 		}
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 		if(w < Ny - line0) {
 #pragma unroll 4
 			for(int e = threadIdx.x / LT; e < Nx; e += 128 / LT) {
-				const pr x = b[e + e / M];
+				const pr x = b[e / M * PM + e % M];
 				const size_t q = (size_t)e * Ny + line0 + w;
 				if(OUT == PO_TRANS) dst[(pair * 2 + (1 - c)) * N + q] = x;
 				else {
@@ -248,7 +248,8 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	extern __shared__ unsigned char smem_raw[];
 	wait_predecessor();
 	constexpr int LT = 2;
-	const int CH = 32 * W, WS = CH * (M + 1) + 4;  // the two lines' buffers 4 entries apart modulo 8
+	constexpr int PM = part_pitch(M);
+	const int CH = 32 * W, WS = CH * PM + 4;  // the two lines' buffers 4 entries apart modulo 8
 	pr* const bufs = reinterpret_cast<pr*>(smem_raw);
 	const int ln = threadIdx.x / CH, ci = threadIdx.x % CH, warp = ci / 32, lane = ci % 32;
 	pr* sG = bufs + LT * WS + ln * (4 * W + 2);  // [2][W]: g (first yf) of the warps' first chunks
@@ -268,7 +269,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 #pragma unroll 1
 		for(int t = 0; t < M; t++) {
 			const int e = ci + CH * t;
-			buf[e + e / M] = e < n ? rhs(e) : pr{0, 0, 0, 0};
+			buf[e / M * PM + e % M] = e < n ? rhs(e) : pr{0, 0, 0, 0};
 		}
 	}
 	// the barriers are the block's: both lines take the larger number of steps
@@ -278,7 +279,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	if(ci == 0 && K > 0) atomicMax(&sK, K);
 	pr d, yf;
 	const bool part = live && K >= 0;
-	pr* vb = buf + ci * (M + 1);
+	pr* vb = buf + ci * PM;
 	if(part) pair_forward<M>(vb, Fc, CH, ci, d, yf);
 	else d = yf = pr{0, 0, 0, 0};
 	const int last = (n - 1) / M;
@@ -328,7 +329,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 #pragma unroll 4
 		for(int e = ci; e < Nx; e += CH) {
 			const int ee = e == n ? 0 : e;
-			const pr x = buf[ee + ee / M];
+			const pr x = buf[ee / M * PM + ee % M];
 			o[e] = KIND == ST_WOOD_X ? padd(own[e], x) : x;
 		}
 	}
@@ -351,7 +352,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 				const int e = e0 + u * BE;
 				if(e < Nx && w < nl) {
 					const int ee = e == n ? 0 : e;
-					const pr v = padd(a[u], bufs[w * WS + ee + ee / M]);
+					const pr v = padd(a[u], bufs[w * WS + ee / M * PM + ee % M]);
 					const size_t q = (size_t)e * Ny + line0 + w;
 					if(OUT == PO_TRANS) dst[(pair * 2 + (1 - c)) * N + q] = v;
 					else {

@@ -20,6 +20,7 @@ namespace nbpm {
 inline bool solve_pair_ok(int M, int KS) {
 	switch(M) {
 		case 2: case 4: case 8: return KS == 1 || KS == 2 || KS == 4;
+		case 3: case 5: case 6: case 7: return KS == 1 || KS == 2;  // k_solve_xc only
 		case 16: return KS == 1 || KS == 2;
 		case 32: return KS == 1;
 	}
@@ -81,6 +82,24 @@ struct SolveCfg {
 	bool pairs() const { return pair_x() && pair_y(); }
 };
 
+// Chunk lengths of the partitioned one-warp lines of n unknowns: the shortest with 32 chunks, so that
+// few lanes are idle (96 unknowns: 32 chunks of 3, not 24 of 4), then its double for short lines in
+// FP64, where a longer chunk saves joining steps; with all set, the shortest power of two as well.
+inline std::vector<int> part_chunks(int n, bool fp32, bool all) {
+	std::vector<int> out;
+	for(int M : {2, 3, 4, 5, 6, 7, 8, 16, 32})
+		if(32 * M >= n) { out.push_back(M); break; }
+	if(out.empty()) return out;
+	if(all || (!fp32 && out[0] <= 4)) {
+		const int d = 2 * out[0];
+		if(d <= 8) out.push_back(d);
+	}
+	if(all)
+		for(int M = 2; M <= 32; M *= 2)
+			if(32 * M >= n) { bool have = false; for(int m : out) have |= m == M; if(!have) out.push_back(M); break; }
+	return out;
+}
+
 // What the choice depends on.
 struct SolveShape {
 	int Nx = 0, Ny = 0;
@@ -137,10 +156,11 @@ inline std::vector<SolveCfg> x_candidates(const SolveShape& s0, bool relaxed = f
 		if(ux <= 1024) {
 			int M0 = 0;
 			for(int M = 2; M <= 32; M *= 2) if(32 * M >= ux) { M0 = M; break; }
-			for(int ks : {4, 2, 1})
-				if(s.spg % ks == 0 && solve_pair_ok(M0, ks) && (M0 * ks <= s.cap() || ks == 1)) {
-					SolveCfg c; c.Mx = M0; c.KSx = ks; out.push_back(c);
-				}
+			for(int Mp : part_chunks(ux, s.fp32, relaxed))
+				for(int ks : {4, 2, 1})
+					if(s.spg % ks == 0 && solve_pair_ok(Mp, ks) && (Mp * ks <= s.cap() || ks == 1)) {
+						SolveCfg c; c.Mx = Mp; c.KSx = ks; out.push_back(c);
+					}
 			if(M0 == 32)
 				for(int ks : {4, 2, 1})
 					if(s.spg % ks == 0 && xs_fits(ks, 32, s)) { SolveCfg c; c.Mx = 32; c.KSx = ks; c.xs = true; out.push_back(c); }
@@ -181,8 +201,13 @@ inline std::vector<SolveCfg> y_candidates(const SolveShape& s0, bool relaxed = f
 			for(int ks : {4, 2, 1})
 				if(s.spg % ks == 0 && solve_pair_ok(Mt, ks) && (Mt * ks <= s.cap() || ks == 1)) {
 					SolveCfg c; c.Mt = Mt; c.KSy = ks; out.push_back(c);
-					if(s.Nx > 3 && s.nw == 2) { SolveCfg t; t.Mxt = Mt; t.KSy = ks; out.push_back(t); }
 				}
+			if(s.Nx > 3 && s.nw == 2)
+				for(int Mp : part_chunks(uy, s.fp32, relaxed))
+					for(int ks : {4, 2, 1})
+						if(s.spg % ks == 0 && solve_pair_ok(Mp, ks) && (Mp * ks <= s.cap() || ks == 1)) {
+							SolveCfg t; t.Mxt = Mp; t.KSy = ks; out.push_back(t);
+						}
 		}
 		// long y-lines as several-warps-per-line x-lines of the transposed frame
 		if(uy > 256 && uy <= 2048 && s.Nx > 3 && s.nw == 2) {

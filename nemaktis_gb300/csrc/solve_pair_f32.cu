@@ -4,11 +4,10 @@
 
 namespace nbpm {
 
-// one line per warp: chunk lengths 2, 4, 8; several warps per line: 8
+// one line per warp: chunk lengths 2 .. 8; several warps per line: 8
+#define NBPM_XP_M(F, MM) F(MM, ST_EXPL_Y, PO_SAME) F(MM, ST_WOOD_X, PO_SAME) F(MM, ST_WOOD_X, PO_TRANS) F(MM, ST_WOOD_X, PO_PLAIN)
 #define NBPM_XP_ALL(F) \
-	F(2, ST_EXPL_Y, PO_SAME) F(2, ST_WOOD_X, PO_SAME) F(2, ST_WOOD_X, PO_TRANS) F(2, ST_WOOD_X, PO_PLAIN) \
-	F(4, ST_EXPL_Y, PO_SAME) F(4, ST_WOOD_X, PO_SAME) F(4, ST_WOOD_X, PO_TRANS) F(4, ST_WOOD_X, PO_PLAIN) \
-	F(8, ST_EXPL_Y, PO_SAME) F(8, ST_WOOD_X, PO_SAME) F(8, ST_WOOD_X, PO_TRANS) F(8, ST_WOOD_X, PO_PLAIN)
+	NBPM_XP_M(F, 2) NBPM_XP_M(F, 3) NBPM_XP_M(F, 4) NBPM_XP_M(F, 5) NBPM_XP_M(F, 6) NBPM_XP_M(F, 7) NBPM_XP_M(F, 8)
 #define NBPM_XWP_ALL(F) \
 	F(8, ST_EXPL_Y, PO_SAME) F(8, ST_WOOD_X, PO_SAME) F(8, ST_WOOD_X, PO_TRANS) F(8, ST_WOOD_X, PO_PLAIN)
 
@@ -20,7 +19,7 @@ bool launch_solve_pair(cudaStream_t st, bool dep, int M, int W, int kind, int ou
 	pr* d = reinterpret_cast<pr*>(dst);
 	if(W == 1) {
 		const dim3 grid((unsigned)((size_t)((G.Ny + 3) / 4) * 2 * G.Nq), (unsigned)ng);
-		const size_t smem = (size_t)4 * (32 * (M + 1) + 2) * sizeof(pr);
+		const size_t smem = (size_t)4 * (32 * part_pitch(M) + 2) * sizeof(pr);
 #define NBPM_XP(MM, KD, OO) \
 		if(M == MM && kind == KD && out == OO) { \
 			launch_dep(dep, k_solve_xp<MM, KD, OO>, grid, dim3(128), smem, st, G, coef, fac, plane, lsc, s, d, a, plain); \
@@ -30,7 +29,7 @@ bool launch_solve_pair(cudaStream_t st, bool dep, int M, int W, int kind, int ou
 		return false;
 	}
 	const dim3 grid((unsigned)((size_t)((G.Ny + 1) / 2) * 2 * G.Nq), (unsigned)ng);
-	const size_t smem = (size_t)2 * (32 * W * (M + 1) + 4 + 4 * W + 2) * sizeof(pr);
+	const size_t smem = (size_t)2 * (32 * W * part_pitch(M) + 4 + 4 * W + 2) * sizeof(pr);
 	// Registers: lines of 3 warps and more make blocks of 192 threads and more, of which 64 registers leave
 	// 30 warps per SM resident (1024x1024: 100.5 ms a step with 64, 108 with 80); blocks of two-warp lines, 128
 	// threads, take 72 as k_solve_xp, or 96 when the launch has too few warps to fill the SMs anyway

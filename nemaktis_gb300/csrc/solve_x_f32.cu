@@ -16,7 +16,9 @@ namespace nbpm {
 	}
 #define NBPM_XC_PAIRS(KIND) \
 	NBPM_XC(2, 1, KIND) NBPM_XC(2, 2, KIND) NBPM_XC(2, 4, KIND) NBPM_XC(4, 1, KIND) NBPM_XC(4, 2, KIND) NBPM_XC(4, 4, KIND) \
-	NBPM_XC(8, 1, KIND) NBPM_XC(8, 2, KIND) NBPM_XC(8, 4, KIND) NBPM_XC(16, 1, KIND) NBPM_XC(16, 2, KIND) NBPM_XC(32, 1, KIND)
+	NBPM_XC(8, 1, KIND) NBPM_XC(8, 2, KIND) NBPM_XC(8, 4, KIND) NBPM_XC(16, 1, KIND) NBPM_XC(16, 2, KIND) NBPM_XC(32, 1, KIND) \
+	NBPM_XC(3, 1, KIND) NBPM_XC(3, 2, KIND) NBPM_XC(5, 1, KIND) NBPM_XC(5, 2, KIND) NBPM_XC(6, 1, KIND) NBPM_XC(6, 2, KIND) \
+	NBPM_XC(7, 1, KIND) NBPM_XC(7, 2, KIND)
 
 template <>
 bool launch_solve_xc<float>(const SolveLaunch& L, Geom G, int slot0, int nch, const cx<float>* coef,
@@ -31,7 +33,9 @@ bool launch_solve_xc<float>(const SolveLaunch& L, Geom G, int slot0, int nch, co
 	cudaFuncSetAttribute(k_solve_xc<float, MM, KD, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 #define NBPM_XA_PAIRS(KIND) \
 	NBPM_XA(2, 1, KIND) NBPM_XA(2, 2, KIND) NBPM_XA(2, 4, KIND) NBPM_XA(4, 1, KIND) NBPM_XA(4, 2, KIND) NBPM_XA(4, 4, KIND) \
-	NBPM_XA(8, 1, KIND) NBPM_XA(8, 2, KIND) NBPM_XA(8, 4, KIND) NBPM_XA(16, 1, KIND) NBPM_XA(16, 2, KIND) NBPM_XA(32, 1, KIND)
+	NBPM_XA(8, 1, KIND) NBPM_XA(8, 2, KIND) NBPM_XA(8, 4, KIND) NBPM_XA(16, 1, KIND) NBPM_XA(16, 2, KIND) NBPM_XA(32, 1, KIND) \
+	NBPM_XA(3, 1, KIND) NBPM_XA(3, 2, KIND) NBPM_XA(5, 1, KIND) NBPM_XA(5, 2, KIND) NBPM_XA(6, 1, KIND) NBPM_XA(6, 2, KIND) \
+	NBPM_XA(7, 1, KIND) NBPM_XA(7, 2, KIND)
 
 #define NBPM_XAT(MM, KK) \
 	cudaFuncSetAttribute(k_solve_xc<float, MM, ST_WOOD_X, KK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -40,6 +44,7 @@ void set_solve_smem_x_f32(int bytes) {
 	NBPM_XA_PAIRS(ST_EXPL_Y)
 	NBPM_XA_PAIRS(ST_WOOD_X)
 	NBPM_XAT(2, 1) NBPM_XAT(2, 2) NBPM_XAT(2, 4) NBPM_XAT(4, 1) NBPM_XAT(4, 2) NBPM_XAT(4, 4)
+	NBPM_XAT(3, 1) NBPM_XAT(3, 2) NBPM_XAT(5, 1) NBPM_XAT(5, 2) NBPM_XAT(6, 1) NBPM_XAT(6, 2) NBPM_XAT(7, 1) NBPM_XAT(7, 2)
 	NBPM_XAT(8, 1) NBPM_XAT(8, 2) NBPM_XAT(8, 4) NBPM_XAT(16, 1) NBPM_XAT(16, 2) NBPM_XAT(32, 1)
 }
 

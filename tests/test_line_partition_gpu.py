@@ -26,7 +26,9 @@ def run_both(dims, cfg, **kw):
 
 
 # n = N - 1 unknowns per line: 3, 4 (two chunks), one chunk more or less than a warp, ragged last chunks
-@pytest.mark.parametrize("n,M", [(3, 2), (4, 2), (63, 2), (64, 2), (65, 4), (127, 4), (129, 8), (249, 8), (256, 8)])
+@pytest.mark.parametrize("n,M", [(3, 2), (4, 2), (63, 2), (64, 2), (65, 4), (127, 4), (129, 8), (249, 8), (256, 8),
+                                 # odd chunks (no padding in shared memory), and twice the shortest (half the lanes idle)
+                                 (74, 3), (96, 3), (129, 5), (160, 5), (161, 6), (192, 6), (193, 7), (224, 7), (63, 4), (96, 6)])
 def test_chunk_edges_one_warp(gpu, n, M):
     cfg = "xc:M=%d:KS=%d;yx:M=%d:KS=%d"
     assert run_both((n + 1, 6, 4), cfg % (M, 2, 2, 2)) <= FP64_TOL

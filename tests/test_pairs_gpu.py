@@ -24,6 +24,7 @@ def check(dims, cfg, q=Q3, tol=1e-5, **kw):
 
 
 @pytest.mark.parametrize("n,m,M", [(3, 4, 2), (63, 9, 2), (64, 64, 2), (65, 6, 4), (128, 7, 4), (129, 10, 8), (256, 5, 8),
+                                   (74, 5, 3), (96, 6, 3), (129, 7, 5), (191, 4, 6), (224, 5, 7),
                                    (257, 6, 16), (500, 4, 16)])
 @pytest.mark.parametrize("q", [Q0, Q3])
 def test_one_warp_per_line(gpu, n, m, M, q):
