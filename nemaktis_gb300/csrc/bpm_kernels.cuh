@@ -121,20 +121,52 @@ struct ShiftParams {
 	// converting the FP64 values at each use)
 	float fwx[4], fwy[4];
 	float fph_re, fph_im;
+	// weights of one shift and of two one after the other as 7 taps, the latter sums of products of the above
+	double tx[2][7], ty[2][7];
 };
 
-// Shift weights and phase factor in the arithmetic type R.
+// Weights and phase factor in the arithmetic type R, and the filter of nsh = 1 or 2 shifts of one axis on N
+// consecutive values in place, v[k] for k < N - 6. FP64: one 7-tap filter (7 (N - 6) multiply-adds in place of
+// 4 (N - 3) + 4 (N - 6); the FP64 pipe bounds the transition: 1408 -> 1082 us on 256x256, 3 wavelengths, 13
+// q). FP32: two 4-tap passes, which need fewer registers (473 us on 16 wavelengths, 513 with 7 taps).
 template <typename R>
 struct ShiftW {
+	const int nsh;
 	R wx[4], wy[4];
 	cx<R> ph;
-	__device__ __forceinline__ explicit ShiftW(const ShiftParams& P) {
+	__device__ __forceinline__ ShiftW(const ShiftParams& P, int n) : nsh(n) {
 #pragma unroll
-		for(int k = 0; k < 4; k++) {
-			wx[k] = sizeof(R) == sizeof(float) ? (R)P.fwx[k] : (R)P.wx[k];
-			wy[k] = sizeof(R) == sizeof(float) ? (R)P.fwy[k] : (R)P.wy[k];
+		for(int k = 0; k < 4; k++) { wx[k] = P.fwx[k]; wy[k] = P.fwy[k]; }
+		ph = mk<R>(P.fph_re, P.fph_im);
+	}
+	template <int N>
+	__device__ __forceinline__ void filter(const R* w, cx<R>* v) const {
+#pragma unroll
+		for(int k = 0; k < N - 3; k++) v[k] = w[0] * v[k] + w[1] * v[k + 1] + w[2] * v[k + 2] + w[3] * v[k + 3];
+		if(nsh == 2) {
+#pragma unroll
+			for(int k = 0; k < N - 6; k++) v[k] = w[0] * v[k] + w[1] * v[k + 1] + w[2] * v[k + 2] + w[3] * v[k + 3];
 		}
-		ph = sizeof(R) == sizeof(float) ? mk<R>((R)P.fph_re, (R)P.fph_im) : mk<R>((R)P.ph_re, (R)P.ph_im);
+	}
+};
+template <>
+struct ShiftW<double> {
+	double wx[7], wy[7];
+	cx<double> ph;
+	__device__ __forceinline__ ShiftW(const ShiftParams& P, int n) {
+#pragma unroll
+		for(int k = 0; k < 7; k++) { wx[k] = P.tx[n - 1][k]; wy[k] = P.ty[n - 1][k]; }
+		ph = mk<double>(P.ph_re, P.ph_im);
+	}
+	template <int N>
+	__device__ __forceinline__ void filter(const double* w, cx<double>* v) const {
+#pragma unroll
+		for(int k = 0; k < N - 6; k++) {
+			cx<double> s = w[0] * v[k];
+#pragma unroll
+			for(int m = 1; m < 7; m++) s = mk<double>(fma(w[m], v[k + m].x, s.x), fma(w[m], v[k + m].y, s.y));
+			v[k] = s;
+		}
 	}
 };
 
@@ -2519,14 +2551,13 @@ __global__ void k_shift_y(Geom G, int slot0, const ShiftParams* __restrict__ sp,
 // shift_y(B)): F_out = phase_B(ph^n * Y^n X^n (phase_A(F))), n = nshift (1 or 2). X and Y are
 // the circulant cubic shifts of SimpleShiftOperator (period Nx-1 / Ny-1; they act on rows and
 // columns and commute, so Y X Y X = Y Y X X). For a tile of 32 x 32 outputs of one slot the
-// block stages the input window (phase_A applied) in shared memory; each thread then runs the n
-// x-passes over 8 consecutive outputs of a window row in registers (the 8 + 3n inputs read once)
-// into a second buffer, and the n y-passes over 4 consecutive rows of an output column, and
-// writes the tile. Indices wrap with i mod (N-1), which equals the
-// reference's wrap rule for every index above -(N-1) (the composition of two wrapped passes
-// then also reduces to one mod); a slot whose integer shift reaches -(N-2) or below takes the
-// exact per-point path instead. The duplicate row and column of F are never read, as in the
-// separate passes.
+// block stages the input window (phase_A applied) in shared memory; each thread then filters
+// 8 consecutive outputs of a window row in registers (the 8 + 3n inputs read once) into a second
+// buffer, then 4 consecutive rows of an output column, and writes the tile. Indices wrap with
+// i mod (N-1), which equals the reference's wrap rule for every index above -(N-1) (the composition
+// of two wrapped passes then also reduces to one mod); a slot whose integer shift reaches -(N-2) or
+// below takes the exact per-point path instead. The duplicate row and column of F are never read, as
+// in the separate passes. Bound: the FP64 pipe; in FP32 instruction issue (59 % active).
 constexpr int SHT = 32;  // tile edge
 
 __device__ __forceinline__ int pmod(int i, int n) {
@@ -2596,7 +2627,7 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 	const int g = gs / G.spg - slot0 / G.spg;
 	const int gq = (gs / G.spg) * G.Nq + (gs / 2) % G.Nq;
 	const ShiftParams& P = sp[gq];
-	const ShiftW<R> W(P);
+	const ShiftW<R> W(P, nsh);
 	const size_t N = G.N;
 	const int Nx = G.Nx, Ny = G.Ny;
 	const bool ax = Nx > 3, ay = Ny > 3;
@@ -2666,13 +2697,7 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 			cx<R> w[14];
 #pragma unroll
 			for(int k = 0; k < 14; k++) w[k] = k < nin ? in[k] : mk<R>(0, 0);
-			// first pass: 8 + 3 (n - 1) values, second pass (n = 2): 8
-#pragma unroll
-			for(int k = 0; k < 11; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
-			if(nsh == 2) {
-#pragma unroll
-				for(int k = 0; k < 8; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
-			}
+			W.template filter<14>(W.wx, w);
 			cx<R>* out = B + c * (SHT + 6) * PB + v * PB + seg * 8;
 #pragma unroll
 			for(int k = 0; k < 8; k++) out[k] = w[k];
@@ -2695,12 +2720,7 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 				cx<R> w[10];
 #pragma unroll
 				for(int k = 0; k < 10; k++) w[k] = k < nin ? in[k * PY] : mk<R>(0, 0);
-#pragma unroll
-				for(int k = 0; k < 7; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
-				if(nsh == 2) {
-#pragma unroll
-					for(int k = 0; k < 4; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
-				}
+				W.template filter<10>(W.wy, w);
 #pragma unroll
 				for(int k = 0; k < 4; k++) o[c][k] = w[k];
 			}
@@ -2767,7 +2787,7 @@ static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0,
 	extern __shared__ unsigned char smem_raw[];
 	const int z = blockIdx.z, g = z / G.Nq;
 	const ShiftParams& P = sp[pair0 + z];
-	const ShiftW<R> W(P);
+	const ShiftW<R> W(P, nsh);
 	const size_t N = G.N;
 	const int Nx = G.Nx, Ny = G.Ny;
 	const bool ax = Nx > 3, ay = Ny > 3;
@@ -2838,12 +2858,7 @@ static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0,
 				cx<R> w[14];
 #pragma unroll
 				for(int k = 0; k < 14; k++) w[k] = k < nin ? in[k] : mk<R>(0, 0);
-#pragma unroll
-				for(int k = 0; k < 11; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
-				if(nsh == 2) {
-#pragma unroll
-					for(int k = 0; k < 8; k++) w[k] = W.wx[0] * w[k] + W.wx[1] * w[k + 1] + W.wx[2] * w[k + 2] + W.wx[3] * w[k + 3];
-				}
+			W.template filter<14>(W.wx, w);
 				cx<R>* out = B + c * (SHT + 6) * PB + v * PB + seg * 8;
 #pragma unroll
 				for(int k = 0; k < 8; k++) out[k] = w[k];
@@ -2861,12 +2876,7 @@ static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0,
 				cx<R> w[10];
 #pragma unroll
 				for(int k = 0; k < 10; k++) w[k] = k < nin ? in[k * PY] : mk<R>(0, 0);
-#pragma unroll
-				for(int k = 0; k < 7; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
-				if(nsh == 2) {
-#pragma unroll
-					for(int k = 0; k < 4; k++) w[k] = W.wy[0] * w[k] + W.wy[1] * w[k + 1] + W.wy[2] * w[k + 2] + W.wy[3] * w[k + 3];
-				}
+				W.template filter<10>(W.wy, w);
 #pragma unroll
 				for(int k = 0; k < 4; k++) o[c][k] = w[k];
 			}

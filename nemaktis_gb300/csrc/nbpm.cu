@@ -262,6 +262,12 @@ __global__ void k_shift_params(int ngroups, int Nq, int Nx, int Ny, const GroupP
 	}
 	for(int k = 0; k < 4; k++) { P.fwx[k] = (float)P.wx[k]; P.fwy[k] = (float)P.wy[k]; }
 	P.fph_re = (float)P.ph_re; P.fph_im = (float)P.ph_im;
+	for(int k = 0; k < 7; k++) {
+		P.tx[0][k] = k < 4 ? P.wx[k] : 0;
+		P.ty[0][k] = k < 4 ? P.wy[k] : 0;
+		P.tx[1][k] = P.ty[1][k] = 0;
+		for(int a = max(0, k - 3); a <= min(3, k); a++) { P.tx[1][k] += P.wx[a] * P.wx[k - a]; P.ty[1][k] += P.wy[a] * P.wy[k - a]; }
+	}
 	sp[t] = P;
 }
 
