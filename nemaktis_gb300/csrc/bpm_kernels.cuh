@@ -358,59 +358,6 @@ static __global__ void k_neff_partial(const double* __restrict__ dir, int fd, co
 //    and column points. D1 uses the reference's neighbour indices (ix==Nx-1 -> 1,
 //    ix==0 -> Nx-2) while the stencil columns wrap with period Nx-1.
 // ---------------------------------------------------------------------------------------
-template <typename T>
-struct CoefCtx {
-	const T* A;
-	const T* B;
-	int N, Nx;
-	T hmu, rxx, ryy, rxy, va0, va1;
-	__device__ __forceinline__ T avg(int q, int x, int y) const {
-		int i = x + Nx * y;
-		return (A[q * N + i] + B[q * N + i]) / (T)2;
-	}
-	__device__ __forceinline__ T vsum(int a, int x, int y) const {
-		int i = x + Nx * y, q = a == 0 ? Q_VX : Q_VY;
-		return A[q * N + i] + B[q * N + i];
-	}
-	__device__ __forceinline__ void sinv(int x, int y, T& ixx, T& iyy, T& ixy) const {
-		T exx = avg(Q_XXS, x, y), eyy = avg(Q_YYS, x, y), exy = avg(Q_XYS, x, y);
-		T det = exx * eyy - exy * exy;
-		const T r = (T)1 / det;
-		ixx = eyy * r; iyy = exx * r; ixy = -exy * r;
-	}
-	// One stencil entry of mu*R for the 4 blocks (00, 01, 10, 11). D is the real 2x2 entry
-	// of D at this (row, column) pair; dd is the first-derivative weight of the walk-off
-	// (0 for none) acting on component bT.
-	__device__ void entry(T D00, T D01, T D10, T D11, int cxp, int cyp,
-			T dd, int bT, cx<T> out[4]) const {
-		T re[4] = {0, 0, 0, 0}, im[4] = {0, 0, 0, 0};
-		if(dd != 0) {
-			T vb0 = vsum(0, cxp, cyp), vb1 = vsum(1, cxp, cyp);
-			im[0 + bT] += dd * ((T)0.25 * va0);
-			im[2 + bT] += dd * ((T)0.25 * va1);
-			im[2 * bT + 0] += dd * ((T)0.25 * vb0);
-			im[2 * bT + 1] += dd * ((T)0.25 * vb1);
-		}
-		T cxx, cyy, cxy;
-		sinv(cxp, cyp, cxx, cyy, cxy);
-		T Dm[2][2] = {{D00, D01}, {D10, D11}};
-		const T q4 = (T)0.25;
-		for(int a = 0; a < 2; a++) {
-			re[2 * a] += q4 * Dm[a][0] * cxx;
-			re[2 * a] += q4 * Dm[a][1] * cxy;
-			re[2 * a + 1] += q4 * Dm[a][0] * cxy;
-			re[2 * a + 1] += q4 * Dm[a][1] * cyy;
-		}
-		for(int b = 0; b < 2; b++) {
-			re[b] += q4 * rxx * Dm[0][b];
-			re[b] += q4 * rxy * Dm[1][b];
-			re[2 + b] += q4 * rxy * Dm[0][b];
-			re[2 + b] += q4 * ryy * Dm[1][b];
-		}
-		for(int b = 0; b < 4; b++) out[b] = mk(-hmu * im[b], hmu * re[b]);  // i*hmu*(re+i*im)
-	}
-};
-
 // Phase operator of one point (PhaseEvolutionOperator.cpp:14-32) from eps planes A, B of the
 // slab's two ends, in the arithmetic type T.
 template <typename T>
@@ -458,23 +405,64 @@ __device__ __forceinline__ void phase_op(const T* A, const T* B, int N, int p, T
 	oxy = ((e * mk<T>((T)0, (T)1)) * dxy) * sinc;
 }
 
-template <typename S>
-__global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
+// A block takes a tile of 32 x TY points and first forms what the operators need of a point (S^-1, K, 1/eps_zz,
+// walk-off) once for each point of the tile and around it, in shared memory: a point's ten neighbours would
+// each form it again (a determinant and a division each). The stencil columns wrap with period N - 1 while the
+// first derivatives' weights look at the natural neighbour, so column and row 0 have a place of their own past the
+// tile's edge (index 32 + 2, TY + 2) for the last unknowns. TR: the tile's entries also go to the transposed
+// frame's set (its DX is DY, its DY is DX, its DXDY block b is DXDY block 3 - b with the two middle corners
+// exchanged), through shared memory so that TY consecutive points are written together.
+// Bound: FP64 pipe (FP64), HBM (FP32, 82 % of the copy rate). With every neighbour's values formed again and the
+// transposed set copied by a kernel of its own: 256x256, 16 wavelengths, FP32 88 + 87 us, 96 us so; 3
+// wavelengths FP64 269 + 36 and 179 us; a 64x64 FP64 slab 31 + 8 and 25 us.
+constexpr int COEF_TX = 32;
+enum { CQ_CXX = 0, CQ_CYY, CQ_CXY, CQ_KXX, CQ_KYY, CQ_KXY, CQ_EZ, CQ_V0, CQ_V1, NCQ };
+template <int TY>
+constexpr int coef_tile_points() { return (COEF_TX + 3) * (TY + 3); }
+template <typename S, int TY>
+constexpr size_t coef_smem(bool tr) {
+	return NCQ * coef_tile_points<TY>() * sizeof(S) + 32 + (tr ? (size_t)4 * TY * (COEF_TX + 1) * 4 * sizeof(S) : 0);
+}
+template <typename S, int TY, bool TR>
+__global__ void __launch_bounds__(32 * TY) k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		const double* __restrict__ wts, int iz, Geom G, const GroupParams* __restrict__ gps,
-		cx<S>* __restrict__ coef) {
+		cx<S>* __restrict__ coef, cx<S>* __restrict__ coefT) {
 	typedef S T;  // arithmetic type of the eps planes, the phase operator and the R coefficients
-	int p = blockIdx.x * blockDim.x + threadIdx.x;
-	int g = blockIdx.y;
-	int N = G.N, Nx = G.Nx, Ny = G.Ny;
-	if(p >= N) return;
-	int ix = p % Nx, iy = p / Nx;
-	const GroupParams gp = gps[g];
+	extern __shared__ unsigned char smem_raw[];
+	constexpr int LX = COEF_TX + 3, LY = TY + 3, LP = LX * LY;
+	T* const sm = reinterpret_cast<T*>(smem_raw);
+	const int g = blockIdx.z, N = G.N, Nx = G.Nx, Ny = G.Ny;
+	const int x0 = blockIdx.x * COEF_TX, y0 = blockIdx.y * TY;
+	const GroupParams& gp = gps[g];
 	const T* A = QA + (size_t)g * NQ * N;
 	const T* B = QB + (size_t)g * NQ * N;
 	cx<S>* C = coef + (size_t)g * coef_set_size(N);
-
-	// Phase operator.
-	{
+	const int tid = threadIdx.y * 32 + threadIdx.x;
+	// place l of a tile's axis: l = 0 the point before the tile (period n - 1), 1 .. size + 1 the tile and the
+	// natural next point, size + 2 point 0
+	auto place = [](int l, int size, int o, int n) {
+		const int i = l == size + 2 ? 0 : l == 0 ? (o == 0 ? n - 2 : o - 1) : o + l - 1;
+		return max(0, min(i, n - 1));
+	};
+	for(int e = tid; e < LP; e += 32 * TY) {
+		const int q = place(e % LX, COEF_TX, x0, Nx) + Nx * place(e / LX, TY, y0, Ny);
+		auto avg = [&](int k) { return (A[k * N + q] + B[k * N + q]) * (T)0.5; };
+		const T exx = avg(Q_XXS), eyy = avg(Q_YYS), exy = avg(Q_XYS);
+		const T r = (T)1 / (exx * eyy - exy * exy);
+		sm[CQ_CXX * LP + e] = eyy * r;
+		sm[CQ_CYY * LP + e] = exx * r;
+		sm[CQ_CXY * LP + e] = -exy * r;
+		sm[CQ_KXX * LP + e] = avg(Q_XXTR);
+		sm[CQ_KYY * LP + e] = avg(Q_YYTR);
+		sm[CQ_KXY * LP + e] = avg(Q_XYTR);
+		sm[CQ_EZ * LP + e] = avg(Q_IZZ);
+		sm[CQ_V0 * LP + e] = A[Q_VX * N + q] + B[Q_VX * N + q];
+		sm[CQ_V1 * LP + e] = A[Q_VY * N + q] + B[Q_VY * N + q];
+	}
+	__syncthreads();
+	const int ix = x0 + threadIdx.x, iy = y0 + threadIdx.y, p = ix + Nx * iy;
+	const bool live = ix < Nx && iy < Ny;
+	if(live) {
 		T w0 = (T)0.5, w1 = (T)0.5;
 		if(wts) { size_t vi = (size_t)iz * N + p; w0 = (T)wts[2 * vi]; w1 = (T)wts[2 * vi + 1]; }
 		cx<T> oxx, oyy, oxy;
@@ -483,106 +471,112 @@ __global__ void k_coef(const S* __restrict__ QA, const S* __restrict__ QB,
 		coef_ph(C, 1, p) = oyy;
 		coef_ph(C, 2, p) = oxy;
 	}
-
-	CoefCtx<T> X;
-	X.A = A; X.B = B; X.N = N; X.Nx = Nx;
-	X.hmu = (T)(gp.dZ / 2.);
-	X.sinv(ix, iy, X.rxx, X.ryy, X.rxy);
-	X.va0 = X.vsum(0, ix, iy);
-	X.va1 = X.vsum(1, ix, iy);
+	const int lx = threadIdx.x + 1, ly = threadIdx.y + 1, l0 = lx + LX * ly;
+	const int lxp = ix == Nx - 2 ? COEF_TX + 2 : lx + 1, lyp = iy == Ny - 2 ? TY + 2 : ly + 1;  // next stencil column / row
+	auto Q = [&](int k, int l) { return sm[k * LP + l]; };
+	const T hmu = (T)(gp.dZ / 2.), q4 = (T)0.25, h4 = q4 * hmu;
 	const T rX = (T)gp.rX, rY = (T)gp.rY, rXX = (T)gp.rXX, rYY = (T)gp.rYY, rXY = (T)gp.rXY;
-	auto ezz = [&](int x, int y) { int i = x + Nx * y; return (A[Q_IZZ * N + i] + B[Q_IZZ * N + i]) / (T)2; };
-	T e0 = ezz(ix, iy);
-	int pxq = (ix == Nx - 1) ? 1 : ix + 1, mxq = (ix == 0) ? Nx - 2 : ix - 1;
-	int pyq = (iy == Ny - 1) ? 1 : iy + 1, myq = (iy == 0) ? Ny - 2 : iy - 1;
-	int pxs = (ix == Nx - 2) ? 0 : ix + 1, mxs = (ix == 0) ? Nx - 2 : ix - 1;
-	int pys = (iy == Ny - 2) ? 0 : iy + 1, mys = (iy == 0) ? Ny - 2 : iy - 1;
-	cx<T> r[3][4];
-	const cx<T> z = mk<T>(0, 0);
-
-	// DX: rows ix < Nx-1 when Nx > 3; k = 0 mx, 1 centre, 2 px.
-	{
-		bool ok = Nx > 3 && ix < Nx - 1;
-		T cm = 0, cp = 0, c0 = 0;
-		if(ok) {
-			cm = (T)0.5 * (ezz(mxq, iy) + e0) * rXX;
-			cp = (T)0.5 * (ezz(pxq, iy) + e0) * rXX;
-			c0 = -cm - cp;
-		}
-		const int cols[3] = {mxs, ix, pxs};
-		const T c1[3] = {cm, c0, cp};
-		const T L[3] = {rXX, (T)-2 * rXX, rXX};
-		const T dd[3] = {(T)-0.5 * rX, 0, (T)0.5 * rX};
+	const T rxx = Q(CQ_CXX, l0), ryy = Q(CQ_CYY, l0), rxy = Q(CQ_CXY, l0), e0 = Q(CQ_EZ, l0);
+	const T va0 = Q(CQ_V0, l0), va1 = Q(CQ_V1, l0);
+	// imaginary parts of the four blocks, (dZ/2) (D S^-1 + S^-1 D) / 4 with S^-1 at the neighbour l and at the point
+	auto blocks = [&](T D00, T D01, T D10, T D11, int l, T* im) {
+		const T cxx = Q(CQ_CXX, l), cyy = Q(CQ_CYY, l), cxy = Q(CQ_CXY, l);
+		im[0] = h4 * (D00 * cxx + D01 * cxy + rxx * D00 + rxy * D10);
+		im[1] = h4 * (D00 * cxy + D01 * cyy + rxx * D01 + rxy * D11);
+		im[2] = h4 * (D10 * cxx + D11 * cxy + rxy * D00 + ryy * D10);
+		im[3] = h4 * (D10 * cxy + D11 * cyy + rxy * D01 + ryy * D11);
+	};
+	// the sets of 4 vectors as they are complete: to the point's set and, for TR, to the transposed one
+	v4<S>* const st = reinterpret_cast<v4<S>*>(smem_raw + ((NCQ * LP * sizeof(S) + 31) & ~(size_t)31));
+	cx<S>* CT = coefT + (TR ? (size_t)g * coef_set_size(N) : 0);
+	auto put = [&](const v4<S>* v, int k, int kt, bool corners) {
+		if(live) {
 #pragma unroll
-		for(int k = 0; k < 3; k++) {
-			if(ok) {
-				int cxp = cols[k];
-				T kxx = X.avg(Q_XXTR, cxp, iy), kxy = X.avg(Q_XYTR, cxp, iy);
-				X.entry(c1[k] * kxx, c1[k] * kxy, (T)0, L[k], cxp, iy, dd[k], 0, r[k]);
+			for(int j = 0; j < 4; j++) coef_v(C, k + j, p) = v[j];
+		}
+		if(TR) {
+			__syncthreads();  // the vectors before these have been written
+#pragma unroll
+			for(int j = 0; j < 4; j++)
+				st[(j * TY + threadIdx.y) * (COEF_TX + 1) + threadIdx.x] = corners ? v4<S>{v[3 - j].x, v[3 - j].z, v[3 - j].y, v[3 - j].w} : v[j];
+			__syncthreads();
+			const int ty = tid % TY, tx = tid / TY;
+			if(x0 + tx < Nx && y0 + ty < Ny) {
+#pragma unroll
+				for(int j = 0; j < 4; j++) coef_v(CT, kt + j, (x0 + tx) * Ny + y0 + ty) = st[(j * TY + ty) * (COEF_TX + 1) + tx];
 			}
-			else r[k][0] = r[k][1] = r[k][2] = r[k][3] = z;
 		}
-#pragma unroll
-		for(int b = 0; b < 3; b++) coef_v(C, V_DX + b, p) = v4<S>{r[0][b].x, r[0][b].y, r[2][b].x, r[2][b].y};
-		coef_v(C, V_DX + 3, p) = v4<S>{r[0][3].y, r[2][3].y, r[1][3].y, r[1][2].y};
-		coef_u(C, U_DX, p) = mk(r[1][0].y, r[1][1].y);
+	};
+	v4<S> v[4];
+	const v4<S> zero{0, 0, 0, 0};
+	cx<S> ux = mk<S>(0, 0), uy = mk<S>(0, 0);
+	T m[4], c[4], n[4];
+	// DX: rows ix < Nx-1 when Nx > 3; m, c, n: columns ix - 1, ix, ix + 1
+	v[0] = v[1] = v[2] = v[3] = zero;
+	if(Nx > 3 && ix < Nx - 1) {
+		const int lm = l0 - 1, ln = lxp + LX * ly;
+		const T cm = (T)0.5 * (Q(CQ_EZ, lm) + e0) * rXX, cp = (T)0.5 * (Q(CQ_EZ, l0 + 1) + e0) * rXX, c0 = -cm - cp;
+		blocks(cm * Q(CQ_KXX, lm), cm * Q(CQ_KXY, lm), (T)0, rXX, lm, m);
+		blocks(c0 * Q(CQ_KXX, l0), c0 * Q(CQ_KXY, l0), (T)0, (T)-2 * rXX, l0, c);
+		blocks(cp * Q(CQ_KXX, ln), cp * Q(CQ_KXY, ln), (T)0, rXX, ln, n);
+		// walk-off: -(dZ/2) (-+ 1 / (2 dX)) / 4 times v0 twice, v1 of the neighbour, v1 of the point
+		const T d = hmu * (T)0.5 * rX * q4;
+		v[0] = v4<S>{d * (va0 + Q(CQ_V0, lm)), m[0], -d * (va0 + Q(CQ_V0, ln)), n[0]};
+		v[1] = v4<S>{d * Q(CQ_V1, lm), m[1], -d * Q(CQ_V1, ln), n[1]};
+		v[2] = v4<S>{d * va1, m[2], -d * va1, n[2]};
+		v[3] = v4<S>{m[3], n[3], c[3], c[2]};
+		ux = mk(c[0], c[1]);
 	}
-	// DY: rows iy < Ny-1 when Ny > 3; k = 0 my, 1 centre, 2 py.
-	{
-		bool ok = Ny > 3 && iy < Ny - 1;
-		T cm = 0, cp = 0, c0 = 0;
-		if(ok) {
-			cp = (T)0.5 * (ezz(ix, pyq) + e0) * rYY;
-			cm = (T)0.5 * (ezz(ix, myq) + e0) * rYY;
-			c0 = -cm - cp;
-		}
-		const int rows[3] = {mys, iy, pys};
-		const T c1[3] = {cm, c0, cp};
-		const T L[3] = {rYY, (T)-2 * rYY, rYY};
-		const T dd[3] = {(T)-0.5 * rY, 0, (T)0.5 * rY};
-#pragma unroll
-		for(int k = 0; k < 3; k++) {
-			if(ok) {
-				int cyp = rows[k];
-				T kyy = X.avg(Q_YYTR, ix, cyp), kxy = X.avg(Q_XYTR, ix, cyp);
-				X.entry(L[k], (T)0, c1[k] * kxy, c1[k] * kyy, ix, cyp, dd[k], 1, r[k]);
-			}
-			else r[k][0] = r[k][1] = r[k][2] = r[k][3] = z;
-		}
-#pragma unroll
-		for(int b = 3; b > 0; b--) coef_v(C, V_DY + 3 - b, p) = v4<S>{r[0][b].x, r[0][b].y, r[2][b].x, r[2][b].y};
-		coef_v(C, V_DY + 3, p) = v4<S>{r[0][0].y, r[2][0].y, r[1][0].y, r[1][1].y};
-		coef_u(C, U_DY, p) = mk(r[1][3].y, r[1][2].y);
+	put(v, V_DX, V_DY, false);
+	// DY: rows iy < Ny-1 when Ny > 3; vectors in the order of blocks 3, 2, 1
+	v[0] = v[1] = v[2] = v[3] = zero;
+	if(Ny > 3 && iy < Ny - 1) {
+		const int lm = l0 - LX, ln = lx + LX * lyp;
+		const T cm = (T)0.5 * (Q(CQ_EZ, lm) + e0) * rYY, cp = (T)0.5 * (Q(CQ_EZ, l0 + LX) + e0) * rYY, c0 = -cm - cp;
+		blocks(rYY, (T)0, cm * Q(CQ_KXY, lm), cm * Q(CQ_KYY, lm), lm, m);
+		blocks((T)-2 * rYY, (T)0, c0 * Q(CQ_KXY, l0), c0 * Q(CQ_KYY, l0), l0, c);
+		blocks(rYY, (T)0, cp * Q(CQ_KXY, ln), cp * Q(CQ_KYY, ln), ln, n);
+		const T d = hmu * (T)0.5 * rY * q4;
+		v[0] = v4<S>{d * (va1 + Q(CQ_V1, lm)), m[3], -d * (va1 + Q(CQ_V1, ln)), n[3]};
+		v[1] = v4<S>{d * Q(CQ_V0, lm), m[2], -d * Q(CQ_V0, ln), n[2]};
+		v[2] = v4<S>{d * va0, m[1], -d * va0, n[1]};
+		v[3] = v4<S>{m[0], n[0], c[0], c[1]};
+		uy = mk(c[3], c[2]);
 	}
-	// DXDY: rows ix < Nx-1, iy < Ny-1 when Nx > 3 and Ny > 3; k = pxpy, mxpy, pxmy, mxmy.
-	{
-		bool ok = Nx > 3 && Ny > 3 && ix < Nx - 1 && iy < Ny - 1;
-		T a1 = 0, c1 = 0, a2 = 0, c2 = 0;
-		const T q4 = (T)0.25;
-		if(ok) {
-			a1 = q4 * ezz(pxq, iy) * rXY; c1 = q4 * ezz(mxq, iy) * rXY;
-			a2 = q4 * ezz(ix, pyq) * rXY; c2 = q4 * ezz(ix, myq) * rXY;
+	put(v, V_DY, V_DX, false);
+	// DXDY: rows ix < Nx-1, iy < Ny-1 when Nx > 3 and Ny > 3; corners pxpy, mxpy, pxmy, mxmy
+	v[0] = v[1] = v[2] = v[3] = zero;
+	if(Nx > 3 && Ny > 3 && ix < Nx - 1 && iy < Ny - 1) {
+		const T a1 = q4 * Q(CQ_EZ, l0 + 1) * rXY, c1 = q4 * Q(CQ_EZ, l0 - 1) * rXY;
+		const T a2 = q4 * Q(CQ_EZ, l0 + LX) * rXY, c2 = q4 * Q(CQ_EZ, l0 - LX) * rXY, g0 = q4 * rXY;
+		auto corner = [&](int l, T d01, T d10, T gg, T* im) {
+			const T kxx = Q(CQ_KXX, l), kyy = Q(CQ_KYY, l), kxy = Q(CQ_KXY, l);
+			blocks(d01 * kxy, gg + d01 * kyy, gg + d10 * kxx, d10 * kxy, l, im);
+		};
+		T pp[4], mp[4], pm[4], mm[4];
+		corner(lxp + LX * lyp, a1, a2, -g0, pp);
+		corner(lx - 1 + LX * lyp, -c1, -a2, g0, mp);
+		corner(lxp + LX * (ly - 1), -a1, -c2, g0, pm);
+		corner(l0 - 1 - LX, c1, c2, -g0, mm);
+#pragma unroll
+		for(int b = 0; b < 4; b++) v[b] = v4<S>{pp[b], mp[b], pm[b], mm[b]};
+	}
+	put(v, V_DD, V_DD, true);
+	if(live) {
+		coef_u(C, U_DX, p) = ux;
+		coef_u(C, U_DY, p) = uy;
+	}
+	if(TR) {
+		__syncthreads();
+		st[threadIdx.y * (COEF_TX + 1) + threadIdx.x] = v4<S>{uy.x, uy.y, ux.x, ux.y};
+		__syncthreads();
+		const int ty = tid % TY, tx = tid / TY;
+		if(x0 + tx < Nx && y0 + ty < Ny) {
+			const v4<S> u = st[ty * (COEF_TX + 1) + tx];
+			const int q = (x0 + tx) * Ny + y0 + ty;
+			coef_u(CT, U_DX, q) = mk(u.x, u.y);
+			coef_u(CT, U_DY, q) = mk(u.z, u.w);
 		}
-		const T g0[4] = {-q4 * rXY, q4 * rXY, q4 * rXY, -q4 * rXY};
-		const T d01[4] = {a1, -c1, -a1, c1};
-		const T d10[4] = {a2, -a2, -c2, c2};
-		const int cxs[4] = {pxs, mxs, pxs, mxs};
-		const int cys[4] = {pys, pys, mys, mys};
-		S dq[4][4];
-#pragma unroll
-		for(int k = 0; k < 4; k++) {
-			if(ok) {
-				T kxx = X.avg(Q_XXTR, cxs[k], cys[k]), kyy = X.avg(Q_YYTR, cxs[k], cys[k]);
-				T kxy = X.avg(Q_XYTR, cxs[k], cys[k]);
-				X.entry(d01[k] * kxy, g0[k] + d01[k] * kyy, g0[k] + d10[k] * kxx, d10[k] * kxy,
-					cxs[k], cys[k], (T)0, 0, r[0]);
-			}
-			else r[0][0] = r[0][1] = r[0][2] = r[0][3] = z;
-#pragma unroll
-			for(int b = 0; b < 4; b++) dq[b][k] = r[0][b].y;
-		}
-#pragma unroll
-		for(int b = 0; b < 4; b++) coef_v(C, V_DD + b, p) = v4<S>{dq[b][0], dq[b][1], dq[b][2], dq[b][3]};
 	}
 }
 
@@ -821,50 +815,8 @@ __device__ __forceinline__ cx<R> shfl_xor_c(cx<R> v, int m) {
 // The y-line solves as x-line solves of the transposed frame (x' = y, y' = x, components
 // exchanged): the stencil blocks b become 3 - b (00 <-> 11, 01 <-> 10), the DX and DY stencils
 // exchange, the DXDY corners (px,py), (mx,py), (px,my), (mx,my) become corners 0, 2, 1, 3, and the
-// duplicate-row/column folding and the period-(N-1) wraps map onto themselves. This kernel
-// writes, per wavelength group, the transposed sets those solves read (their phase entries are not
-// used): with the set's order of blocks DY' is DX, DX' is DY and DXDY' block b is DXDY block 3 - b with
-// its two middle corners exchanged. Each block moves a 32x32 tile of one vector (or of the two pairs)
-// through shared memory, coalesced on both sides.
-// Bound: HBM (setup stream).
-constexpr int NCT = NV + 1;  // moves per group: the vectors, and the two pairs together
-template <typename S>
-__global__ void __launch_bounds__(256) k_coef_t(Geom G, const cx<S>* __restrict__ coef, cx<S>* __restrict__ coefT) {
-	__shared__ v4<S> tile[32][33];
-	const int Nx = G.Nx, Ny = G.Ny, N = G.N;
-	const int g = blockIdx.z / NCT, k = blockIdx.z % NCT;
-	const cx<S>* src = coef + (size_t)g * coef_set_size(N);
-	cx<S>* dst = coefT + (size_t)g * coef_set_size(N);
-	const int sv = k < V_DX ? 3 - k : k < V_DY ? k + 4 : k - 4;  // source vector of destination vector k
-	const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-	for(int r = threadIdx.y; r < 32; r += blockDim.y) {
-		const int x = x0 + threadIdx.x, y = y0 + r;
-		if(x < Nx && y < Ny) {
-			const int q = y * Nx + x;
-			v4<S> v;
-			if(k == NV) {
-				const cx<S> a = coef_u(src, U_DY, q), b = coef_u(src, U_DX, q);
-				v = v4<S>{a.x, a.y, b.x, b.y};
-			}
-			else v = coef_v(src, sv, q);
-			if(k < V_DX) v = v4<S>{v.x, v.z, v.y, v.w};
-			tile[r][threadIdx.x] = v;
-		}
-	}
-	__syncthreads();
-	for(int r = threadIdx.y; r < 32; r += blockDim.y) {
-		const int y = y0 + threadIdx.x, x = x0 + r;  // destination row x, column y
-		if(x < Nx && y < Ny) {
-			const int q = x * Ny + y;
-			const v4<S> v = tile[threadIdx.x][r];
-			if(k == NV) {
-				coef_u(dst, U_DX, q) = mk(v.x, v.y);
-				coef_u(dst, U_DY, q) = mk(v.z, v.w);
-			}
-			else coef_v(dst, k, q) = v;
-		}
-	}
-}
+// duplicate-row/column folding and the period-(N-1) wraps map onto themselves. k_coef writes the
+// transposed sets those solves read (their phase entries are not used).
 
 // Pre-factorisation of the periodic line solves (I - mu*R_cc) x = b per (group, comp, line), in
 // the plan's precision. Restates shifted_block_vmult_inv (BlockSparseMatrix.cpp:195-258 and

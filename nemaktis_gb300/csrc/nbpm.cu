@@ -339,6 +339,9 @@ struct Plan : PlanBase {
 	std::vector<std::string> tune_notes;  // per sample: how its configuration was chosen
 	std::vector<SolveCfg> scfg;
 
+	// Rows of k_coef's tiles: 8, or 4 in FP64, where twice the blocks halve the FP64 work of a small mesh's warps
+	static constexpr int COEF_TY = sizeof(R) == sizeof(double) ? 4 : 8;
+
 	// Makes h's lane current: its streams, events and workspace.
 	void select(SampleHost& h) {
 		auto& L = h.lane;
@@ -503,6 +506,8 @@ struct Plan : PlanBase {
 			(int)((size_t)16 * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>))));
 		CK(cudaFuncSetAttribute(k_shift_fused<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)((size_t)4 * (SHT + 6) * (SHT + 6) * sizeof(cx<R>))));
+		CK(cudaFuncSetAttribute(k_coef<R, COEF_TY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			(int)coef_smem<R, COEF_TY>(true)));
 		CK(cudaFuncSetAttribute(k_shift_pair, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			(int)((size_t)4 * (SHT + 6) * (SHT + 6) * sizeof(cx<float>))));
 		if(sizeof(R) == sizeof(float)) {
@@ -1108,8 +1113,11 @@ struct Plan : PlanBase {
 			});
 			// coef(iz) overwrites the set the transition of slab iz-1 read (slab iz-2)
 			if(iz >= 1) CK(cudaStreamWaitEvent(streamB, eTrans, 0));
-			launch("coef", (double)N * ng * (2 * NQ * sizeof(R) + CSET * sizeof(R) + (wts ? 16 : 0)), [&] {
-				k_coef<R><<<pgrid(N, ng, 128), 128, 0, cs>>>(QA, QB, wts, iz, Gm, gps, C);
+			cx<R>* CT = scf.Mxt ? W->coefT.as<cx<R>>() + (size_t)(iz & 1) * ng * coef_set_size(N) : nullptr;
+			launch("coef", (double)N * ng * (2 * NQ * sizeof(R) + (CT ? 2 * CSET - 6 : CSET) * sizeof(R) + (wts ? 16 : 0)), [&] {
+				const dim3 gr((unsigned)((Nx + COEF_TX - 1) / COEF_TX), (unsigned)((Ny + COEF_TY - 1) / COEF_TY), (unsigned)ng), bl(32, COEF_TY);
+				if(CT) k_coef<R, COEF_TY, true><<<gr, bl, coef_smem<R, COEF_TY>(true), cs>>>(QA, QB, wts, iz, Gm, gps, C, CT);
+				else k_coef<R, COEF_TY, false><<<gr, bl, coef_smem<R, COEF_TY>(false), cs>>>(QA, QB, wts, iz, Gm, gps, C, nullptr);
 			});
 			CK(cudaEventRecord(eCoef, streamB));
 			// factor(iz) overwrites the half the line solves of slab iz-2 used
@@ -1123,15 +1131,9 @@ struct Plan : PlanBase {
 				k_factor_chunked<R, 0><<<dim3((unsigned)((Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
 					Gm, ng, scf.Mx, 32 * scf.WPLx, 1, C, fx, scf.plane_x, lx);
 			});
-			cx<R>* CT = scf.Mxt ? W->coefT.as<cx<R>>() + (size_t)(iz & 1) * ng * coef_set_size(N) : nullptr;
 			if(scf.Mxt) {
-				// y-lines as x-lines of the transposed frame: transposed coefficients and diagonals,
-				// then the x-line factorisation of that frame
+				// y-lines as x-lines of the transposed frame
 				const Geom Gt = transposed(Gm);
-				launch("coef_t", 2.0 * N * ng * (CSET - 6) * sizeof(R), [&] {
-					k_coef_t<R><<<dim3((unsigned)((Nx + 31) / 32), (unsigned)((Ny + 31) / 32), (unsigned)(ng * NCT)), dim3(32, 8), 0,
-						cs>>>(Gm, C, CT);
-				});
 				rec_factor_part("factor_y", fb, Gt, ng, scf.Mxt, scf.WPLt, CT, fy, scf.plane_y, ly);
 			}
 			else {
