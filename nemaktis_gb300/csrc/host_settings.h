@@ -16,6 +16,8 @@
 #include <utility>
 #include <vector>
 
+#include <omp.h>
+
 #include "host_expr.h"
 #include "host_json.h"
 
@@ -209,7 +211,8 @@ inline BackendSettings parse_settings(const std::string& json_str) {
 // formula's sign changes disagree with the mask, the reference prints a notice and falls
 // back to 0.5/0.5 everywhere (its resize at :111 truncates the array; the evident intent,
 // uniform weights, is applied here).
-inline void mask_weights(const BackendSettings& s, const double* mask_vals, const std::string& formula,
+// Returns whether any weight differs from 0.5. The vectors keep their memory from call to call.
+inline bool mask_weights(const BackendSettings& s, const double* mask_vals, const std::string& formula,
 		std::vector<unsigned char>& mask_out, std::vector<double>& w_out) {
 	int Nx = s.Nx, Ny = s.Ny, Nz = s.Nz;
 	size_t nv = (size_t)Nx * Ny * Nz;
@@ -220,45 +223,54 @@ inline void mask_weights(const BackendSettings& s, const double* mask_vals, cons
 	w_out.resize(nw);
 	#pragma omp parallel for schedule(static)
 	for(long long i = 0; i < (long long)nw; i++) w_out[i] = 0.5;
-	if(formula.empty() || Nz < 2) return;
+	if(formula.empty() || Nz < 2) return false;
 	Expr ex;
 	try { ex = Expr(formula, {"x", "y", "z"}); }
 	catch(ExprError& e) { throw BackendError(E_EXPR, std::string("Wrong mask formula: ") + e.what()); }
-	int failed = 0;
-	#pragma omp parallel for reduction(|:failed) schedule(dynamic, 64)
-	for(long long iperp = 0; iperp < (long long)Nx * Ny; iperp++) {
-		int ix = (int)(iperp % Nx), iy = (int)(iperp / Nx);
-		double v[3] = {(ix - 0.5 * (Nx - 1)) * s.dx, (iy - 0.5 * (Ny - 1)) * s.dy, 0};
-		// the formula at the upper plane of a cell is the one at the lower plane of the next
-		// (the same z), so each plane is evaluated once
-		double f_next = 0;
-		for(int iz = 0; iz < Nz - 1; iz++) {
-			size_t i = iperp + (size_t)Nx * Ny * iz;
-			double zi = (iz - 0.5 * (Nz - 1)) * s.dz, zm = zi, zp = (iz + 1 - 0.5 * (Nz - 1)) * s.dz;
-			double& z = v[2];
-			double fm;
-			if(iz == 0) { z = zm; fm = ex.eval(v); }
-			else fm = f_next;
-			z = zp; double fp = ex.eval(v);
-			f_next = fp;
-			if(fm * fp <= 0) {
+	// the formula on the mesh from tables of its one-variable parts (pow of a coordinate: once per
+	// coordinate value instead of once per voxel), inside a cell with x and y from the tables
+	std::vector<double> ax[3];
+	for(int i = 0; i < Nx; i++) ax[0].push_back((i - 0.5 * (Nx - 1)) * s.dx);
+	for(int i = 0; i < Ny; i++) ax[1].push_back((i - 0.5 * (Ny - 1)) * s.dy);
+	for(int i = 0; i < Nz; i++) ax[2].push_back((i - 0.5 * (Nz - 1)) * s.dz);
+	const Expr::Grid mesh(ex, ax, 7u), cell(ex, ax, 3u);
+	const size_t per = (mesh.depth() + 1) * (size_t)Nz;
+	std::vector<double> scratch(per * (size_t)omp_get_max_threads());
+	int failed = 0, changed = 0;
+	#pragma omp parallel reduction(|:failed, changed) num_threads((int)(scratch.size() / per))
+	{
+		double* f = scratch.data() + per * (size_t)omp_get_thread_num();
+		#pragma omp for schedule(dynamic, 64)
+		for(long long iperp = 0; iperp < (long long)Nx * Ny; iperp++) {
+			const int ix = (int)(iperp % Nx), iy = (int)(iperp / Nx);
+			mesh.line((size_t)ix, (size_t)iy, (size_t)Nz, f, f + Nz);
+			for(int iz = 0; iz < Nz - 1; iz++) {
+				double fm = f[iz];
+				if(!(fm * f[iz + 1] <= 0)) continue;
+				const size_t i = iperp + (size_t)Nx * Ny * iz;
 				if(mask_out[i] == mask_out[i + (size_t)Nx * Ny]) failed = 1;
 				// bisection to 1e-3 dz; fm always holds the formula at zm
+				const double zi = ax[2][iz];
+				double zm = zi, zp = ax[2][iz + 1], z = zp;
 				while(std::abs(zp - zm) >= 1e-3 * s.dz) {
-					z = 0.5 * (zp + zm); double f = ex.eval(v);
-					if(f == 0) break;
-					else if(f * fm < 0) zp = z;
-					else { zm = z; fm = f; }
+					z = 0.5 * (zp + zm);
+					const double fz = cell.point((size_t)ix, (size_t)iy, z);
+					if(fz == 0) break;
+					else if(fz * fm < 0) zp = z;
+					else { zm = z; fm = fz; }
 				}
 				w_out[2 * i] = (z - zi) / s.dz;
 				w_out[2 * i + 1] = 1 - w_out[2 * i];
+				if(w_out[2 * i] != 0.5) changed = 1;
 			}
 		}
 	}
 	if(failed) {
 		std::printf("Mask values do not corresponds to the given formula, will ignore interpolation correction\n");
 		std::fill(w_out.begin(), w_out.end(), 0.5);
+		return false;
 	}
+	return changed != 0;
 }
 
 }  // namespace nbpm

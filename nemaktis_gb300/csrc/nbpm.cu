@@ -136,6 +136,9 @@ struct SampleHost {
 	int fd = 3;
 	std::vector<unsigned char> mask;
 	std::vector<double> wts;
+	// the next call's, kept with the plan: their pages (17 bytes per voxel) are touched once
+	std::vector<unsigned char> mask_next;
+	std::vector<double> wts_next;
 	bool has_mask = false, has_wts = false;
 	double* E = nullptr;  // user buffer, complex128 interleaved
 	int G = 0, Nq = 0, spg = 0, slots = 0;
@@ -417,10 +420,8 @@ struct Plan : PlanBase {
 			h->E = in.E_field_vals;
 			if(in.mask_vals) {
 				h->has_mask = true;
-				mask_weights(s, in.mask_vals, in.mask_formula ? std::string(in.mask_formula) : std::string(),
+				h->has_wts = mask_weights(s, in.mask_vals, in.mask_formula ? std::string(in.mask_formula) : std::string(),
 					h->mask, h->wts);
-				h->has_wts = false;
-				for(double w : h->wts) if(w != 0.5) { h->has_wts = true; break; }
 			}
 			h->geom.Nx = s.Nx; h->geom.Ny = s.Ny; h->geom.N = s.Nx * s.Ny; h->geom.Nz = s.Nz;
 			h->geom.spg = h->spg; h->geom.Nq = h->Nq;
@@ -903,8 +904,6 @@ struct Plan : PlanBase {
 				return false;
 			}
 		}
-		std::vector<std::vector<unsigned char>> masks(ns);
-		std::vector<std::vector<double>> wts(ns);
 		for(int i = 0; i < ns; i++) {
 			SampleHost& h = *S[i];
 			const nbpm_sample& in = samples[i];
@@ -914,17 +913,16 @@ struct Plan : PlanBase {
 				return false;
 			if(in.mask_vals) {
 				if((size_t)in.n_mask_vals != h.nvox) return false;
-				mask_weights(h.s, in.mask_vals, in.mask_formula ? std::string(in.mask_formula) : std::string(), masks[i], wts[i]);
-				bool nonuniform = false;
-				for(double w : wts[i]) if(w != 0.5) { nonuniform = true; break; }
-				if(nonuniform != h.has_wts) return false;
+				if(mask_weights(h.s, in.mask_vals, in.mask_formula ? std::string(in.mask_formula) : std::string(), h.mask_next,
+						h.wts_next) != h.has_wts)
+					return false;
 			}
 		}
 		for(int i = 0; i < ns; i++) {
 			SampleHost& h = *S[i];
 			h.lc = samples[i].lc_field_vals;
 			h.E = samples[i].E_field_vals;
-			if(h.has_mask) { h.mask.swap(masks[i]); h.wts.swap(wts[i]); }
+			if(h.has_mask) { h.mask.swap(h.mask_next); h.wts.swap(h.wts_next); }
 		}
 		return true;
 	}
