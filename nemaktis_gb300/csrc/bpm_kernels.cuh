@@ -61,7 +61,7 @@ __device__ __forceinline__ const cx<S>& part_e(const cx<S>* Fc, int k, int CH, i
 // derivatives, which only the outer entries of DX blocks 0, 1, 2 and of DY blocks 1, 2, 3 have. So an
 // entry is one real number (its imaginary part) except those twelve, 52 numbers in place of 80, and a
 // tap with a real number costs two multiply-adds in place of four. They are kept as 12 vectors of
-// four, which a thread loads at once, and two pairs (m, c, p: the entries of the previous point, the
+// four and two pairs (m, c, p: the entries of the previous point, the
 // point itself and the next one; the index is the block):
 //   V_DD + b   DXDY block b: (px,py), (mx,py), (px,my), (mx,my)
 //   V_DX + i   DX block i = 0, 1, 2: m (complex), p (complex)       V_DX + 3: m3, p3, c3, c2    U_DX: c0, c1
@@ -75,13 +75,19 @@ enum { CSET = 4 * NV + 2 * NU + 6 };  // scalars per point: vectors, pairs, 3 co
 __host__ __device__ __forceinline__ size_t coef_set_size(int N) { return (size_t)(CSET / 2) * (((size_t)N + 31) & ~(size_t)31); }
 template <typename C>
 __device__ __forceinline__ C* coef_tile(C* coef, int p) { return coef + (size_t)(p >> 5) * (CSET / 2 * 32); }
+// half h of vector k: a tile's halves are apart, for threads that need one of them at a time (StripRhs) and so that
+// a warp's 16-byte accesses to FP64 halves are contiguous
+template <typename C>
+__device__ __forceinline__ C& coef_h(C* coef, int k, int h, int p) { return coef_tile(coef, p)[(2 * k + h) * 32 + (p & 31)]; }
 template <typename S>
-__device__ __forceinline__ const v4<S>& coef_v(const cx<S>* coef, int k, int p) {
-	return reinterpret_cast<const v4<S>*>(coef_tile(coef, p))[k * 32 + (p & 31)];
+__device__ __forceinline__ v4<S> coef_v(const cx<S>* coef, int k, int p) {
+	const cx<S> a = coef_h(coef, k, 0, p), b = coef_h(coef, k, 1, p);
+	return v4<S>{a.x, a.y, b.x, b.y};
 }
 template <typename S>
-__device__ __forceinline__ v4<S>& coef_v(cx<S>* coef, int k, int p) {
-	return reinterpret_cast<v4<S>*>(coef_tile(coef, p))[k * 32 + (p & 31)];
+__device__ __forceinline__ void coef_put(cx<S>* coef, int k, int p, v4<S> v) {
+	coef_h(coef, k, 0, p) = mk(v.x, v.y);
+	coef_h(coef, k, 1, p) = mk(v.z, v.w);
 }
 // pairs and phase entries follow the vectors
 template <typename C>
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(32 * TY) k_coef(const S* __restrict__ QA, cons
 	auto put = [&](const v4<S>* v, int k, int kt, bool corners) {
 		if(live) {
 #pragma unroll
-			for(int j = 0; j < 4; j++) coef_v(C, k + j, p) = v[j];
+			for(int j = 0; j < 4; j++) coef_put(C, k + j, p, v[j]);
 		}
 		if(TR) {
 			__syncthreads();  // the vectors before these have been written
@@ -503,7 +509,7 @@ __global__ void __launch_bounds__(32 * TY) k_coef(const S* __restrict__ QA, cons
 			const int ty = tid % TY, tx = tid / TY;
 			if(x0 + tx < Nx && y0 + ty < Ny) {
 #pragma unroll
-				for(int j = 0; j < 4; j++) coef_v(CT, kt + j, (x0 + tx) * Ny + y0 + ty) = st[(j * TY + ty) * (COEF_TX + 1) + tx];
+				for(int j = 0; j < 4; j++) coef_put(CT, kt + j, (x0 + tx) * Ny + y0 + ty, st[(j * TY + ty) * (COEF_TX + 1) + tx]);
 			}
 		}
 	};

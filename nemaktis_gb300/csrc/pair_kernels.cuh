@@ -30,65 +30,109 @@ __device__ __forceinline__ pr at_byte(const pr* f, unsigned o) {
 	return *reinterpret_cast<const pr*>(reinterpret_cast<const char*>(f) + o);
 }
 
-// Right-hand side of x-lines (composite_m with KIND ST_EXPL_Y or ST_WOOD_X) of one component at point
-// (x, iy), x < Nx - 1, for a pair; f0, f1: the pair's component planes. The row offsets are bytes.
-template <int KIND>
-struct PairRhs {
+// Right-hand sides of x-lines (composite_m with KIND ST_EXPL_Y or ST_WOOD_X) of one component for a pair, at
+// column x < Nx - 1 of the L lines iy0, iy0 + 1, ... (pairs have Nx, Ny > 3); f0, f1: the pair's component planes. A
+// field row is loaded once and used by the up to three lines it touches: 4 lines with corners take 24 instead of 32
+// corner loads, and 6 instead of 12 in the column itself. Each case is straight-line code, so that the loads of later
+// rows are issued before the first are used: with the component and the corners as branches inside the row loop the
+// explicit step at 256x256 took 508 us, 324 us without. Coefficients come by halves, as a row needs them: whole
+// vectors held for three rows spilled (explicit step 515 us). Rows of lines past Ny - 1 are held inside the
+// plane; their results are not used. The row offsets are bytes.
+template <int KIND, int L>
+struct StripRhs {
 	const cx<float>* C;
 	const pr *f0, *f1;
-	int Nx, Ny, iy, yy, comp;
-	bool both;
-	unsigned r0, rm, rp, ro;  // rows of the point, of its y neighbours, and iy itself
-	__device__ __forceinline__ PairRhs(const cx<float>* C_, const pr* f, const Geom& G, int comp_, int iy_) : C(C_), f0(f), f1(f + G.N),
-			Nx(G.Nx), Ny(G.Ny), iy(iy_), comp(comp_) {
-		constexpr bool XDIR = KIND == ST_WOOD_X;
-		const bool mixed = XDIR ? comp == 0 : comp == 1;
-		both = mixed && Nx > 3 && Ny > 3;
-		yy = (!XDIR || both) && iy == Ny - 1 ? 0 : iy;
-		const unsigned w = (unsigned)Nx * (unsigned)sizeof(pr);
-		ro = (unsigned)iy * w;
-		r0 = (unsigned)yy * w;
-		rm = yy == 0 ? (unsigned)max(Ny - 2, 0) * w : r0 - w;
-		rp = yy == Ny - 2 ? 0u : r0 + w;
+	int Nx, Ny, iy0, comp;
+	__device__ __forceinline__ StripRhs(const cx<float>* C_, const pr* f, const Geom& G, int comp_, int iy0_) : C(C_), f0(f), f1(f + G.N),
+			Nx(G.Nx), Ny(G.Ny), iy0(iy0_), comp(comp_) {}
+	// row iy0 - 1 + k on the periodic lines 0 .. Ny - 2
+	__device__ __forceinline__ int row(int k) const {
+		const int P = Ny - 1, r = iy0 - 1 + k;
+		return r < 0 ? r + P : r < P ? r : min(r - P, P);
 	}
-	__device__ __forceinline__ pr operator()(int x) const {
+	// the two corners of a row
+	static __device__ __forceinline__ pr corners(cx<float> v, pr m, pr p, pr c) { return pifma(v.y, m, pifma(v.x, p, c)); }
+	__device__ __forceinline__ void operator()(int x, pr (&out)[L]) const {
 		constexpr unsigned SZ = sizeof(pr);
-		const unsigned o = (unsigned)x * SZ;
+		const unsigned o = (unsigned)x * SZ, w = (unsigned)Nx * SZ;
 		const unsigned om = x == 0 ? (unsigned)(Nx - 2) * SZ : o - SZ, op = x == Nx - 2 ? 0u : o + SZ;
-		const int p = x + Nx * yy;
-		pr out{0, 0, 0, 0};
-		auto corners = [&](v4<float> v, const pr* f) {
-			out = pifma(v.w, at_byte(f, rm + om), pifma(v.z, at_byte(f, rm + op), pifma(v.y, at_byte(f, rp + om),
-				pifma(v.x, at_byte(f, rp + op), out))));
-		};
+#pragma unroll
+		for(int l = 0; l < L; l++) out[l] = pr{0, 0, 0, 0};
 		if(KIND == ST_WOOD_X) {
-			auto taps = [&](v4<float> v, float c, const pr* f) {
-				out = pfma(mk(v.z, v.w), at_byte(f, r0 + op), pifma(c, at_byte(f, r0 + o), pfma(mk(v.x, v.y), at_byte(f, r0 + om), out)));
-			};
-			if(comp == 0) {
-				taps(coef_v(C, V_DX + 1, p), coef_u(C, U_DX, p).y, f1);
-				if(both) { corners(coef_v(C, V_DD + 0, p), f0); corners(coef_v(C, V_DD + 1, p), f1); }
-			}
-			else taps(coef_v(C, V_DX + 2, p), coef_v(C, V_DX + 3, p).w, f0);
-			return out;
+			if(comp == 0) wood0(x, o, om, op, w, out);
+			else wood1(x, o, om, op, w, out);
 		}
-		if(Ny > 3) {
-			auto taps = [&](v4<float> v, float c, const pr* f) {
-				out = pfma(mk(v.z, v.w), at_byte(f, rp + o), pifma(c, at_byte(f, r0 + o), pfma(mk(v.x, v.y), at_byte(f, rm + o), out)));
-			};
-			if(comp == 0) {
-				const v4<float> w = coef_v(C, V_DY + 3, p);
-				out = pifma(w.y, at_byte(f0, rp + o), pifma(w.z, at_byte(f0, r0 + o), pifma(w.x, at_byte(f0, rm + o), out)));
-				taps(coef_v(C, V_DY + 2, p), w.w, f1);
+		else if(comp == 0) expl<0>(x, o, om, op, w, out);
+		else expl<1>(x, o, om, op, w, out);
+	}
+	__device__ __forceinline__ void wood0(int x, unsigned o, unsigned om, unsigned op, unsigned w, pr (&out)[L]) const {
+#pragma unroll
+		for(int k = 0; k < L + 2; k++) {
+			const int yr = row(k), q = x + Nx * yr;
+			const unsigned r = (unsigned)yr * w;
+			const pr am = at_byte(f0, r + om), ap = at_byte(f0, r + op), bm = at_byte(f1, r + om), bp = at_byte(f1, r + op);
+			if(k >= 2) {
+				const int qp = x + Nx * row(k - 1);
+				out[k - 2] = corners(coef_h(C, V_DD + 0, 0, qp), am, ap, corners(coef_h(C, V_DD + 1, 0, qp), bm, bp, out[k - 2]));
 			}
-			else {
-				const cx<float> u = coef_u(C, U_DY, p);
-				taps(coef_v(C, V_DY + 0, p), u.x, f1);
-				taps(coef_v(C, V_DY + 1, p), u.y, f0);
-				if(both) { corners(coef_v(C, V_DD + 3, p), f1); corners(coef_v(C, V_DD + 2, p), f0); }
+			if(k >= 1 && k <= L) {
+				const v4<float> v = coef_v(C, V_DX + 1, q);
+				pr& t = out[k - 1];
+				t = pfma(mk(v.z, v.w), bp, pifma(coef_u(C, U_DX, q).y, at_byte(f1, r + o), pfma(mk(v.x, v.y), bm, t)));
+			}
+			if(k < L) {
+				const int qn = x + Nx * row(k + 1);
+				out[k] = corners(coef_h(C, V_DD + 0, 1, qn), am, ap, corners(coef_h(C, V_DD + 1, 1, qn), bm, bp, out[k]));
 			}
 		}
-		return padd(out, at_byte(comp == 0 ? f0 : f1, ro + o));
+	}
+	__device__ __forceinline__ void wood1(int x, unsigned o, unsigned om, unsigned op, unsigned w, pr (&out)[L]) const {
+#pragma unroll
+		for(int l = 0; l < L; l++) {
+			const int yy = min(iy0 + l, Ny - 1), q = x + Nx * yy;
+			const unsigned r = (unsigned)yy * w;
+			const v4<float> v = coef_v(C, V_DX + 2, q);
+			out[l] = pfma(mk(v.z, v.w), at_byte(f0, r + op), pifma(coef_h(C, V_DX + 3, 1, q).y, at_byte(f0, r + o),
+				pmul(mk(v.x, v.y), at_byte(f0, r + om))));
+		}
+	}
+	template <int COMP>
+	__device__ __forceinline__ void expl(int x, unsigned o, unsigned om, unsigned op, unsigned w, pr (&out)[L]) const {
+		const pr *fa = COMP == 0 ? f0 : f1, *fb = COMP == 0 ? f1 : f0;  // this component, the other one
+		pr own[L];
+#pragma unroll
+		for(int k = 0; k < L + 2; k++) {
+			const unsigned r = (unsigned)row(k) * w;
+			const pr a = at_byte(fa, r + o), b = at_byte(fb, r + o);
+			pr am, ap, bm, bp;
+			if(COMP == 1) {
+				am = at_byte(fa, r + om);
+				ap = at_byte(fa, r + op);
+				bm = at_byte(fb, r + om);
+				bp = at_byte(fb, r + op);
+			}
+			if(k >= 2) {
+				const int q = x + Nx * row(k - 1);
+				pr& t = out[k - 2];
+				if(COMP == 0) t = pfma(coef_h(C, V_DY + 2, 1, q), b, pifma(coef_h(C, V_DY + 3, 0, q).y, a, t));
+				else t = pfma(coef_h(C, V_DY + 1, 1, q), b, pfma(coef_h(C, V_DY + 0, 1, q), a, t));
+				if(COMP == 1) t = corners(coef_h(C, V_DD + 2, 0, q), bm, bp, corners(coef_h(C, V_DD + 3, 0, q), am, ap, t));
+				t = padd(t, own[k - 2]);
+			}
+			if(k >= 1 && k <= L) {
+				const int q = x + Nx * row(k);
+				const cx<float> u = COMP == 0 ? coef_h(C, V_DY + 3, 1, q) : coef_u(C, U_DY, q);
+				out[k - 1] = pifma(u.y, b, pifma(u.x, a, out[k - 1]));
+				own[k - 1] = iy0 + k - 1 == Ny - 1 ? at_byte(fa, (unsigned)(Ny - 1) * w + o) : a;
+			}
+			if(k < L) {
+				const int q = x + Nx * row(k + 1);
+				pr& t = out[k];
+				if(COMP == 0) t = pfma(coef_h(C, V_DY + 2, 0, q), b, pifma(coef_h(C, V_DY + 3, 0, q).x, a, t));
+				else t = pfma(coef_h(C, V_DY + 1, 0, q), b, pfma(coef_h(C, V_DY + 0, 0, q), a, t));
+				if(COMP == 1) t = corners(coef_h(C, V_DD + 2, 1, q), bm, bp, corners(coef_h(C, V_DD + 3, 1, q), am, ap, t));
+			}
+		}
 	}
 };
 
@@ -129,11 +173,14 @@ __device__ __forceinline__ void pair_backward(pr* vb, const cx<float>* Fc, int C
 // Partitioned x-line solve with its right-hand side (k_solve_xc) for a pair of slots: a warp per line, 4
 // lines per block; the blocks of a line group, both components and all pairs of the wavelength follow each
 // other, so that they find its coefficients and factors in L2.
-// Bound: L1 wavefronts (70 %) and load latency. 7 blocks per SM: at 8 the 64 registers spill (206 against
-// 195 ms for the whole step), at 6 too few warps wait for loads (205 ms). 256x256, 16 wavelengths, 13 q: Woodbury
-// solves 477 us as k_solve_xc with two slots per thread, 402 us here; explicit step 491 and 378 us. The rows of
-// a block staged in shared memory (cp.async) gave 438 and 415 us, x neighbours from lane shuffles 478 and
-// 498 us.
+// Bound: L1 wavefronts and load latency. 7 blocks per SM: at 8 the 64 registers spill (206 against 195 ms
+// for the whole step), at 6 too few warps wait for loads (205 ms). Right-hand sides: a thread takes a column of
+// the block's 4 lines (StripRhs), for short lines (M < 6) a point of one line, where a column per thread leaves warps
+// without work (64x64: explicit step 16.6 us, with 2 lines per thread 18.3 us, with 4 lines 22.6 us; 224x224: 55.0
+// us with 1 or 2 lines, 50.7 us with 4). 256x256, 16 wavelengths, 13 q: Woodbury solves 477 us as k_solve_xc with
+// two slots per thread, 402 us here with a line per warp for the right-hand sides too, 324 us with strips;
+// explicit step 491, 378 and 324 us. The rows of a block staged in shared memory (cp.async) gave 438 and
+// 415 us, x neighbours from lane shuffles 478 and 498 us.
 template <int M, int KIND, int OUT>
 __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __restrict__ coef,
 		const cx<float>* __restrict__ fac, size_t plane, const cx<double>* __restrict__ lsc, const pr* __restrict__ src,
@@ -152,17 +199,25 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 	const int n = Nx - 1;
 	const size_t pair = (size_t)g * nch + ch;
 	const pr* f = src + pair * 2 * N;
+	{
+		constexpr int L = M >= 6 ? 4 : 1, COLS = 128 * L / LT;
+		const int l0 = threadIdx.x / COLS * L;
+		const StripRhs<KIND, L> rhs(coef + (size_t)g * coef_set_size(N), f, G, c, line0 + l0);
+		if(line0 + l0 < Ny) {
+#pragma unroll 1
+			for(int e = threadIdx.x % COLS; e < 32 * M; e += COLS) {
+				pr v[L];
+				if(e < n) rhs(e, v);
+#pragma unroll
+				for(int l = 0; l < L; l++) bufs[(l0 + l) * WS + e / M * PM + e % M] = e < n ? v[l] : pr{0, 0, 0, 0};  // chunk e / M
+			}
+		}
+		__syncthreads();
+	}
 	if(iy < Ny) {
 		const cx<float>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
 		const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
 		pr* buf = bufs + warp * WS;
-		const PairRhs<KIND> rhs(coef + (size_t)g * coef_set_size(N), f, G, c, iy);
-#pragma unroll 1
-		for(int t = 0; t < M; t++) {
-			const int e = lane + 32 * t;
-			buf[e / M * PM + e % M] = e < n ? rhs(e) : pr{0, 0, 0, 0};  // chunk e / M
-		}
-		__syncwarp();
 		if(K >= 0) {
 			pr* vb = buf + lane * PM;
 			pr d, yf;
@@ -239,8 +294,10 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 // The same for long lines: W warps per line and 2 lines per block (32-byte segments of the transposed plane), 32*W
 // chunks of M points, border unknowns of chunks in different warps through shared memory as in k_solve_xw.
 // REGS: registers per thread, by the launch (launch_solve_pair).
-// 1024x1024, 2 wavelengths, 7 q: Woodbury solves 1007 us as k_solve_xw, 508 us here (a line's coefficients and
-// factors, 190 MB per wavelength, were read again from DRAM for every two slots), explicit step 810 and 503 us.
+// 1024x1024, 2 wavelengths, 7 q: Woodbury solves 1007 us as k_solve_xw (a line's coefficients and factors, 190 MB
+// per wavelength, were read again from DRAM for every two slots), 508 us here, 462 us with the right-hand
+// sides of both lines from one thread (StripRhs); explicit step 810, 503 and 425 us. 4 lines per block: 461 and 491
+// us; 512x512, 14 pairs: 14.4 ms a step with 2 lines, 16.2 ms with 4.
 template <int M, int KIND, int OUT, int REGS>
 __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __restrict__ coef,
 		const cx<float>* __restrict__ fac, size_t plane, const cx<double>* __restrict__ lsc, const pr* __restrict__ src,
@@ -264,12 +321,14 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	const cx<float>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, CH);
 	const int K = live ? (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x : 0;
 	pr* buf = bufs + ln * WS;
-	if(live) {
-		const PairRhs<KIND> rhs(coef + (size_t)g * coef_set_size(N), f, G, c, iy);
+	{
+		const StripRhs<KIND, LT> rhs(coef + (size_t)g * coef_set_size(N), f, G, c, lb * LT);
 #pragma unroll 1
-		for(int t = 0; t < M; t++) {
-			const int e = ci + CH * t;
-			buf[e / M * PM + e % M] = e < n ? rhs(e) : pr{0, 0, 0, 0};
+		for(int e = threadIdx.x; e < M * CH; e += LT * CH) {
+			pr v[LT];
+			if(e < n) rhs(e, v);
+#pragma unroll
+			for(int l = 0; l < LT; l++) bufs[l * WS + e / M * PM + e % M] = e < n ? v[l] : pr{0, 0, 0, 0};
 		}
 	}
 	// the barriers are the block's: both lines take the larger number of steps

@@ -31,7 +31,7 @@ bool launch_solve_pair(cudaStream_t st, bool dep, int M, int W, int kind, int ou
 	const dim3 grid((unsigned)((size_t)((G.Ny + 1) / 2) * 2 * G.Nq), (unsigned)ng);
 	const size_t smem = (size_t)2 * (32 * W * part_pitch(M) + 4 + 4 * W + 2) * sizeof(pr);
 	// Registers: lines of 3 warps and more make blocks of 192 threads and more, of which 64 registers leave
-	// 30 warps per SM resident (1024x1024: 100.5 ms a step with 64, 108 with 80); blocks of two-warp lines, 128
+	// 30 warps per SM resident (1024x1024: 83.8 ms a step with 64, 90.4 with 72); blocks of two-warp lines, 128
 	// threads, take 72 as k_solve_xp, or 96 when the launch has too few warps to fill the SMs anyway
 	// (512x512, one pair: 21.4 ms with 96, 23.2 with 72, 23.8 with 64).
 	const int regs = W > 2 ? 64 : (size_t)grid.x * grid.y * 4 <= (size_t)152 * 20 ? 96 : 72;
