@@ -2575,6 +2575,58 @@ __device__ void shift_point_exact(const Geom& G, const ShiftParams& P, const cx<
 	}
 }
 
+// The window of a transition tile: the tile's points inside the plane and, along a filtered axis, 3 more per
+// shift; phase_A is applied as it is loaded. Its points are dealt out to the 256 threads one after the other: a
+// warp per row of 38 points took two rounds, the second with 6 lanes, and the loads of a point waited for those of
+// the point before. Here the loads of U points are in flight together. 256x256: FP32 pairs, 16
+// wavelengths, 13 q, 472 us as rows, 364 us so; FP64, 3 wavelengths, 13 q, 1082 and 957 us. The clipping to the plane
+// spares a 97x75 mesh a third of its window points (FP64, 3 wavelengths, 7 q: 137 and 110 us).
+template <typename R>
+struct ShiftWindow {
+	static constexpr int U = sizeof(R) == 4 ? 3 : 2, PA = SHT + 7;
+	int wx, wy, magic;
+	int* at;  // [2][SHT + 6]: the columns, and the first points of the rows
+	// places: shared memory for 2 * (SHT + 6) numbers. By all threads of the block, with a barrier.
+	__device__ __forceinline__ ShiftWindow(const Geom& G, const ShiftParams& P, int nsh, int x0, int y0, int* places) : at(places) {
+		const bool ax = G.Nx > 3, ay = G.Ny > 3;
+		wx = min(SHT, G.Nx - x0) + (ax ? 3 * nsh : 0);
+		wy = min(SHT, G.Ny - y0) + (ay ? 3 * nsh : 0);
+		magic = 65536 / wx + 1;  // e / wx = e * magic >> 16 for e < 38 * wx, wx <= 38
+		const int u = threadIdx.x, v = threadIdx.x - 64;
+		if(u < wx) at[u] = ax ? pmod(x0 + nsh * (P.msx - 1) + u, G.Nx - 1) : x0 + u;
+		if(v >= 0 && v < wy) at[SHT + 6 + v] = G.Nx * (ay ? pmod(y0 + nsh * (P.msy - 1) + v, G.Ny - 1) : y0 + v);
+		__syncthreads();
+	}
+	// f: component planes of a slot; A: [2][SHT + 6][PA]. All threads of the block; the caller's barrier follows.
+	__device__ __forceinline__ void load(const cx<R>* f, const cx<R>* Ca, size_t N, cx<R>* A) const {
+		if(Ca) points<true>(f, Ca, N, A);
+		else points<false>(f, Ca, N, A);
+	}
+	template <bool PHASE>
+	__device__ __forceinline__ void points(const cx<R>* f, const cx<R>* Ca, size_t N, cx<R>* A) const {
+		const int cnt = wx * wy;
+#pragma unroll 1
+		for(int e0 = threadIdx.x; e0 < cnt; e0 += U * 256) {
+			cx<R> a[U], b[U];
+			int to[U];
+#pragma unroll
+			for(int j = 0; j < U; j++) {
+				// past the end: the last point once more, the same value
+				const int e = min(e0 + 256 * j, cnt - 1), v = e * magic >> 16, u = e - v * wx, q = at[u] + at[SHT + 6 + v];
+				to[j] = v * PA + u;
+				a[j] = f[q];
+				b[j] = f[N + q];
+				if(PHASE) phase_apply(Ca, N, q, a[j], b[j]);
+			}
+#pragma unroll
+			for(int j = 0; j < U; j++) {
+				A[to[j]] = a[j];
+				A[(SHT + 6) * PA + to[j]] = b[j];
+			}
+		}
+	}
+};
+
 template <typename R>
 __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const ShiftParams* __restrict__ sp,
 		const cx<R>* __restrict__ CA, const cx<R>* __restrict__ CB, int nsh, const cx<R>* __restrict__ F,
@@ -2596,8 +2648,6 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 	const cx<R>* Ca = CA ? CA + (size_t)g * coef_set_size(N) : nullptr;
 	const cx<R>* Cb = CB ? CB + (size_t)g * coef_set_size(N) : nullptr;
 	const int Px = Nx - 1, Py = Ny - 1;
-	const int bx = ax ? nsh * (P.msx - 1) : 0, by = ay ? nsh * (P.msy - 1) : 0;
-	const int wx = ax ? SHT + 3 * nsh : SHT, wy = ay ? SHT + 3 * nsh : SHT;
 	cx<R> ph = W.ph;
 	if(nsh == 2) ph = ph * ph;
 	// every tap index of both passes stays above -(N-1): mod arithmetic equals the wrap rule
@@ -2617,40 +2667,25 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 		}
 		return;
 	}
-	// 1. input window, phase_A applied: warp w takes the window rows w, w + 8, ..., lane l the
-	// columns l and l + 32; the wrapped source row and columns are computed once per row / thread
+	// 1. input window, phase_A applied
 	constexpr int PA = SHT + 7, PB = SHT + 1;  // odd pitches (8-byte words): no bank conflicts
 	cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);  // [2][wy][PA]: the window
 	cx<R>* B = A + 2 * (SHT + 6) * PA;             // [2][wy][PB]: the window after the x-passes
-	const int lane = tid % 32, warp = tid / 32, nwarp = blockDim.x / 32;
-	int xc[2];
-#pragma unroll
-	for(int h = 0; h < 2; h++) {
-		const int u = lane + 32 * h;
-		xc[h] = u >= wx ? -1 : ax ? pmod(x0 + bx + u, Px) : (x0 + u < Nx ? x0 + u : -1);
-	}
-	for(int v = warp; v < wy; v += nwarp) {
-		const int yi = ay ? pmod(y0 + by + v, Py) : (y0 + v < Ny ? y0 + v : -1);
-#pragma unroll
-		for(int h = 0; h < 2; h++) {
-			const int u = lane + 32 * h;
-			if(u < wx) {
-				cx<R> a = mk<R>(0, 0), b = mk<R>(0, 0);
-				if(xc[h] >= 0 && yi >= 0) tap_in(f, Ca, N, xc[h] + Nx * yi, a, b);
-				A[v * PA + u] = a;
-				A[(SHT + 6) * PA + v * PA + u] = b;
-			}
-		}
-	}
+	__shared__ int places[2 * (SHT + 6)];
+	const ShiftWindow<R> win(G, P, nsh, x0, y0, places);
+	const int wy = win.wy, nseg = (min(SHT, Nx - x0) + 7) / 8;
+	win.load(f, Ca, N, A);
 	__syncthreads();
 	// 2. the n x-passes of one component over 8 consecutive outputs of a window row per thread, in
 	// registers (consecutive threads take consecutive rows)
 	const cx<R>* Y = A;  // what the y-passes read, with its pitch
 	int PY = PA;
 	if(ax) {
-		const int nin = 8 + 3 * nsh;
-		for(int t = tid; t < 2 * 4 * wy; t += blockDim.x) {
-			const int v = t % wy, r = t / wy, seg = r % 4, c = r / 4;
+		for(int t = tid; t < 2 * nseg * wy; t += blockDim.x) {
+			const int v = t % wy, r = t / wy, c = r >= nseg, seg = r - c * nseg;
+			// past the window shared memory is not initialised: FP64's one filter for both shifts (ShiftW) takes
+			// seven values with zero weights among them, the 4-tap passes none that is not in the window
+			const int nin = sizeof(R) == 8 ? min(8 + 3 * nsh, win.wx - seg * 8) : 8 + 3 * nsh;
 			const cx<R>* in = A + c * (SHT + 6) * PA + v * PA + seg * 8;
 			cx<R> w[14];
 #pragma unroll
@@ -2669,12 +2704,13 @@ __global__ void __launch_bounds__(256) k_shift_fused(Geom G, int slot0, const Sh
 	for(int t = tid; t < SHT * (SHT / 4); t += blockDim.x) {
 		const int u = t % SHT, seg = t / SHT;
 		const int ix = x0 + u;
+		if(ix >= Nx || y0 + seg * 4 >= Ny) continue;
 		cx<R> o[2][4];
 #pragma unroll
 		for(int c = 0; c < 2; c++) {
 			const cx<R>* in = Y + c * (SHT + 6) * PY + seg * 4 * PY + u;
 			if(ay) {
-				const int nin = 4 + 3 * nsh;
+				const int nin = sizeof(R) == 8 ? min(4 + 3 * nsh, wy - seg * 4) : 4 + 3 * nsh;
 				cx<R> w[10];
 #pragma unroll
 				for(int k = 0; k < 10; k++) w[k] = k < nin ? in[k * PY] : mk<R>(0, 0);
@@ -2756,8 +2792,6 @@ static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0,
 	const cx<R>* Ca = CA ? CA + (size_t)g * coef_set_size(N) : nullptr;
 	const cx<R>* Cb = CB + (size_t)g * coef_set_size(N);
 	const int Px = Nx - 1, Py = Ny - 1;
-	const int bx = ax ? nsh * (P.msx - 1) : 0, by = ay ? nsh * (P.msy - 1) : 0;
-	const int wx = ax ? SHT + 3 * nsh : SHT, wy = ay ? SHT + 3 * nsh : SHT;
 	cx<R> ph = W.ph;
 	if(nsh == 2) ph = ph * ph;
 	const bool regular = (!ax || P.msx - 1 > -Px) && (!ay || P.msy - 1 > -Py);  // see k_shift_fused
@@ -2779,44 +2813,27 @@ static __global__ void __launch_bounds__(256, 4) k_shift_pair(Geom G, int pair0,
 	constexpr int PA = SHT + 7, PB = SHT + 1;
 	cx<R>* A = reinterpret_cast<cx<R>*>(smem_raw);  // [2][wy][PA]: the window
 	cx<R>* B = A + 2 * (SHT + 6) * PA;             // [2][wy][PB]: the window after the x-passes
-	const int lane = tid % 32, warp = tid / 32, nwarp = blockDim.x / 32;
-	int xc[2];
-#pragma unroll
-	for(int h = 0; h < 2; h++) {
-		const int u = lane + 32 * h;
-		xc[h] = u >= wx ? -1 : ax ? pmod(x0 + bx + u, Px) : (x0 + u < Nx ? x0 + u : -1);
-	}
+	__shared__ int places[2 * (SHT + 6)];
+	const ShiftWindow<R> win(G, P, nsh, x0, y0, places);
+	const int wy = win.wy, nseg = (min(SHT, Nx - x0) + 7) / 8;
 	// the thread's outputs: 4 rows of one column (SHT * SHT / 4 threads)
 	const int ix = x0 + tid % SHT, iy0 = y0 + tid / SHT * 4;
 	cx<R> keep[2][4];
 	for(int pol = 0; pol < 2; pol++) {
-		const cx<R>* fp = f + pol * 2 * N;
 		if(pol) __syncthreads();  // the first slot's window has been read
-		for(int v = warp; v < wy; v += nwarp) {
-			const int yi = ay ? pmod(y0 + by + v, Py) : (y0 + v < Ny ? y0 + v : -1);
-#pragma unroll
-			for(int h = 0; h < 2; h++) {
-				const int u = lane + 32 * h;
-				if(u < wx) {
-					cx<R> a = mk<R>(0, 0), b = mk<R>(0, 0);
-					if(xc[h] >= 0 && yi >= 0) tap_in(fp, Ca, N, xc[h] + Nx * yi, a, b);
-					A[v * PA + u] = a;
-					A[(SHT + 6) * PA + v * PA + u] = b;
-				}
-			}
-		}
+		win.load(f + pol * 2 * N, Ca, N, A);
 		__syncthreads();
 		const cx<R>* Y = A;
 		int PY = PA;
 		if(ax) {
-			const int nin = 8 + 3 * nsh;
-			for(int t = tid; t < 2 * 4 * wy; t += blockDim.x) {
-				const int v = t % wy, r = t / wy, seg = r % 4, c = r / 4;
+			for(int t = tid; t < 2 * nseg * wy; t += blockDim.x) {
+				const int v = t % wy, r = t / wy, c = r >= nseg, seg = r - c * nseg;
+				const int nin = 8 + 3 * nsh;
 				const cx<R>* in = A + c * (SHT + 6) * PA + v * PA + seg * 8;
 				cx<R> w[14];
 #pragma unroll
 				for(int k = 0; k < 14; k++) w[k] = k < nin ? in[k] : mk<R>(0, 0);
-			W.template filter<14>(W.wx, w);
+				W.template filter<14>(W.wx, w);
 				cx<R>* out = B + c * (SHT + 6) * PB + v * PB + seg * 8;
 #pragma unroll
 				for(int k = 0; k < 8; k++) out[k] = w[k];
