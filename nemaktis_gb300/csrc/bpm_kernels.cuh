@@ -29,16 +29,20 @@ enum { Q_XXTR = 0, Q_YYTR, Q_XYTR, Q_XXS, Q_YYS, Q_XYS, Q_VX, Q_VY, Q_IZZ, NQ };
 enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
 // Factor planes of the partitioned x-line solves (k_factor_part): every chunk of M points of a line
 // is factored by itself. F_A = -l_i (forward recurrence d_i = r_i - l_i d_{i-1}, l_i = a_i/beta_{i-1},
-// 0 at the chunk's first point), F_RB = 1/beta_i, F_C = -c_i/beta_i, F_Z = (product of F_C over the
-// points before i) * F_RB, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
-// unknown before the chunk adds to point i before the backward sweep.
-enum { F_Z = F_W, F_E = F_COR };
+// 0 at the chunk's first point), F_DB = 1/beta_i - base, F_C = -c_i/beta_i, F_Z = (product of F_C over the
+// points before i) / beta_i, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
+// unknown before the chunk adds to point i before the backward sweep. base is 1 in FP32 on lines of weak coupling,
+// where the difference is rounded to its own, smaller size: in a uniform region every point of every slab repeats
+// the rounding of 1/beta_i, which took 7.7e-8 of the amplitude per slab (64 slabs 256x256: 4.9e-6, 0.8e-6 so; the
+// solves 324 -> 332 us). Else 0.
+// It is in the line scalar lsc[line][0].y.
+enum { F_DB = F_RB, F_Z = F_W, F_E = F_COR };
 // Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
 // first one): h = I_HD d_last + I_HY yf' and g = I_GD d_last + I_GY yf' from the two chunks alone,
 // I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds.
 enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, NIF };
 // Layout of a line's factors: for each point k of a chunk the vectors {F_A, F_Z} of the CH chunks, then
-// {F_RB, F_C}, then F_E; after the M points the NIF interface coefficients of the chunks.
+// {F_DB, F_C}, then F_E; after the M points the NIF interface coefficients of the chunks.
 __host__ __device__ __forceinline__ size_t part_line_size(int M, int CH) { return (size_t)CH * (M * NFAC + NIF); }
 template <typename S>
 struct alignas(4 * sizeof(S)) v4 {
@@ -1158,6 +1162,12 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	// factors of the points [i0, i0 + m) as one chunk; returns through vf, vl, wf, wl, rbl the
 	// border responses to the unknowns before (v) and after (w) the chunk and the last 1/beta
 	cx<S> vf = zero, vl = zero, wf = zero, wl = zero, rbl = zero;
+	S base = 0;
+	if(sizeof(S) == sizeof(float) && active) {
+		cx<S> em, ec, en;
+		coef_diag<0>(Cg, c, p0, em, ec, en);
+		base = l1abs(ec) < (S)1 ? 1 : 0;  // |1/beta| > 0.6 then
+	}
 	// 1 / b with one division: the pivots are 1 + O(dz / (k0 n dx^2)), far from the ends of the range
 	auto recip = [](cx<S> b) {
 		const S r = (S)1 / (b.x * b.x + b.y * b.y);
@@ -1170,20 +1180,20 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 			const int i = i0 + k;
 			cx<S> em, ec, en;
 			coef_diag<0>(Cg, c, p0 + i, em, ec, en);
-			const cx<S> a = -em, b = one - ec, cs = -en;
+			const cx<S> a = -em, cs = -en;
 			cx<S> al = zero;  // -l
 			if(k == 0) ev = -a;
 			else {
 				al = -(a * rb);
 				ev = al * ev;
 			}
-			const cx<S> beta = k == 0 ? b : cfma(al, cprev, b);
-			rb = recip(beta);
+			const cx<S> b1 = k == 0 ? -ec : cfma(al, cprev, -ec);  // beta - 1
+			rb = recip(one + b1);
 			cprev = cs;
-			const cx<S> cc = -(rb * cs), z = cpz * rb, e = rb * ev;
+			const cx<S> db = base != 0 ? -(rb * b1) : rb, cc = -(rb * cs), z = cpz * rb, e = rb * ev;
 			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH;
 			reinterpret_cast<v4<S>*>(F)[i / M] = v4<S>{al.x, al.y, z.x, z.y};
-			reinterpret_cast<v4<S>*>(F + 2 * CH)[i / M] = v4<S>{rb.x, rb.y, cc.x, cc.y};
+			reinterpret_cast<v4<S>*>(F + 2 * CH)[i / M] = v4<S>{db.x, db.y, cc.x, cc.y};
 			F[4 * CH + i / M] = e;
 			vf = cfma(z, ev, vf);
 			cpz = cpz * cc;
@@ -1202,7 +1212,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		for(int k = max(0, min(M, n - i0)); k < M; k++) {
 			cx<S>* F = Fc + (size_t)k * NFAC * CH;
 			reinterpret_cast<v4<S>*>(F)[t] = v4<S>{1, 0, 0, 0};
-			reinterpret_cast<v4<S>*>(F + 2 * CH)[t] = v4<S>{0, 0, 1, 0};
+			reinterpret_cast<v4<S>*>(F + 2 * CH)[t] = v4<S>{-base, 0, 1, 0};
 			F[4 * CH + t] = zero;
 		}
 	}
@@ -1247,7 +1257,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		const S k = ceil(lt / log(rho)) - 1;
 		K = k <= (S)PART_KMAX ? (int)k : -1;
 	}
-	ls[0] = mk((double)K, 0.0);
+	ls[0] = mk((double)K, (double)base);
 	if(K >= 0) return;
 	// the whole line as one chunk that is its own neighbour: h = vl h + wl g + 1/beta_last d_last,
 	// g = vf h + wf g + yf. (The block's other threads have written their chunks' factors: those of
@@ -1261,11 +1271,17 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	If[I_GY * CH] = m * p;
 }
 
+// v / beta from F_DB
+template <typename R>
+__device__ __forceinline__ cx<R> from_base(cx<R> db, R base, cx<R> v) {
+	return sizeof(R) == sizeof(float) ? cfma(db, v, mk<R>(base * v.x, base * v.y)) : db * v;
+}
+
 // The sequential solve of a line flagged -1 by k_factor_part, by one thread: buf holds the right-hand
 // sides of KS slots (element i of slot j at ((i / M) * part_pitch(M) + i % M) * ES + j * PITCH) and receives the
 // solution.
 template <typename R, int M, int KS, int ES = 1>
-__device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n) {
+__device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n, R base) {
 	const cx<R>* If = Fc + (size_t)M * NFAC * CH;
 #pragma unroll 1
 	for(int j = 0; j < KS; j++) {
@@ -1283,7 +1299,7 @@ __device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* 
 		for(int i = n - 1; i >= 0; i--) {
 			const v4<R> rc = part_rc(Fc, i % M, CH, i / M);
 			cx<R>& v = b[((i / M) * part_pitch(M) + i % M) * ES];
-			x = cfma(mk(rc.z, rc.w), x, cfma(part_e(Fc, i % M, CH, i / M), h, mk(rc.x, rc.y) * v));
+			x = cfma(mk(rc.z, rc.w), x, cfma(part_e(Fc, i % M, CH, i / M), h, from_base<R>(mk(rc.x, rc.y), base, v)));
 			v = x;
 		}
 	}
@@ -1400,7 +1416,9 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 	cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw) + (size_t)warp * KS * PITCH;
 	if(iy < Ny) {  // always true unless TOUT (whose block writes together after a barrier)
 	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
-	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
+	const cx<double> kb = lsc[(((size_t)g * 2 + c) * Ny + iy) * 2];
+	const int K = (int)kb.x;
+	const R base = (R)kb.y;
 	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
 	const cx<R>* f0 = src + (size_t)s0 * 2 * N;
@@ -1480,16 +1498,16 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 		for(int k = M - 1; k >= 0; k--) {
 			{
 				const v4<R> rc = part_rc(Fc, k, 32, lane);
-				const cx<R> rb = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, 32, lane);
+				const cx<R> db = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, 32, lane);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
-					x[j] = cfma(cc, x[j], cfma(ee, h[j], rb * vb[j * PITCH + k]));
+					x[j] = cfma(cc, x[j], cfma(ee, h[j], from_base<R>(db, base, vb[j * PITCH + k])));
 					vb[j * PITCH + k] = x[j];
 				}
 			}
 		}
 	}
-	else if(lane == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, 32, n_unk);
+	else if(lane == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, 32, n_unk, base);
 	// the explicit-step solves never accumulate; the accumulating ones load the accumulator inputs
 	// of several points before storing any (their latency would otherwise be paid point by point)
 	const bool acc = KIND != ST_EXPL_Y && acc_out;
@@ -1972,7 +1990,9 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 	cx<R>* sG = buf + KS * PITCH;                     // [2][KS][W]: g (first yf) of the warps' first chunks
 	cx<R>* sH = sG + 2 * KS * W;                      // [2][KS][W + 1]: h of the warps' last chunks, then of the line's
 	const cx<R>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, CH);
-	const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
+	const cx<double> kb = lsc[(((size_t)g * 2 + c) * Ny + iy) * 2];
+	const int K = (int)kb.x;
+	const R base = (R)kb.y;
 	const int last = (n_unk - 1) / M;  // last chunk
 	const cx<R> zero = mk<R>(0, 0);
 	const Stencil<R> st{coef + (size_t)g * coef_set_size(N), N, Nx, Ny};
@@ -2074,16 +2094,16 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		for(int k = M - 1; k >= 0; k--) {
 			{
 				const v4<R> rc = part_rc(Fc, k, CH, ci);
-				const cx<R> rb = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, CH, ci);
+				const cx<R> db = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, CH, ci);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
-					x[j] = cfma(cc, x[j], cfma(ee, hl[j], rb * vb[j * PITCH + k]));
+					x[j] = cfma(cc, x[j], cfma(ee, hl[j], from_base<R>(db, base, vb[j * PITCH + k])));
 					vb[j * PITCH + k] = x[j];
 				}
 			}
 		}
 	}
-	else if(threadIdx.x == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, CH, n_unk);
+	else if(threadIdx.x == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, CH, n_unk, base);
 	__syncthreads();
 	// write-out: the accumulator inputs of several points are loaded before any store
 	constexpr int U = 4;

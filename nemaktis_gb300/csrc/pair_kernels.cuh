@@ -160,12 +160,12 @@ __device__ __forceinline__ void pair_forward(pr* vb, const cx<float>* Fc, int CH
 	}
 }
 template <int M>
-__device__ __forceinline__ void pair_backward(pr* vb, const cx<float>* Fc, int CH, int ci, pr h, pr x) {
+__device__ __forceinline__ void pair_backward(pr* vb, const cx<float>* Fc, int CH, int ci, float base, pr h, pr x) {
 #pragma unroll
 	for(int k = M - 1; k >= 0; k--) {
 		const v4<float> rc = part_rc(Fc, k, CH, ci);
 		const cx<float> e = part_e(Fc, k, CH, ci);
-		x = pfma(mk(rc.z, rc.w), x, pfma(e, h, pmul(mk(rc.x, rc.y), vb[k])));
+		x = pfma(mk(rc.z, rc.w), x, pfma(e, h, pfma(mk(rc.x, rc.y), vb[k], pr{base * vb[k].x, base * vb[k].y, base * vb[k].z, base * vb[k].w})));
 		vb[k] = x;
 	}
 }
@@ -178,8 +178,8 @@ __device__ __forceinline__ void pair_backward(pr* vb, const cx<float>* Fc, int C
 // the block's 4 lines (StripRhs), for short lines (M < 6) a point of one line, where a column per thread leaves warps
 // without work (64x64: explicit step 16.6 us, with 2 lines per thread 18.3 us, with 4 lines 22.6 us; 224x224: 55.0
 // us with 1 or 2 lines, 50.7 us with 4). 256x256, 16 wavelengths, 13 q: Woodbury solves 477 us as k_solve_xc with
-// two slots per thread, 402 us here with a line per warp for the right-hand sides too, 324 us with strips;
-// explicit step 491, 378 and 324 us. The rows of a block staged in shared memory (cp.async) gave 438 and
+// two slots per thread, 402 us here with a line per warp for the right-hand sides too, 332 us with strips;
+// explicit step 491, 378 and 330 us. The rows of a block staged in shared memory (cp.async) gave 438 and
 // 415 us, x neighbours from lane shuffles 478 and 498 us.
 template <int M, int KIND, int OUT>
 __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __restrict__ coef,
@@ -216,7 +216,9 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 	}
 	if(iy < Ny) {
 		const cx<float>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, 32);
-		const int K = (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x;
+		const cx<double> kb = lsc[(((size_t)g * 2 + c) * Ny + iy) * 2];
+		const int K = (int)kb.x;
+		const float base = (float)kb.y;
 		pr* buf = bufs + warp * WS;
 		if(K >= 0) {
 			pr* vb = buf + lane * PM;
@@ -238,9 +240,9 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 				}
 			}
 			h = pshfl(h, left);
-			pair_backward<M>(vb, Fc, 32, lane, h, x);
+			pair_backward<M>(vb, Fc, 32, lane, base, h, x);
 		}
-		else if(lane == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, 32, n);
+		else if(lane == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, 32, n, base);
 		__syncwarp();
 		// out, or for the transposed outputs the sums into the buffer, where the added field comes with
 		// aligned loads (point n repeats point 0; its entry is free or padding)
@@ -319,7 +321,9 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	const size_t pair = (size_t)g * nch + ch;
 	const pr* f = src + pair * 2 * N;
 	const cx<float>* Fc = fac + ((size_t)g * 2 + c) * NFAC * plane + (size_t)iy * part_line_size(M, CH);
-	const int K = live ? (int)lsc[(((size_t)g * 2 + c) * Ny + iy) * 2].x : 0;
+	const cx<double> kb = live ? lsc[(((size_t)g * 2 + c) * Ny + iy) * 2] : mk(0., 0.);
+	const int K = (int)kb.x;
+	const float base = (float)kb.y;
 	pr* buf = bufs + ln * WS;
 	{
 		const StripRhs<KIND, LT> rhs(coef + (size_t)g * coef_set_size(N), f, G, c, lb * LT);
@@ -378,8 +382,8 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 			x = pfma(qg, gr, pfma(pg, hl, bg));
 		}
 	}
-	if(part) pair_backward<M>(vb, Fc, CH, ci, hl, x);
-	else if(live && ci == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, CH, n);
+	if(part) pair_backward<M>(vb, Fc, CH, ci, base, hl, x);
+	else if(live && ci == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, CH, n, base);
 	__syncthreads();
 	if(OUT == PO_SAME) {
 		if(!live) return;
