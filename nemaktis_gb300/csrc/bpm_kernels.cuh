@@ -2414,22 +2414,6 @@ __global__ void __launch_bounds__(256) k_solve_ys(Geom G, int slot0, int nch, co
 	}
 }
 
-// Point-wise symmetric 2x2 phase operator (PhaseEvolutionOperator.cpp:14-32).
-template <typename R>
-__global__ void k_phase(Geom G, int slot0, const cx<R>* __restrict__ coef, cx<R>* F) {
-	int p = blockIdx.x * blockDim.x + threadIdx.x;
-	if(p >= G.N) return;
-	int s = blockIdx.y;
-	int N = G.N;
-	int g = (slot0 + s) / G.spg - slot0 / G.spg;
-	const cx<R>* C = coef + (size_t)g * coef_set_size(N);
-	cx<R> oxx = coef_ph(C, 0, p), oyy = coef_ph(C, 1, p), oxy = coef_ph(C, 2, p);
-	cx<R>* f = F + (size_t)s * 2 * N + p;
-	cx<R> a = f[0], b = f[N];
-	f[0] = oxx * a + oxy * b;
-	f[N] = oxy * a + oyy * b;
-}
-
 // Transverse translation for tilted incidence (SimpleShiftOperator.cpp:52-93): 4-tap cubic
 // interpolation with period Nx-1 / Ny-1 (wrap rule SimpleShiftOperator.h:24-39).
 __device__ __forceinline__ int ref_wrap(int i, int n) {
