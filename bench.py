@@ -268,14 +268,14 @@ def run_ours(args):
     # DRAM bytes per launch of the dominant kernel from one ncu capture (dram__bytes_read.sum +
     # dram__bytes_write.sum), scaled to this workload's launch by the slots it processes; the
     # capture and its command are summarised under profiles/.
-    PROF = "profiles/solve_xc_koehler_256x256x8_fp32.md"
-    PSF = "profiles/shift_fused_koehler_256x256x8_fp32.md"
-    W = 2 * (319.7e6 + 190.0e6 + 560.9e6 + 196.6e6) / 2  # mean of the two Woodbury launches, x2 slots
-    TRAFFIC = {("koehler", "fp32", "wood_solve_x"): (W, PROF),
-               ("koehler", "fp32", "wood_solve_y"): (W, PROF + " (the same kernel in the transposed frame)"),
-               ("koehler", "fp32", "expl_solve_x"): (2 * (345.0e6 + 188.0e6), PROF),
-               ("koehler", "fp32", "expl_solve_y"): (2 * (345.0e6 + 188.0e6), PROF + " (the same kernel in the transposed frame)"),
-               ("koehler", "fp32", "shift_fused"): (2 * (242.6e6 + 181.1e6), PSF)}
+    PROF = "profiles/solve_xp_koehler_256x256x8_fp32.md"
+    WX = 2 * (309.2e6 + 184.7e6 + 527.5e6 + 189.0e6) / 2  # mean of the two Woodbury launches, x2 slots
+    WY = 2 * (309.1e6 + 184.3e6 + 527.6e6 + 188.7e6) / 2
+    TRAFFIC = {("koehler", "fp32", "wood_solve_x"): (WX, PROF),
+               ("koehler", "fp32", "wood_solve_y"): (WY, PROF),
+               ("koehler", "fp32", "expl_solve_x"): (2 * (322.1e6 + 185.5e6), PROF),
+               ("koehler", "fp32", "expl_solve_y"): (2 * (321.9e6 + 183.4e6), PROF),
+               ("koehler", "fp32", "shift_fused"): (2 * (242.5e6 + 176.1e6), PROF)}
     roof = None
     if prof:
         top = max(prof, key=lambda k: prof[k]["ms"])
