@@ -18,6 +18,8 @@
 #include <cstdint>
 
 #include "cplx.cuh"
+#include "line_join.cuh"
+#include "solve_config.h"
 
 namespace nbpm {
 
@@ -39,8 +41,12 @@ enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
 enum { F_DB = F_RB, F_Z = F_W, F_E = F_COR };
 // Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
 // first one): h = I_HD d_last + I_HY yf' and g = I_GD d_last + I_GY yf' from the two chunks alone,
-// I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds.
-enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, NIF };
+// I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds. Lines joined
+// by ring_solve (line_join.cuh) hold the node's coefficients in place of those four and after them, and the right-hand
+// sides' coefficients include f2 and d; the line's closing coefficients are the first four entries of I_X.
+enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, I_ETA, I_KAP, I_TAU, I_X, NIF };
+enum { I_F = I_PH };  // RN_F .. RN_RHO there, RN_ETA .. RN_TAU from I_ETA on
+static_assert(NIF == PART_NIF, "part_plane");
 // Layout of a line's factors: for each point k of a chunk the vectors {F_A, F_Z} of the CH chunks, then
 // {F_DB, F_C}, then F_E; after the M points the NIF interface coefficients of the chunks.
 __host__ __device__ __forceinline__ size_t part_line_size(int M, int CH) { return (size_t)CH * (M * NFAC + NIF); }
@@ -796,23 +802,6 @@ __global__ void k_solve(Geom G, int slot0, int nslots, const cx<R>* __restrict__
 	if(acc_out) acc_out[off + qe] = acc_in[off + qe] + x;
 }
 
-template <typename R>
-__device__ __forceinline__ cx<R> shfl_up_c(cx<R> v, int d) {
-	return mk<R>(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d));
-}
-template <typename R>
-__device__ __forceinline__ cx<R> shfl_down_c(cx<R> v, int d) {
-	return mk<R>(__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d));
-}
-template <typename R>
-__device__ __forceinline__ cx<R> shfl_idx_c(cx<R> v, int l) {
-	return mk<R>(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
-}
-template <typename R>
-__device__ __forceinline__ cx<R> shfl_xor_c(cx<R> v, int m) {
-	return mk<R>(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
-}
-
 // x-line solve fused with the right-hand side that precedes it (KIND: explicit y half-step or
 // x Woodbury term), chunked parallel form: one warp per (line, comp, KS slots of one
 // wavelength); lane l owns the unknowns [l*M, l*M+M) of the line. The forward and backward
@@ -853,34 +842,12 @@ __device__ __forceinline__ cx<R> shfl_xor_c(cx<R> v, int m) {
 // rows, combined through shared memory. Intermediate values go to the output planes and are
 // read back by the same thread.
 template <typename T>
-struct Mob {
-	cx<T> a, b, c, d;  // [[a, b], [c, d]]
-};
-template <typename T>
-__device__ __forceinline__ Mob<T> mob_mul(const Mob<T>& X, const Mob<T>& Y) {  // X . Y
-	return Mob<T>{X.a * Y.a + X.b * Y.c, X.a * Y.b + X.b * Y.d, X.c * Y.a + X.d * Y.c, X.c * Y.b + X.d * Y.d};
-}
-template <typename T>
-__device__ __forceinline__ T l1abs(cx<T> z) { return fabs(z.x) + fabs(z.y); }
-template <typename T>
-__device__ __forceinline__ void mob_norm(Mob<T>& X) {
-	T m = fmax(fmax(l1abs(X.a), l1abs(X.b)), fmax(l1abs(X.c), l1abs(X.d)));
-	if(m > (T)0) {
-		T r = (T)1 / m;
-		X.a = X.a * r; X.b = X.b * r; X.c = X.c * r; X.d = X.d * r;
-	}
-}
-template <typename T>
 struct Aff {
 	cx<T> A, B;  // x -> A x + B
 };
 template <typename T>
 __device__ __forceinline__ Aff<T> aff_after(const Aff<T>& second, const Aff<T>& first) {
 	return Aff<T>{second.A * first.A, second.A * first.B + second.B};
-}
-template <typename T>
-__device__ __forceinline__ Mob<T> shfl_up_m(const Mob<T>& X, int o) {
-	return Mob<T>{shfl_up_c(X.a, o), shfl_up_c(X.b, o), shfl_up_c(X.c, o), shfl_up_c(X.d, o)};
 }
 template <typename T>
 __device__ __forceinline__ Aff<T> shfl_up_a(const Aff<T>& X, int o) { return Aff<T>{shfl_up_c(X.A, o), shfl_up_c(X.B, o)}; }
@@ -1137,15 +1104,22 @@ __global__ void __launch_bounds__(DIRN == 1 ? 512 : 256) k_factor_chunked(Geom G
 // scalar lsc[line][0].x receives the number of Jacobi steps K that the interface system needs to
 // reach rounding: a step multiplies the error by rho, the largest row sum of the interface couplings,
 // about the M-th power of the decay from point to point (K = 0 for 8-point chunks at the usual mesh
-// spacings in FP32, 1 in FP64). Lines with rho^KMAX above rounding (spacings far below a
-// wavelength) and lines of one chunk are factored as a single chunk by one thread and flagged -1;
-// their solve is sequential.
+// spacings in FP32, 1 in FP64). Where that would be more than PART_KMAX steps (spacings far below a
+// wavelength, a last chunk of few points) and on lines of one chunk K is -1 and the line is joined exactly by
+// ring_solve, which costs about as much as PART_KMAX steps at any coupling.
 // Bound: HBM and the latency of the reciprocals (M in a row). The scans over Moebius and affine maps
 // of k_factor_chunked it replaces here took 107 us per launch on the 256x256, 16-wavelength FP32 case
 // and 47 us on a 64x64 FP64 one.
-constexpr int PART_KMAX = 24;
+constexpr int PART_KMAX = 10;
+// a function of its own, so that it takes no registers from the other lines
+template <bool MULTI, typename S>
+__device__ __noinline__ RingNode<S> part_ring_factor(LineThreads T, cx<S> ph, cx<S> pg, cx<S> qh, cx<S> qg, cx<S>* sh) {
+	return ring_factor<MULTI>(T, ph, pg, qh, qg, sh);
+}
+// Registers: 64 in FP64 and 48 in FP32, what the chunks' sweeps take (102 and 63 with those of ring_factor made a
+// 128x128 FP64 step 4 % slower).
 template <typename S>
-__global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>* __restrict__ coef,
+__global__ void __launch_bounds__(256, sizeof(S) == sizeof(double) ? 4 : 5) k_factor_part(Geom G, int M, const cx<S>* __restrict__ coef,
 		cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
 	const int N = G.N, nlines = G.Ny, n = G.Nx - 1;
 	const int CH = blockDim.x, t = threadIdx.x;
@@ -1159,8 +1133,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	cx<S>* If = Fc + (size_t)M * NFAC * CH;
 	cx<double>* ls = lsc + ((size_t)gc * nlines + line) * 2;
 	const cx<S> one = mk<S>(1, 0), zero = mk<S>(0, 0);
-	// factors of the points [i0, i0 + m) as one chunk; returns through vf, vl, wf, wl, rbl the
-	// border responses to the unknowns before (v) and after (w) the chunk and the last 1/beta
+	// border responses to the unknowns before (v) and after (w) the chunk, and the last 1/beta
 	cx<S> vf = zero, vl = zero, wf = zero, wl = zero, rbl = zero;
 	S base = 0;
 	if(sizeof(S) == sizeof(float) && active) {
@@ -1173,9 +1146,11 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		const S r = (S)1 / (b.x * b.x + b.y * b.y);
 		return mk(b.x * r, -b.y * r);
 	};
-	auto chunk = [&](int i0, int m) {
+	const int i0 = t * M;
+	const bool own = active && i0 < n;
+	if(own) {
+		const int m = min(M, n - i0);
 		cx<S> rb = zero, cprev = zero, ev = zero, cpz = one;
-		vf = zero;
 		for(int k = 0; k < m; k++) {
 			const int i = i0 + k;
 			cx<S> em, ec, en;
@@ -1191,10 +1166,10 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 			rb = recip(one + b1);
 			cprev = cs;
 			const cx<S> db = base != 0 ? -(rb * b1) : rb, cc = -(rb * cs), z = cpz * rb, e = rb * ev;
-			cx<S>* F = Fc + (size_t)(i % M) * NFAC * CH;
-			reinterpret_cast<v4<S>*>(F)[i / M] = v4<S>{al.x, al.y, z.x, z.y};
-			reinterpret_cast<v4<S>*>(F + 2 * CH)[i / M] = v4<S>{db.x, db.y, cc.x, cc.y};
-			F[4 * CH + i / M] = e;
+			cx<S>* F = Fc + (size_t)k * NFAC * CH;
+			reinterpret_cast<v4<S>*>(F)[t] = v4<S>{al.x, al.y, z.x, z.y};
+			reinterpret_cast<v4<S>*>(F + 2 * CH)[t] = v4<S>{db.x, db.y, cc.x, cc.y};
+			F[4 * CH + t] = e;
 			vf = cfma(z, ev, vf);
 			cpz = cpz * cc;
 			vl = e;
@@ -1202,10 +1177,7 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		}
 		wf = cpz;
 		rbl = rb;
-	};
-	const int i0 = t * M;
-	const bool own = active && i0 < n;
-	if(own) chunk(i0, min(M, n - i0));
+	}
 	if(active) {
 		// past the line's end: entries that leave the sweeps' values as they are, so that the solves need no
 		// condition at every point (a branch there makes each point wait for its own factors)
@@ -1224,20 +1196,14 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 	shw[tid] = wf;
 	__syncthreads();
 	S rho = 0;
+	cx<S> ph = zero, pg = zero, qh = zero, qg = zero, hd = zero, hy = zero, gd = zero, gy = zero;
 	if(own) {
 		const int nx = threadIdx.y * CH + (t == nchk - 1 ? 0 : t + 1);
 		const cx<S> vfn = shv[nx], wfn = shw[nx];
 		const cx<S> m = recip(cfnma(wl, vfn, one));
 		const cx<S> mw = m * wl, mv = m * vfn;
-		const cx<S> ph = m * vl, pg = mv * vl, qh = mw * wfn, qg = m * wfn;
-		If[I_HD * CH + t] = m * rbl;
-		If[I_HY * CH + t] = mw;
-		If[I_GD * CH + t] = mv * rbl;
-		If[I_GY * CH + t] = m;
-		If[I_PH * CH + t] = ph;
-		If[I_PG * CH + t] = pg;
-		If[I_QH * CH + t] = qh;
-		If[I_QG * CH + t] = qg;
+		ph = m * vl; pg = mv * vl; qh = mw * wfn; qg = m * wfn;
+		hd = m * rbl; hy = mw; gd = mv * rbl; gy = m;
 		rho = fmax(l1abs(ph) + l1abs(qh), l1abs(pg) + l1abs(qg));
 		if(!(rho < (S)1)) rho = 1;  // NaN too
 	}
@@ -1249,7 +1215,6 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		__syncthreads();
 		for(int w = 0; w < CH / 32; w++) rho = fmax(rho, shr[w]);
 	}
-	if(!active || t != 0) return;
 	const S lt = sizeof(S) == sizeof(float) ? (S)-18.7 : (S)-39.5;  // ln of 2^-27, 2^-57
 	int K = 0;
 	if(nchk < 2 || !(rho < (S)1)) K = -1;
@@ -1257,18 +1222,23 @@ __global__ void __launch_bounds__(256) k_factor_part(Geom G, int M, const cx<S>*
 		const S k = ceil(lt / log(rho)) - 1;
 		K = k <= (S)PART_KMAX ? (int)k : -1;
 	}
-	ls[0] = mk((double)K, (double)base);
-	if(K >= 0) return;
-	// the whole line as one chunk that is its own neighbour: h = vl h + wl g + 1/beta_last d_last,
-	// g = vf h + wf g + yf. (The block's other threads have written their chunks' factors: those of
-	// this line before the barriers above.)
-	chunk(0, n);
-	const cx<S> p = one - vl, q = one - wf;
-	const cx<S> m = crecip(cfnma(wl, vf, p * q));
-	If[I_HD * CH] = m * q * rbl;
-	If[I_HY * CH] = m * wl;
-	If[I_GD * CH] = m * vf * rbl;
-	If[I_GY * CH] = m * p;
+	if(active && t == 0) ls[0] = mk((double)K, (double)base);
+	auto put = [&](int f, cx<S> v) { if(own) If[f * CH + t] = v; };
+	if(K >= 0) {
+		put(I_PH, ph); put(I_PG, pg); put(I_QH, qh); put(I_QG, qg);
+	}
+	else {
+		// the same for all threads of a line: a warp, or the block
+		const LineThreads T{CH / 32, 0, t / 32, t % 32, t, nchk - 1};
+		__shared__ cx<S> shf[ring_factor_shared(8)];
+		const RingNode<S> r = CH > 32 ? part_ring_factor<true>(T, ph, pg, qh, qg, shf) : part_ring_factor<false>(T, ph, pg, qh, qg, shf);
+		hd = cfma(r.f2, gd, hd); hy = cfma(r.f2, gy, hy);
+		gd = r.d * gd; gy = r.d * gy;
+		#pragma unroll
+		for(int k = 0; k < RN_ALL; k++) put(k < 4 ? I_F + k : I_ETA + k - 4, r.v[k]);
+		if(active && t < 4) If[I_X * CH + t] = r.X[t];
+	}
+	put(I_HD, hd); put(I_HY, hy); put(I_GD, gd); put(I_GY, gy);
 }
 
 // v / beta from F_DB
@@ -1277,32 +1247,29 @@ __device__ __forceinline__ cx<R> from_base(cx<R> db, R base, cx<R> v) {
 	return sizeof(R) == sizeof(float) ? cfma(db, v, mk<R>(base * v.x, base * v.y)) : db * v;
 }
 
-// The sequential solve of a line flagged -1 by k_factor_part, by one thread: buf holds the right-hand
-// sides of KS slots (element i of slot j at ((i / M) * part_pitch(M) + i % M) * ES + j * PITCH) and receives the
-// solution.
-template <typename R, int M, int KS, int ES = 1>
-__device__ __noinline__ void part_solve_seq(cx<R>* buf, int PITCH, const cx<R>* Fc, int CH, int n, R base) {
-	const cx<R>* If = Fc + (size_t)M * NFAC * CH;
-#pragma unroll 1
-	for(int j = 0; j < KS; j++) {
-		cx<R>* b = buf + j * PITCH;
-		cx<R> d = mk<R>(0, 0), yf = mk<R>(0, 0);
-		for(int i = 0; i < n; i++) {
-			const v4<R> az = part_az(Fc, i % M, CH, i / M);
-			cx<R>& v = b[((i / M) * part_pitch(M) + i % M) * ES];
-			d = cfma(mk(az.x, az.y), d, v);
-			v = d;
-			yf = cfma(mk(az.z, az.w), d, yf);
-		}
-		const cx<R> h = cfma(If[I_HY * CH], yf, If[I_HD * CH] * d);
-		cx<R> x = cfma(If[I_GY * CH], yf, If[I_GD * CH] * d);
-		for(int i = n - 1; i >= 0; i--) {
-			const v4<R> rc = part_rc(Fc, i % M, CH, i / M);
-			cx<R>& v = b[((i / M) * part_pitch(M) + i % M) * ES];
-			x = cfma(mk(rc.z, rc.w), x, cfma(part_e(Fc, i % M, CH, i / M), h, from_base<R>(mk(rc.x, rc.y), base, v)));
-			v = x;
-		}
-	}
+// The node coefficients of a thread's chunk on a line flagged -1 by k_factor_part (If: its interface coefficients, CH
+// apart), read when they are used.
+template <typename R>
+struct PartNode {
+	const cx<R>*If, *close0;
+	int CH;
+	__device__ __forceinline__ cx<R> get(int k) const { return If[(k < 4 ? I_F + k : I_ETA + k - 4) * CH]; }
+	__device__ __forceinline__ cx<R> close(int k) const { return close0[k]; }
+};
+// Border unknowns of a chunk: on entry h and g from the two chunks alone, on return what the backward sweep
+// takes, the previous chunk's last unknown and the next one's first.
+template <typename V, int KS>
+struct Border {
+	V h[KS], x[KS];
+};
+// Such a line's join. A function of its own, so that it takes no registers from the other lines.
+template <bool MULTI, int KS, typename R, typename V>
+__device__ __noinline__ Border<V, KS> part_ring(LineThreads T, const cx<R>* If, int CH, Border<V, KS> b, V* s) {
+	V hl[KS];
+	ring_solve<MULTI, KS, R>(T, PartNode<R>{If, If - T.ci + I_X * CH, CH}, b.h, b.x, hl, s);
+#pragma unroll
+	for(int j = 0; j < KS; j++) b.h[j] = hl[j];
+	return b;
 }
 
 // One combine of the chunk maps of a line whose chunks sit on the 32 lanes of a warp (chunk =
@@ -1437,7 +1404,7 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * part_pitch(M) + e % M] = r[j];
 	}
 	__syncwarp();
-	if(K >= 0) {
+	{
 		// forward sweep of the lane's chunk (written back over the right-hand sides) and its first
 		// unknown yf with nothing outside the chunk
 		cx<R> d[KS], yf[KS];
@@ -1491,8 +1458,18 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 				}
 			}
 		}
+		if(K >= 0) {
 #pragma unroll
-		for(int j = 0; j < KS; j++) h[j] = shfl_idx_c(h[j], left);
+			for(int j = 0; j < KS; j++) h[j] = shfl_idx_c(h[j], left);
+		}
+		else {
+			Border<cx<R>, KS> b;
+#pragma unroll
+			for(int j = 0; j < KS; j++) { b.h[j] = h[j]; b.x[j] = x[j]; }
+			b = part_ring<false, KS, R>(LineThreads{1, 0, 0, lane, lane, last}, If, 32, b, (cx<R>*)nullptr);
+#pragma unroll
+			for(int j = 0; j < KS; j++) { h[j] = b.h[j]; x[j] = b.x[j]; }
+		}
 		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
 #pragma unroll
 		for(int k = M - 1; k >= 0; k--) {
@@ -1507,7 +1484,6 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 			}
 		}
 	}
-	else if(lane == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, 32, n_unk, base);
 	// the explicit-step solves never accumulate; the accumulating ones load the accumulator inputs
 	// of several points before storing any (their latency would otherwise be paid point by point)
 	const bool acc = KIND != ST_EXPL_Y && acc_out;
@@ -2010,7 +1986,7 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		for(int j = 0; j < KS; j++) buf[j * PITCH + (e / M) * part_pitch(M) + e % M] = r[j];
 	}
 	__syncthreads();
-	if(K >= 0) {
+	{
 		// forward sweep of the thread's chunk and its first unknown with nothing outside the chunk
 		cx<R> d[KS], yf[KS];
 		cx<R>* vb = buf + ci * part_pitch(M);
@@ -2060,6 +2036,15 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 		cx<R> bh[KS], bg[KS];
 #pragma unroll
 		for(int j = 0; j < KS; j++) { bh[j] = h[j]; bg[j] = x[j]; }
+		if(K < 0) {
+			Border<cx<R>, KS> b;
+#pragma unroll
+			for(int j = 0; j < KS; j++) { b.h[j] = h[j]; b.x[j] = x[j]; }
+			b = part_ring<true, KS, R>(LineThreads{W, 0, warp, lane, ci, last}, If, CH, b, sG);
+#pragma unroll
+			for(int j = 0; j < KS; j++) { hl[j] = b.h[j]; x[j] = b.x[j]; }
+		}
+		else
 #pragma unroll 1
 		for(int it = 0;; it++) {
 			// two buffers in turn: the one written here was last read two barriers ago
@@ -2103,7 +2088,6 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 			}
 		}
 	}
-	else if(threadIdx.x == 0) part_solve_seq<R, M, KS>(buf, PITCH, Fc, CH, n_unk, base);
 	__syncthreads();
 	// write-out: the accumulator inputs of several points are loaded before any store
 	constexpr int U = 4;

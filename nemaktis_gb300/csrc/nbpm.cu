@@ -212,10 +212,19 @@ static void CUDART_CB bulk_host_fn(void* p) {
 	}
 }
 
-// The step count of k_factor_part's line scalars, for the tuner's timing runs.
-__global__ void k_fill_steps(int lines, int K, cx<double>* lsc) {
-	int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i < lines) lsc[2 * (size_t)i] = mk((double)K, 0.0);
+// A set whose lines have the couplings ax and ay from point to point (second differences alone), for the tuner's
+// timing runs.
+template <typename R>
+__global__ void k_fill_coupling(int N, R ax, R ay, cx<R>* coef) {
+	const int p = blockIdx.x * blockDim.x + threadIdx.x;
+	if(p >= N) return;
+	cx<R>* C = coef + (size_t)blockIdx.y * coef_set_size(N);
+	coef_put(C, V_DX, p, v4<R>{0, ax, 0, ax});
+	coef_put(C, V_DX + 3, p, v4<R>{ax, ax, -2 * ax, 0});
+	coef_u(C, U_DX, p) = mk<R>(-2 * ax, 0);
+	coef_put(C, V_DY, p, v4<R>{0, ay, 0, ay});
+	coef_put(C, V_DY + 3, p, v4<R>{ay, ay, -2 * ay, 0});
+	coef_u(C, U_DY, p) = mk<R>(-2 * ay, 0);
 }
 
 // Nearest-index divisions used by the shift operator are computed on the device from nref;
@@ -752,36 +761,40 @@ struct Plan : PlanBase {
 
 	std::string tune_key(const SampleHost& h) const {
 		char b[160];
-		std::snprintf(b, sizeof b, "%s|%dx%d|spg%d|ng%d|nw%d|sm%d", sizeof(R) == sizeof(float) ? "fp32" : "fp64", h.s.Nx,
-			h.s.Ny, h.spg, tune_groups(h), h.s.n_woodbury, nsm);
+		// couplings to half an octave
+		std::snprintf(b, sizeof b, "%s|%dx%d|spg%d|ng%d|nw%d|sm%d|a%d,%d", sizeof(R) == sizeof(float) ? "fp32" : "fp64", h.s.Nx,
+			h.s.Ny, h.spg, tune_groups(h), h.s.n_woodbury, nsm, (int)std::lround(2 * std::log2(coupling(h, 0))),
+			(int)std::lround(2 * std::log2(coupling(h, 1))));
 		return b;
 	}
 
-	// Zeroes the workspace the timing runs read (their values do not change the kernels' speed,
-	// but uninitialised memory could hold NaN or denormal patterns).
+	// Zeroes the workspace the timing runs read (uninitialised memory could hold NaN or denormal patterns) and
+	// gives its coefficient sets the sample's couplings.
 	void zero_workspace() {
 		for(auto& hp : S) {
 			auto& L = hp->lane;
 			for(DevBuf* b : {&L.T, &L.T2, &L.T3, &L.coef, &L.facx, &L.facy, &L.lscx, &L.lscy, &L.coefT, &hp->F})
 				if(b->p) CK(cudaMemsetAsync(b->p, 0, b->bytes, stream0));
+			const int N = hp->geom.N;
+			const dim3 grid((unsigned)((N + 255) / 256), (unsigned)(2 * gpp(*hp)));
+			const R ax = (R)coupling(*hp, 0), ay = (R)coupling(*hp, 1);
+			k_fill_coupling<R><<<grid, 256, 0, stream0>>>(N, ax, ay, L.coef.as<cx<R>>());
+			if(L.coefT.p) k_fill_coupling<R><<<grid, 256, 0, stream0>>>(N, ay, ax, L.coefT.as<cx<R>>());
+			CK(cudaGetLastError());
 		}
 		CK(cudaStreamSynchronize(stream0));
 	}
 
-	// Jacobi steps K (k_factor_part) that the partitioned lines of direction dirn take at the sample's longest
-	// wavelength with chunks of M points: the decay from point to point is about a / |1 + 2 i a| for the
-	// coupling a = dz / (4 n k0 d^2). The workspace of the timing runs holds no factors, and K is part of a
-	// configuration's cost (64x64 FP64: 7 steps for chunks of 2 points, 3 for 4).
-	int usual_steps(const SampleHost& h, int dirn, int M) const {
+	// Coupling from point to point of the lines of direction dirn at the sample's longest wavelength. How the chunks of
+	// a line are joined depends on it, and with that what a configuration costs.
+	double coupling(const SampleHost& h, int dirn) const {
 		double lam = 0, ne = 1;
 		for(size_t g = 0; g < h.s.wavelengths.size(); g++) { lam = std::max(lam, h.s.wavelengths[g]); ne = std::max(ne, std::abs(h.s.no[g])); }
-		const double d = dirn == 0 ? h.s.dx : h.s.dy, a = h.s.dz / (4 * ne * (2 * 3.14159265 / lam) * d * d);
-		const double rho = 2 * std::pow(a / std::sqrt(1 + 4 * a * a), M), lt = sizeof(R) == sizeof(float) ? -18.7 : -39.5;
-		if(!(rho < 1)) return PART_KMAX;
-		return std::min((int)PART_KMAX, std::max(0, (int)std::ceil(lt / std::log(rho)) - 1));
+		const double d = dirn == 0 ? h.s.dx : h.s.dy;
+		return std::max(1e-6, std::min(1e6, h.s.dz / (4 * ne * (2 * 3.14159265 / lam) * d * d)));
 	}
 
-	// Device time of one slab's solves of one direction with the current configuration of
+	// Device time of one slab's factorisation and solves of one direction with the current configuration of
 	// sample h (explicit step + Woodbury iterates, eager launches on the main stream): the best of
 	// three runs after one warm-up.
 	double time_direction(SampleHost& h, int dirn) {
@@ -792,16 +805,10 @@ struct Plan : PlanBase {
 		fx_cur = W->facx.as<cx<R>>(); fy_cur = W->facy.as<cx<R>>();
 		lx_cur = W->lscx.as<cx<double>>(); ly_cur = W->lscy.as<cx<double>>();
 		ct_cur = W->coefT.as<cx<R>>();
-		{
-			const SolveCfg& c = scfg[h.index];
-			const int M = dirn == 0 ? (c.xs ? 0 : c.Mx) : c.Mxt;
-			const int lines = (dirn == 0 ? Gm.Ny : Gm.Nx) * 2 * ng;
-			k_fill_steps<<<(lines + 255) / 256, 256, 0, stream>>>(lines, M ? usual_steps(h, dirn, M) : 0, dirn == 0 ? lx_cur : ly_cur);
-			CK(cudaGetLastError());
-		}
 		float best = 1e30f;
 		for(int r = 0; r < 4; r++) {
 			CK(cudaEventRecord(ev[2], stream));
+			rec_factor(h, Gm, ng, dirn, W->coef.as<cx<R>>(), ct_cur, dirn == 0 ? fx_cur : fy_cur, dirn == 0 ? lx_cur : ly_cur);
 			rec_adi(h, Gm, 0, nsl, ng, h.s.n_woodbury, W->coef.as<cx<R>>(), Fp, W->T.as<cx<R>>(), W->T2.as<cx<R>>(), Fp, dirn);
 			CK(cudaEventRecord(ev[3], stream));
 			CK(cudaEventSynchronize(ev[3]));
@@ -1069,14 +1076,38 @@ struct Plan : PlanBase {
 		return ps;
 	}
 
-	// Factorisation for the partitioned x-line solves: one block of 4 lines, or of one line of wpl warps.
-	void rec_factor_part(const char* name, double bytes, const Geom& Gm, int ng, int M, int wpl, const cx<R>* C, cx<R>* fac,
-			size_t plane, cx<double>* lsc) {
-		const int LT = wpl > 1 ? 1 : 4;
-		launch(name, bytes, [&] {
-			k_factor_part<R><<<dim3((unsigned)((Gm.Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32 * wpl, LT), 0, cs>>>(
-				Gm, M, C, fac, plane, lsc);
-		});
+	// Factorisation of the lines of one direction from the coefficient sets C (CT: of the transposed frame).
+	void rec_factor(const SampleHost& h, const Geom& Gm, int ng, int dirn, const cx<R>* C, const cx<R>* CT, cx<R>* fac, cx<double>* lsc) {
+		const SolveCfg& c = scfg[h.index];
+		const char* name = dirn == 0 ? "factor_x" : "factor_y";
+		const double bytes = (double)Gm.N * ng * 2 * (2 + NFAC) * sizeof(cx<R>);  // 4 scalars of the set read per component
+		const size_t plane = dirn == 0 ? c.plane_x : c.plane_y;
+		if(dirn == 0 ? c.Mx && !c.xs : c.Mxt > 0) {
+			// partitioned: one block of 4 lines, or of one line of several warps; the y-lines as x-lines of the
+			// transposed frame
+			const Geom G = dirn == 0 ? Gm : transposed(Gm);
+			const int M = dirn == 0 ? c.Mx : c.Mxt, W = dirn == 0 ? c.WPLx : c.WPLt, LT = W > 1 ? 1 : 4;
+			launch(name, bytes, [&] {
+				k_factor_part<R><<<dim3((unsigned)((G.Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32 * W, LT), 0, cs>>>(
+					G, M, dirn == 0 ? C : CT, fac, plane, lsc);
+			});
+		}
+		else if(dirn == 0) {
+			const int LT = 4;
+			launch(name, bytes, [&] {
+				k_factor_chunked<R, 0><<<dim3((unsigned)((Gm.Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
+					Gm, ng, c.Mx, 32 * c.WPLx, 1, C, fac, plane, lsc);
+			});
+		}
+		else {
+			// 8 chunk warps per 32 columns, 16 when the grid leaves SMs idle
+			const int WF = ((Gm.Nx + 31) / 32) * 2 * ng < nsm && Gm.Ny - 1 >= 256 ? 16 : 8;
+			const size_t smem = (size_t)WF * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>);
+			launch(name, bytes, [&] {
+				k_factor_chunked<R, 1><<<dim3((unsigned)((Gm.Nx + 31) / 32), (unsigned)(ng * 2)), dim3(32, WF), smem, cs>>>(
+					Gm, ng, 0, 32, WF, C, fac, plane, lsc);
+			});
+		}
 	}
 
 	// Slabs [ps.iz, iz_end) of a pass. Setup of slab iz (eps plane iz+1, coefficients,
@@ -1120,27 +1151,7 @@ struct Plan : PlanBase {
 			CK(cudaEventRecord(eCoef, streamB));
 			// factor(iz) overwrites the half the line solves of slab iz-2 used
 			if(iz >= 2) CK(cudaStreamWaitEvent(streamB, eAdi[iz & 1], 0));
-			const double fb = (double)N * ng * 2 * (2 * sc + NFAC * sc);  // 4 scalars of the set read per component
-			// y factorisation: 8 chunk warps per 32 columns, 16 when the grid leaves SMs idle
-			const int LT = 4, WF = ((Nx + 31) / 32) * 2 * ng < nsm && Ny - 1 >= 256 ? 16 : 8;
-			if(scf.Mx && !scf.xs)
-				rec_factor_part("factor_x", fb, Gm, ng, scf.Mx, scf.WPLx, C, fx, scf.plane_x, lx);
-			else launch("factor_x", fb, [&] {
-				k_factor_chunked<R, 0><<<dim3((unsigned)((Ny + LT - 1) / LT), (unsigned)(ng * 2)), dim3(32, LT), 0, cs>>>(
-					Gm, ng, scf.Mx, 32 * scf.WPLx, 1, C, fx, scf.plane_x, lx);
-			});
-			if(scf.Mxt) {
-				// y-lines as x-lines of the transposed frame
-				const Geom Gt = transposed(Gm);
-				rec_factor_part("factor_y", fb, Gt, ng, scf.Mxt, scf.WPLt, CT, fy, scf.plane_y, ly);
-			}
-			else {
-				size_t smem = (size_t)WF * 32 * 8 * sizeof(cx<R>) + 64 * sizeof(cx<R>);
-				launch("factor_y", fb, [&] {
-					k_factor_chunked<R, 1><<<dim3((unsigned)((Nx + 31) / 32), (unsigned)(ng * 2)), dim3(32, WF), smem, cs>>>(
-						Gm, ng, 0, 32, WF, C, fy, scf.plane_y, ly);
-				});
-			}
+			for(int dirn = 0; dirn < 2; dirn++) rec_factor(h, Gm, ng, dirn, C, CT, dirn == 0 ? fx : fy, dirn == 0 ? lx : ly);
 			CK(cudaEventRecord(eFac, streamB));
 			// ---- main stream ----
 			cs = stream;

@@ -26,6 +26,9 @@ __device__ __forceinline__ pr pshfl(pr v, int l) {
 	return pr{__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l), __shfl_sync(0xffffffffu, v.z, l),
 		__shfl_sync(0xffffffffu, v.w, l)};
 }
+// for ring_solve
+__device__ __forceinline__ pr vfma(cx<float> a, pr b, pr c) { return pfma(a, b, c); }
+__device__ __forceinline__ pr vshfl(pr v, int l) { return pshfl(v, l); }
 __device__ __forceinline__ pr at_byte(const pr* f, unsigned o) {
 	return *reinterpret_cast<const pr*>(reinterpret_cast<const char*>(f) + o);
 }
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 		const int K = (int)kb.x;
 		const float base = (float)kb.y;
 		pr* buf = bufs + warp * WS;
-		if(K >= 0) {
+		{
 			pr* vb = buf + lane * PM;
 			pr d, yf;
 			pair_forward<M>(vb, Fc, 32, lane, d, yf);
@@ -239,10 +242,14 @@ __global__ void __launch_bounds__(128, 7) k_solve_xp(Geom G, const cx<float>* __
 					x = pfma(qg, gr, pfma(pg, hl, bg));
 				}
 			}
-			h = pshfl(h, left);
+			if(K >= 0) h = pshfl(h, left);
+			else {
+				const Border<pr, 1> b = part_ring<false, 1, float>(LineThreads{1, 0, 0, lane, lane, last}, If, 32, Border<pr, 1>{{h}, {x}}, (pr*)nullptr);
+				h = b.h[0];
+				x = b.x[0];
+			}
 			pair_backward<M>(vb, Fc, 32, lane, base, h, x);
 		}
-		else if(lane == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, 32, n, base);
 		__syncwarp();
 		// out, or for the transposed outputs the sums into the buffer, where the added field comes with
 		// aligned loads (point n repeats point 0; its entry is free or padding)
@@ -341,9 +348,8 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	__syncthreads();
 	if(ci == 0 && K > 0) atomicMax(&sK, K);
 	pr d, yf;
-	const bool part = live && K >= 0;
 	pr* vb = buf + ci * PM;
-	if(part) pair_forward<M>(vb, Fc, CH, ci, d, yf);
+	if(live) pair_forward<M>(vb, Fc, CH, ci, d, yf);
 	else d = yf = pr{0, 0, 0, 0};
 	const int last = (n - 1) / M;
 	const bool edge_r = lane == 31 || ci == last;
@@ -358,9 +364,16 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 	const cx<float>* If = Fc + (size_t)M * NFAC * CH + ci;
 	const pr yn = next(yf, sG);
 	pr h{0, 0, 0, 0}, x{0, 0, 0, 0}, hl;
-	if(part) {
+	if(live) {
 		h = pfma(If[I_HY * CH], yn, pmul(If[I_HD * CH], d));
 		x = pfma(If[I_GY * CH], yn, pmul(If[I_GD * CH], d));
+	}
+	// a line without Jacobi steps is joined by its own threads, at a barrier of theirs; it only waits in the loop below
+	const bool part = live && K >= 0;
+	if(live && K < 0) {
+		const Border<pr, 1> b = part_ring<true, 1, float>(LineThreads{W, 1 + ln, warp, lane, ci, last}, If, CH, Border<pr, 1>{{h}, {x}}, sG);
+		hl = b.h[0];
+		x = b.x[0];
 	}
 	const pr bh = h, bg = x;
 #pragma unroll 1
@@ -368,12 +381,14 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 		// two buffers in turn: the one written here was last read two barriers ago
 		pr* H = sH + (it & 1) * (W + 1);
 		pr* Gn = sG + ((it + 1) & 1) * W;
-		if(lane == 31) H[warp] = h;
-		if(ci == last) H[W] = h;
-		if(lane == 0) Gn[warp] = x;
+		if(part) {
+			if(lane == 31) H[warp] = h;
+			if(ci == last) H[W] = h;
+			if(lane == 0) Gn[warp] = x;
+		}
 		__syncthreads();
 		const pr up = pshfl(h, (lane + 31) & 31);
-		hl = lane > 0 ? up : H[warp > 0 ? warp - 1 : W];
+		if(part) hl = lane > 0 ? up : H[warp > 0 ? warp - 1 : W];
 		if(it >= Kb) break;
 		const pr gr = next(x, Gn);
 		if(part) {
@@ -382,8 +397,7 @@ __global__ void __maxnreg__(REGS) k_solve_xwp(Geom G, int W, const cx<float>* __
 			x = pfma(qg, gr, pfma(pg, hl, bg));
 		}
 	}
-	if(part) pair_backward<M>(vb, Fc, CH, ci, base, hl, x);
-	else if(live && ci == 0) part_solve_seq<float, M, 2, 2>(reinterpret_cast<cx<float>*>(buf), 1, Fc, CH, n, base);
+	if(live) pair_backward<M>(vb, Fc, CH, ci, base, hl, x);
 	__syncthreads();
 	if(OUT == PO_SAME) {
 		if(!live) return;

@@ -116,9 +116,10 @@ struct SolveShape {
 };
 
 // Elements per factor plane of `lines` partitioned lines (part_line_size in bpm_kernels.cuh: 5 factors
-// per point and 8 interface coefficients per chunk).
+// per point and PART_NIF interface coefficients per chunk).
+constexpr int PART_NIF = 12;
 inline size_t part_plane(int lines, int M, int wpl) {
-	return ((size_t)lines * 32 * wpl * (5 * M + 8) + 4) / 5 + 1;
+	return ((size_t)lines * 32 * wpl * (5 * M + PART_NIF) + 4) / 5 + 1;
 }
 
 inline size_t plane_x_of(const SolveCfg& c, const SolveShape& s) {
