@@ -162,7 +162,7 @@ int nbpm_mask_weights(const char* json_str, const char* mask_formula, const doub
  * inf, mid, sup, rhs and x are device arrays of nlines*L complex values (line-major; entry
  * L-1 of inf/mid/sup/rhs is ignored, x[L-1] receives x[0]). Requires L >= 4. stream is a
  * cudaStream_t (NULL: default stream); the call returns after the solve completed. Lines that do
- * not fit in shared memory (above about 3000 points) need scratch, 5*nlines*(L-1) + 2*nlines complex,
+ * not fit in shared memory (above 2750 unknowns, L - 1) need scratch, 5*nlines*(L-1) + 2*nlines complex,
  * which is allocated stream-ordered. */
 int nbpm_periodic_tridiag_solve(int L, int nlines, const double* inf, const double* mid, const double* sup,
 		const double* rhs, double* x, void* stream);

@@ -15,6 +15,7 @@
 
 #include "../../include/nbpm.h"
 #include "cplx.cuh"
+#include "line_join.cuh"
 
 namespace nbpm {
 
@@ -121,12 +122,14 @@ __global__ void k_pt_solve(int L, int nlines, long long ls_b, const cx<double>* 
 	xx[n] = v;  // duplicate point
 }
 
-// Largest smaller-than-rounding coupling: ln of 2^-57; Jacobi steps beyond which a line is not joined
-// from its chunks.
+// Largest smaller-than-rounding coupling: ln of 2^-57; Jacobi steps beyond which the chunks are joined by
+// ring_solve, which costs about as much; and the change of a border unknown, relative to itself, that one more
+// step may make.
 constexpr double PT_LN_TOL = -39.5;
-constexpr int PT_KMAX = 24;
+constexpr int PT_KMAX = 6;
+constexpr double PT_CHANGE = 1.0 / (1ll << 50);
 
-__device__ __forceinline__ double pt_l1(cx<double> z) { return fabs(z.x) + fabs(z.y); }
+__device__ __forceinline__ double pt_l1(cx<double> z) { return l1abs(z); }
 // 1 / b; clears ok where |b|^2 leaves the range of doubles.
 __device__ __forceinline__ cx<double> pt_recip(cx<double> b, bool& ok) {
 	const double d = b.x * b.x + b.y * b.y;
@@ -142,10 +145,14 @@ __device__ __forceinline__ cx<double> pt_recip(cx<double> b, bool& ok) {
 // unknown before and the one after the chunk, yl, vl and wl those of its last one. Neighbouring chunks
 // then join through their border unknowns: h (a chunk's last) and g (the next one's first) from the two
 // chunks alone, corrected by K Jacobi steps for the chunks beyond, K from the couplings so that what is
-// left is below rounding. A line whose multipliers, join pivots or K are large (not diagonally dominant) is
+// left is below rounding. Lines that would need many steps, and those where one step more changes an unknown
+// noticeably against its own size (right-hand sides of very different magnitudes along the line, NaN and
+// infinities) are joined by ring_solve instead: its scans keep small unknowns beside large ones as exact as
+// a sweep along the line does. A line whose multipliers or join pivots are large (not diagonally dominant) is
 // solved again from its inputs by one thread, as k_pt_factor and k_pt_solve do.
 // Bound: the FP64 pipe, about 58 multiply-adds per point plus the reciprocal. 2048 lines of 512: one
-// thread per line with strided loads took 3.02 ms, this kernel 0.18 ms.
+// thread per line with strided loads took 3.02 ms, this kernel 0.18 ms. 2000 lines of 249 unknowns (last chunk of
+// one point, joined by ring_solve): 1.51 ms, 0.20 ms here (2.12 ms where such lines were swept by one thread).
 __global__ void __launch_bounds__(256) k_pt_part(int L, int M, const cx<double>* __restrict__ inf,
 		const cx<double>* __restrict__ mid, const cx<double>* __restrict__ sup, const cx<double>* rhs, cx<double>* x) {
 	extern __shared__ unsigned char smem_raw[];
@@ -218,17 +225,21 @@ __global__ void __launch_bounds__(256) k_pt_part(int L, int M, const cx<double>*
 		ph = p * vl; pg = pv * vl; qh = pw * wn; qg = p * wn;
 		const float rho = (float)fmax(pt_l1(ph) + pt_l1(qh), pt_l1(pg) + pt_l1(qg));
 		int K = PT_KMAX + 1;
-		if(ok && rho < 1.f) {
+		if(rho < 1.f) {
 			const float lr = logf(rho);  // -inf for rho = 0
 			K = lr < (float)PT_LN_TOL ? 0 : (int)fminf(ceilf((float)PT_LN_TOL / lr) - 1.f, PT_KMAX + 1.f);
 		}
+		if(!ok) K = PT_KMAX + 2;
 		if(K) atomicMax(&sK, K);
 	}
 	__syncthreads();
-	const int K = nchk < 2 ? PT_KMAX + 1 : sK;
-	if(K <= PT_KMAX) {
+	const int K = nchk < 2 ? PT_KMAX + 2 : sK;
+	bool seq = K > PT_KMAX + 1;
+	if(!seq) {
 		const cx<double> bh = h, bg = g;
 		cx<double> hl;
+		bool done = K <= PT_KMAX;
+		if(done)
 		for(int it = 0;; it++) {
 			// two buffers in turn: the one written here was last read two barriers ago
 			cx<double>* H = sH + (it & 1) * T;
@@ -237,18 +248,36 @@ __global__ void __launch_bounds__(256) k_pt_part(int L, int M, const cx<double>*
 			Gb[t] = g;
 			__syncthreads();
 			hl = H[prev];
-			if(it == K) break;
-			const cx<double> gr = Gb[next];
-			h = cfma(qh, gr, cfma(ph, hl, bh));
-			g = cfma(qg, gr, cfma(pg, hl, bg));
+			const cx<double> gr = Gb[next], hn = cfma(qh, gr, cfma(ph, hl, bh)), gn = cfma(qg, gr, cfma(pg, hl, bg));
+			if(it == K) {
+				done = __syncthreads_and(m <= 0 || pt_l1(hn - h) + pt_l1(gn - g) <= PT_CHANGE * fmin(pt_l1(h), pt_l1(g)));
+				break;
+			}
+			h = hn;
+			g = gn;
 		}
-		cx<double> v = g;
-		for(int k = m - 1; k >= 0; k--) {
-			v = cfma(sC[q0 + k], v, sB[q0 + k] * cfma(sA[q0 + k], hl, sD[q0 + k]));
-			sD[q0 + k] = v;
+		if(!done) {
+			const LineThreads lt{T / 32, 0, t / 32, t % 32, t, nchk - 1};
+			RingNode<double> r;
+			if(T > 32) r = ring_factor<true>(lt, ph, pg, qh, qg, sv);
+			else r = ring_factor<false>(lt, ph, pg, qh, qg, sv);
+			seq = !__syncthreads_and(m <= 0 || pt_l1(r.d) <= 4.0);
+			if(!seq) {
+				h = cfma(r.f2, bg, bh);
+				g = r.d * bg;
+				if(T > 32) ring_solve<true, 1, double>(lt, r, &h, &g, &hl, sw);
+				else ring_solve<false, 1, double>(lt, r, &h, &g, &hl, sw);
+			}
+		}
+		if(!seq) {
+			cx<double> v = g;
+			for(int k = m - 1; k >= 0; k--) {
+				v = cfma(sC[q0 + k], v, sB[q0 + k] * cfma(sA[q0 + k], hl, sD[q0 + k]));
+				sD[q0 + k] = v;
+			}
 		}
 	}
-	else {
+	if(seq) {
 		__syncthreads();
 		stage();
 		__syncthreads();
@@ -291,7 +320,7 @@ __global__ void __launch_bounds__(256) k_pt_part(int L, int M, const cx<double>*
 }
 
 // Threads and chunk length of k_pt_part for a line of n unknowns, and its shared memory; false if the line
-// does not fit (about 3000 points). One warp a line as long as several lines share an SM (512 points: 35
+// does not fit (above 2750 unknowns). One warp a line as long as several lines share an SM (512 points: 35
 // KB); more for longer lines, and when the lines are too few to give every SM four warps. Chunks of at
 // least 4 points: shorter ones need more steps to join than they save.
 static bool pt_part_shape(int n, int nlines, int& T, int& M, size_t& smem) {
@@ -299,9 +328,13 @@ static bool pt_part_shape(int n, int nlines, int& T, int& M, size_t& smem) {
 	while(T < 128 && (long long)nlines * (T / 32) < 4 * 152 && n >= 8 * T) T *= 2;
 	M = (n + T - 1) / T;
 	if(M < 4) M = 4;
-	const int nchk = (n + M - 1) / M;
-	smem = ((size_t)4 * nchk * (M | 1) + (size_t)7 * T) * sizeof(cx<double>);
-	return smem <= 200 * 1024;
+	for(int k = 0; k < 2; k++, M++) {
+		const int nchk = (n + M - 1) / M;
+		smem = ((size_t)4 * nchk * (M | 1) + (size_t)7 * T) * sizeof(cx<double>);
+		// an even length is padded to the next odd one, which may fit where it does not
+		if(smem <= 200 * 1024) return true;
+	}
+	return false;
 }
 
 // Whether a call needs the scratch of pt_scratch_elems.
