@@ -41,7 +41,8 @@ static thread_local std::string g_last_error;
 void set_last_error(const std::string& m) { g_last_error = m; }
 
 // Tuned line-solve configurations, per shape key (direction | precision | mesh | slots per
-// wavelength | wavelengths per pass | Woodbury steps | SMs), shared by every plan of the process.
+// wavelength | wavelengths per pass | Woodbury steps | SMs | couplings, and what the other direction is where
+// the choice depends on it), shared by every plan of the process.
 // With NBPM_TUNE_CACHE set to a file name, entries are read from that file when the cache is
 // first used and each new entry is appended to it, so later processes skip the timing runs.
 namespace {
@@ -664,28 +665,40 @@ struct Plan : PlanBase {
 			}
 			if(!zeroed) { zero_workspace(); zeroed = true; }
 			const std::string key = tune_key(h);
+			const size_t semi = forced.find(';');
+			const bool x_forced = !forced.empty() && forced.substr(0, semi) != "auto";
+			const bool y_forced = semi != std::string::npos && forced.substr(semi + 1) != "auto";
 			std::string note;
 			double best_sum = 0;
 			int timed = 0;
 			no_pairs = true;
 			for(int dirn = 0; dirn < 2; dirn++) {
-				if(!forced.empty() && (dirn == 0 ? forced.substr(0, forced.find(';')) != "auto"
-						: (forced.find(';') != std::string::npos && forced.substr(forced.find(';') + 1) != "auto")))
-					continue;
+				if(dirn == 0 ? x_forced : y_forced) continue;
 				const auto& cands = dirn == 0 ? xc : yc;
+				const SolveCfg keep = sc;
+				// y solves in the transposed frame need an x solve that hands the fields over: what fits y depends on
+				// x, which is part of y's key, and x is chosen for a forced y
+				auto fits = [&](const SolveCfg& c) { return dirn == 0 ? !(y_forced && keep.Mxt) || c.x_hands_over() : !c.Mxt || keep.x_hands_over(); };
+				const std::string dkey = dirn == 0 ? "x|" + key + (y_forced ? "|" + keep.ystr() : "") : "y|" + key + "|" + keep.xstr();
 				std::string hit;
-				if(tune_cache_get((dirn == 0 ? "x|" : "y|") + key, hit)) {
+				bool found = false;
+				if(tune_cache_get(dkey, hit))
 					for(auto& c : cands)
-						if((dirn == 0 ? c.xstr() : c.ystr()) == hit) { if(dirn == 0) sc.set_x(c); else sc.set_y(c); }
+						if((dirn == 0 ? c.xstr() : c.ystr()) == hit && fits(c)) {
+							if(dirn == 0) sc.set_x(c);
+							else sc.set_y(c);
+							found = true;
+							break;
+						}
+				if(found) {
 					note += std::string(dirn == 0 ? "x" : "y") + " cached " + hit + "; ";
 					continue;
 				}
-				const SolveCfg keep = sc;
 				double best = 1e300;
 				SolveCfg win = sc;
 				std::string times;
 				for(auto& c : cands) {
-					if(dirn == 1 && c.Mxt && !keep.x_hands_over()) continue;
+					if(!fits(c)) continue;
 					SolveCfg t = keep;
 					if(dirn == 0) t.set_x(c); else t.set_y(c);
 					t.plane_x = pmax;
@@ -698,7 +711,7 @@ struct Plan : PlanBase {
 				}
 				sc = win;
 				const std::string ws = dirn == 0 ? win.xstr() : win.ystr();
-				tune_cache_put((dirn == 0 ? "x|" : "y|") + key, ws);
+				tune_cache_put(dkey, ws);
 				note += std::string(dirn == 0 ? "x" : "y") + " tuned " + ws + " [" + times + "]; ";
 				best_sum += best;
 				timed++;
@@ -735,7 +748,7 @@ struct Plan : PlanBase {
 				sc = sum < best_sum ? win : keep;
 				if(sum < best_sum) {
 					tune_cache_put("x|" + key, win.xstr());
-					tune_cache_put("y|" + key, win.ystr());
+					tune_cache_put("y|" + key + "|" + win.xstr(), win.ystr());
 				}
 				note += "pairs " + std::string(sum < best_sum ? win.str() : "slower") + " [" + times + "]; ";
 			}
