@@ -669,88 +669,42 @@ struct Plan : PlanBase {
 			const bool x_forced = !forced.empty() && forced.substr(0, semi) != "auto";
 			const bool y_forced = semi != std::string::npos && forced.substr(semi + 1) != "auto";
 			std::string note;
-			double best_sum = 0;
-			int timed = 0;
-			no_pairs = true;
-			for(int dirn = 0; dirn < 2; dirn++) {
-				if(dirn == 0 ? x_forced : y_forced) continue;
-				const auto& cands = dirn == 0 ? xc : yc;
-				const SolveCfg keep = sc;
-				// y solves in the transposed frame need an x solve that hands the fields over: what fits y depends on
-				// x, which is part of y's key, and x is chosen for a forced y
-				auto fits = [&](const SolveCfg& c) { return dirn == 0 ? !(y_forced && keep.Mxt) || c.x_hands_over() : !c.Mxt || keep.x_hands_over(); };
-				const std::string dkey = dirn == 0 ? "x|" + key + (y_forced ? "|" + keep.ystr() : "") : "y|" + key + "|" + keep.xstr();
-				std::string hit;
-				bool found = false;
-				if(tune_cache_get(dkey, hit))
-					for(auto& c : cands)
-						if((dirn == 0 ? c.xstr() : c.ystr()) == hit && fits(c)) {
-							if(dirn == 0) sc.set_x(c);
-							else sc.set_y(c);
-							found = true;
-							break;
-						}
-				if(found) {
-					note += std::string(dirn == 0 ? "x" : "y") + " cached " + hit + "; ";
-					continue;
-				}
-				double best = 1e300;
-				SolveCfg win = sc;
-				std::string times;
-				for(auto& c : cands) {
-					if(!fits(c)) continue;
-					SolveCfg t = keep;
-					if(dirn == 0) t.set_x(c); else t.set_y(c);
-					t.plane_x = pmax;
-					sc = t;
-					double ms = time_direction(h, dirn);
-					char b[96];
-					std::snprintf(b, sizeof b, "%s %.3f ms", (dirn == 0 ? c.xstr() : c.ystr()).c_str(), ms);
-					times += (times.empty() ? "" : ", ") + std::string(b);
-					if(ms < best) { best = ms; win = t; }
-				}
-				sc = win;
-				const std::string ws = dirn == 0 ? win.xstr() : win.ystr();
-				tune_cache_put(dkey, ws);
-				note += std::string(dirn == 0 ? "x" : "y") + " tuned " + ws + " [" + times + "]; ";
-				best_sum += best;
-				timed++;
-			}
-			no_pairs = false;
-			// the pair kernels need both directions: their best x and y together against the best of each
-			if(timed == 2 && sizeof(R) == sizeof(float)) {
-				const SolveCfg keep = sc;
-				SolveCfg win = sc;
-				double sum = 0;
-				std::string times;
-				for(int dirn = 0; dirn < 2; dirn++) {
-					const auto& cands = dirn == 0 ? xc : yc;
-					double best = 1e300;
-					for(auto& c : cands) {
-						if(!(dirn == 0 ? c.pair_x() : c.pair_y())) continue;
-						SolveCfg t = win;
-						if(dirn == 0) {
-							t.set_x(c);
-							for(auto& d : yc) if(d.pair_y()) { t.set_y(d); break; }
-						}
-						else t.set_y(c);
-						t.plane_x = pmax;
-						if(!t.pairs()) continue;
-						sc = t;
-						const double ms = time_direction(h, dirn);
-						char b[96];
-						std::snprintf(b, sizeof b, "%s %.3f ms", (dirn == 0 ? c.xstr() : c.ystr()).c_str(), ms);
-						times += (times.empty() ? "" : ", ") + std::string(b);
-						if(ms < best) { best = ms; win = t; }
+			// y solves in the transposed frame need an x solve that hands the fields over: what fits y depends on
+			// x, which is part of y's key, and x is chosen for a forced y
+			const std::string xkey = "x|" + key + (y_forced ? "|" + sc.ystr() : "");
+			auto ykey = [&] { return "y|" + key + "|" + sc.xstr(); };
+			bool x_known = x_forced, y_known = y_forced;
+			std::string hit;
+			if(!x_known && tune_cache_get(xkey, hit))
+				for(auto& c : xc)
+					if(c.xstr() == hit && (!(y_forced && sc.Mxt) || c.x_hands_over())) {
+						sc.set_x(c);
+						x_known = true;
+						note += "x cached " + hit + "; ";
+						break;
 					}
-					sum += best;
+			// y's entry: x and y, x with its choice of pairs
+			if(x_known && !y_known && tune_cache_get(ykey(), hit))
+				for(auto& c : yc) {
+					SolveCfg t = sc;
+					t.set_y(c);
+					for(int k = 0; k < 2 && !y_known; k++) {
+						t.single = k ? !sc.single : sc.single;
+						if(t.str() == hit && (!c.Mxt || t.x_hands_over())) {
+							sc = t;
+							y_known = true;
+							note += "y cached " + c.ystr() + "; ";
+						}
+					}
 				}
-				sc = sum < best_sum ? win : keep;
-				if(sum < best_sum) {
-					tune_cache_put("x|" + key, win.xstr());
-					tune_cache_put("y|" + key + "|" + win.xstr(), win.ystr());
+			if(!x_known || !y_known) {
+				const std::string yk = x_known ? ykey() : std::string();
+				tune(h, sc, x_known, y_known, xc, yc, note);
+				if(!x_known) tune_cache_put(xkey, sc.xstr());
+				if(!y_known) {
+					tune_cache_put(ykey(), sc.str());
+					if(!yk.empty() && yk != ykey()) tune_cache_put(yk, sc.str());
 				}
-				note += "pairs " + std::string(sum < best_sum ? win.str() : "slower") + " [" + times + "]; ";
 			}
 			sc.plane_x = pmax;
 			tune_notes[h.index] = (tune_notes[h.index].empty() ? "" : tune_notes[h.index] + ", ") + note;
@@ -765,6 +719,70 @@ struct Plan : PlanBase {
 			if(!scfg[hp->index].Mxt && L.coefT.p) drop(L.coefT);
 		}
 		select(*S[0]);
+	}
+
+	// Times the directions of sc (the sample's configuration) that are not known, and takes the fastest: first every
+	// candidate on the general kernels, x then y, then, in FP32, the candidates that run on pairs of slots, which need
+	// both directions, against those together. A known direction stays, but for the choice of pairs.
+	void tune(SampleHost& h, SolveCfg& sc, bool x_known, bool y_known, const std::vector<SolveCfg>& xc, const std::vector<SolveCfg>& yc,
+			std::string& note) {
+		const size_t pmax = sc.plane_x;
+		const SolveCfg given = sc;
+		auto best_of = [&](int dirn, const SolveCfg& base, const std::vector<SolveCfg>& cands, bool pairs, SolveCfg& win, std::string& times) {
+			double best = 1e300;
+			for(auto& c : cands) {
+				SolveCfg t = base;
+				if(dirn == 0) t.set_x(c); else t.set_y(c);
+				t.single = !pairs && sizeof(R) == sizeof(float);
+				t.plane_x = pmax;
+				if(t.Mxt && !t.x_hands_over()) continue;
+				if(pairs && !t.pairs()) continue;
+				sc = t;
+				const double ms = time_direction(h, dirn);
+				char b[96];
+				SolveCfg shown = t;
+				shown.single = false;
+				std::snprintf(b, sizeof b, "%s %.3f ms", (dirn == 0 ? shown.xstr() : shown.ystr()).c_str(), ms);
+				times += (times.empty() ? "" : ", ") + std::string(b);
+				if(ms < best) { best = ms; win = t; }
+			}
+			return best;
+		};
+		auto without_twins = [&](const std::vector<SolveCfg>& v) {
+			std::vector<SolveCfg> out;
+			for(auto& c : v) if(!c.single) out.push_back(c);
+			return out;
+		};
+		const std::vector<SolveCfg> xs = x_known ? std::vector<SolveCfg>{given} : without_twins(xc);
+		const std::vector<SolveCfg> ys = y_known ? std::vector<SolveCfg>{given} : yc;
+		SolveCfg win = given;
+		std::string tx, ty;
+		// x before y: without transposed y solves while y is open
+		SolveCfg base = given;
+		if(!y_known) base.Mxt = 0;
+		double sum = best_of(0, base, xs, false, win, tx);
+		if(!y_known) { win.set_y(given); }
+		sum += best_of(1, win, ys, false, win, ty);
+		if(!x_known) { SolveCfg w = win; w.single = false; note += "x tuned " + w.xstr() + " [" + tx + "]; "; }
+		if(!y_known) note += "y tuned " + win.ystr() + " [" + ty + "]; ";
+		if(sizeof(R) == sizeof(float) && !(x_known && given.single)) {
+			// the pair kernels' best x beside any of their y solves, then the best y
+			SolveCfg p = given;
+			for(auto& c : ys) if(c.pair_y()) { p.set_y(c); break; }
+			std::string tp;
+			SolveCfg pw = p;
+			double psum = 1e300;
+			if(p.pair_y()) {
+				psum = best_of(0, p, xs, true, pw, tp);
+				if(psum < 1e300) psum += best_of(1, pw, ys, true, pw, tp);
+			}
+			if(psum < 1e300) note += "pairs " + std::string(psum < sum ? pw.str() : "slower") + " [" + tp + "]; ";
+			if(psum < sum) win = pw;
+			else win.single = win.pair_x() && win.pair_y();  // said only where it matters
+		}
+		else win.single = given.single;
+		win.plane_x = pmax;
+		sc = win;
 	}
 
 	// Wavelengths per pass the tuner times with (and keys on): at most four. Beyond that every
@@ -1546,8 +1564,7 @@ struct Plan : PlanBase {
 	}
 
 	// Whether a sample's slabs run on pairs of slots (FP32).
-	bool no_pairs = false;  // the tuner's timings of the general kernels
-	bool on_pairs(const SampleHost& h) const { return sizeof(R) == sizeof(float) && !no_pairs && scfg[h.index].pairs(); }
+	bool on_pairs(const SampleHost& h) const { return sizeof(R) == sizeof(float) && scfg[h.index].pairs(); }
 
 	// The line solves of a slab on pairs: x frame, then the transposed frame, two Woodbury iterates each.
 	void rec_adi_pairs(SampleHost& h, const Geom& Gm, int nsl, int ng, const cx<R>* C, cx<R>* Fp, cx<R>* Tb, cx<R>* T2b,

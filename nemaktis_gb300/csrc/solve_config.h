@@ -33,6 +33,7 @@ struct SolveCfg {
 	// per line with M-point lane chunks (k_solve_xc). KSx slots per thread.
 	int Mx = 0, KSx = 1, WPLx = 1;
 	bool xs = false;
+	bool single = false;  // FP32: not on pairs of slots, though both directions could be (pairs() below)
 	// y-lines: yq > 0 sequential per column (k_solve_yq, yq slots per thread); ys chunks held in
 	// a scratch field (k_solve_ys, KSy slots); My > 0 32 columns x WY warps of M-row chunks
 	// (k_solve_yc, KSy slots; y1024w: the Woodbury solves with 32 warps of 8-row chunks and 2
@@ -53,7 +54,7 @@ struct SolveCfg {
 		if(WPLx > 1) std::snprintf(b, sizeof b, "xw:M=%d:KS=%d:W=%d", Mx, KSx, WPLx);
 		else if(xs) std::snprintf(b, sizeof b, "xs:M=%d:KS=%d", Mx, KSx);
 		else std::snprintf(b, sizeof b, "xc:M=%d:KS=%d", Mx, KSx);
-		return b;
+		return std::string(b) + (single ? ":single" : "");
 	}
 	std::string ystr() const {
 		char b[64];
@@ -67,7 +68,7 @@ struct SolveCfg {
 		return b;
 	}
 	std::string str() const { return xstr() + ";" + ystr(); }
-	void set_x(const SolveCfg& o) { Mx = o.Mx; KSx = o.KSx; WPLx = o.WPLx; xs = o.xs; }
+	void set_x(const SolveCfg& o) { Mx = o.Mx; KSx = o.KSx; WPLx = o.WPLx; xs = o.xs; single = o.single; }
 	void set_y(const SolveCfg& o) {
 		My = o.My; WY = o.WY; KSy = o.KSy; yq = o.yq; Mt = o.Mt; Mxt = o.Mxt; WPLt = o.WPLt; ys = o.ys;
 		y1024w = o.y1024w;
@@ -76,10 +77,11 @@ struct SolveCfg {
 	// to the transposed frame
 	bool x_hands_over() const { return Mx > 0 && !xs; }
 	// Both directions partitioned with two slots per thread: in FP32 they run on pairs of slots
-	// (pair_kernels.cuh).
+	// (pair_kernels.cuh) unless the x part says ":single", which the tuner adds where pairs are slower (and
+	// FP64, which has no pairs, takes with the same kernels).
 	bool pair_x() const { return x_hands_over() && KSx == 2 && Mx <= 8; }
 	bool pair_y() const { return Mxt > 0 && KSy == 2 && Mxt <= 8; }
-	bool pairs() const { return pair_x() && pair_y(); }
+	bool pairs() const { return !single && pair_x() && pair_y(); }
 };
 
 // Chunk lengths of the partitioned one-warp lines of n unknowns: the shortest with 32 chunks, so that
@@ -174,6 +176,9 @@ inline std::vector<SolveCfg> x_candidates(const SolveShape& s0, bool relaxed = f
 				}
 		}
 	}
+	if(s.fp32 || relaxed)
+		for(size_t i = 0, n = out.size(); i < n; i++)
+			if(out[i].pair_x()) { SolveCfg c = out[i]; c.single = true; out.push_back(c); }
 	if(out.empty()) out.push_back(SolveCfg());
 	for(auto& c : out) finalize(c, s);
 	return out;
