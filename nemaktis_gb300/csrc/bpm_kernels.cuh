@@ -33,10 +33,11 @@ enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
 // is factored by itself. F_A = -l_i (forward recurrence d_i = r_i - l_i d_{i-1}, l_i = a_i/beta_{i-1},
 // 0 at the chunk's first point), F_DB = 1/beta_i - base, F_C = -c_i/beta_i, F_Z = (product of F_C over the
 // points before i) / beta_i, so that the chunk's first unknown is sum_i F_Z d_i, and F_E = what the
-// unknown before the chunk adds to point i before the backward sweep. base is 1 in FP32 on lines of weak coupling,
+// unknown before the chunk adds to point i before the backward sweep. base is 1 on lines of weak coupling,
 // where the difference is rounded to its own, smaller size: in a uniform region every point of every slab repeats
-// the rounding of 1/beta_i, which took 7.7e-8 of the amplitude per slab (64 slabs 256x256: 4.9e-6, 0.8e-6 so; the
-// solves 324 -> 332 us). Else 0.
+// the rounding of 1/beta_i, which took 7.7e-8 of the amplitude per slab in FP32 (64 slabs 256x256: 4.9e-6, 0.8e-6
+// so; the solves 324 -> 332 us; FP64, droplets of 128 and 256 points: errors of 2.7e-14, 1.8 and 1.9e-14 so, 2 % of the
+// step). Else 0.
 // It is in the line scalar lsc[line][0].y.
 enum { F_DB = F_RB, F_Z = F_W, F_E = F_COR };
 // Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
@@ -1135,12 +1136,6 @@ __global__ void __launch_bounds__(256, sizeof(S) == sizeof(double) ? 4 : 5) k_fa
 	const cx<S> one = mk<S>(1, 0), zero = mk<S>(0, 0);
 	// border responses to the unknowns before (v) and after (w) the chunk, and the last 1/beta
 	cx<S> vf = zero, vl = zero, wf = zero, wl = zero, rbl = zero;
-	S base = 0;
-	if(sizeof(S) == sizeof(float) && active) {
-		cx<S> em, ec, en;
-		coef_diag<0>(Cg, c, p0, em, ec, en);
-		base = l1abs(ec) < (S)1 ? 1 : 0;  // |1/beta| > 0.6 then
-	}
 	// 1 / b with one division: the pivots are 1 + O(dz / (k0 n dx^2)), far from the ends of the range
 	auto recip = [](cx<S> b) {
 		const S r = (S)1 / (b.x * b.x + b.y * b.y);
@@ -1148,13 +1143,16 @@ __global__ void __launch_bounds__(256, sizeof(S) == sizeof(double) ? 4 : 5) k_fa
 	};
 	const int i0 = t * M;
 	const bool own = active && i0 < n;
+	// base: lines of weak coupling (|1/beta| > 0.6), by their chunks' first points
+	cx<S> em = zero, ec = zero, en = zero;
+	if(own) coef_diag<0>(Cg, c, p0 + i0, em, ec, en);
+	const bool weak = l1abs(ec) < (S)1;
+	const S base = (CH > 32 ? __syncthreads_and(weak) : __all_sync(0xffffffffu, weak)) ? 1 : 0;
 	if(own) {
 		const int m = min(M, n - i0);
 		cx<S> rb = zero, cprev = zero, ev = zero, cpz = one;
 		for(int k = 0; k < m; k++) {
-			const int i = i0 + k;
-			cx<S> em, ec, en;
-			coef_diag<0>(Cg, c, p0 + i, em, ec, en);
+			if(k) coef_diag<0>(Cg, c, p0 + i0 + k, em, ec, en);
 			const cx<S> a = -em, cs = -en;
 			cx<S> al = zero;  // -l
 			if(k == 0) ev = -a;
@@ -1241,10 +1239,20 @@ __global__ void __launch_bounds__(256, sizeof(S) == sizeof(double) ? 4 : 5) k_fa
 	put(I_HD, hd); put(I_HY, hy); put(I_GD, gd); put(I_GY, gy);
 }
 
-// v / beta from F_DB
-template <typename R>
+// v / beta from F_DB. FP64, whose pipe is the bound, takes a sweep for each base (ONE) and no product with it.
+template <bool B>
+struct Flag {
+	static constexpr bool on = B;
+};
+template <bool ONE, typename R>
 __device__ __forceinline__ cx<R> from_base(cx<R> db, R base, cx<R> v) {
-	return sizeof(R) == sizeof(float) ? cfma(db, v, mk<R>(base * v.x, base * v.y)) : db * v;
+	if(sizeof(R) == sizeof(double)) return ONE ? cfma(db, v, v) : db * v;
+	return cfma(db, v, mk<R>(base * v.x, base * v.y));
+}
+template <typename R, typename F>
+__device__ __forceinline__ void with_base(R base, F sweep) {
+	if(sizeof(R) == sizeof(float) || base != 0) sweep(Flag<true>());
+	else sweep(Flag<false>());
 }
 
 // The node coefficients of a thread's chunk on a line flagged -1 by k_factor_part (If: its interface coefficients, CH
@@ -1471,18 +1479,18 @@ __global__ void __launch_bounds__(128, NBPM_XC_MINB(M * KS)) k_solve_xc(Geom G, 
 			for(int j = 0; j < KS; j++) { h[j] = b.h[j]; x[j] = b.x[j]; }
 		}
 		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
+		with_base(base, [&](auto one) {
 #pragma unroll
-		for(int k = M - 1; k >= 0; k--) {
-			{
+			for(int k = M - 1; k >= 0; k--) {
 				const v4<R> rc = part_rc(Fc, k, 32, lane);
 				const cx<R> db = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, 32, lane);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
-					x[j] = cfma(cc, x[j], cfma(ee, h[j], from_base<R>(db, base, vb[j * PITCH + k])));
+					x[j] = cfma(cc, x[j], cfma(ee, h[j], from_base<decltype(one)::on>(db, base, vb[j * PITCH + k])));
 					vb[j * PITCH + k] = x[j];
 				}
 			}
-		}
+		});
 	}
 	// the explicit-step solves never accumulate; the accumulating ones load the accumulator inputs
 	// of several points before storing any (their latency would otherwise be paid point by point)
@@ -2075,18 +2083,18 @@ __global__ void __launch_bounds__(256) k_solve_xw(Geom G, int slot0, int nch, co
 			}
 		}
 		// backward sweep from the next chunk's first unknown, with the previous chunk's last one
+		with_base(base, [&](auto one) {
 #pragma unroll
-		for(int k = M - 1; k >= 0; k--) {
-			{
+			for(int k = M - 1; k >= 0; k--) {
 				const v4<R> rc = part_rc(Fc, k, CH, ci);
 				const cx<R> db = mk(rc.x, rc.y), cc = mk(rc.z, rc.w), ee = part_e(Fc, k, CH, ci);
 #pragma unroll
 				for(int j = 0; j < KS; j++) {
-					x[j] = cfma(cc, x[j], cfma(ee, hl[j], from_base<R>(db, base, vb[j * PITCH + k])));
+					x[j] = cfma(cc, x[j], cfma(ee, hl[j], from_base<decltype(one)::on>(db, base, vb[j * PITCH + k])));
 					vb[j * PITCH + k] = x[j];
 				}
 			}
-		}
+		});
 	}
 	__syncthreads();
 	// write-out: the accumulator inputs of several points are loaded before any store
