@@ -339,12 +339,13 @@ __global__ void k_screen_filter(cx<R>* F, ScreenParams sp, int g0, const double*
 
 // Which Fourier columns of a (wavelength, q) reach the aperture: |kx / k0 + qx| < NA. Outside, the matrix of every
 // mode of the column is zero: sqrt(q0^2 + q1^2) is not below |q0| in floating point either.
-static __global__ void k_screen_keep(ScreenParams sp, const double* __restrict__ wl, const double* __restrict__ qv,
+static __global__ void k_screen_keep(ScreenParams sp, size_t n, const double* __restrict__ wl, const double* __restrict__ qv,
 		unsigned char* __restrict__ keep) {
-	const int ix = blockIdx.x * blockDim.x + threadIdx.x, gq = blockIdx.y;
-	if(ix >= sp.Nx) return;
+	const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if(t >= n) return;
+	const int ix = (int)(t % sp.Nx), gq = (int)(t / sp.Nx);
 	const double q0 = screen_q(ix, sp.Nx, sp.dx, wl[gq / sp.Nq], qv[2 * (gq % sp.Nq)]);
-	keep[(size_t)gq * sp.Nx + ix] = fabs(q0) < sp.NA;
+	keep[t] = fabs(q0) < sp.NA;
 }
 
 // The y half of the screen filter in one pass, after the row transforms: forward transform of `nc` columns of both
@@ -365,7 +366,8 @@ __global__ void __launch_bounds__(512) k_screen_cols(cx<R>* F, ScreenParams sp, 
 	cx<R>* sB = sA + (size_t)2 * nc * pitch;
 	cx<R>* wp = sB + (size_t)2 * nc * pitch;
 	double* sq = reinterpret_cast<double*>(wp + P.pmax + (P.pmax & 1));  // [n] q1 of the modes, [nc] q0 of the columns
-	const int x0 = blockIdx.x * nc, m = min(nc, Nx - x0), slot = blockIdx.y, gq = slot / 2;
+	// blocks: the column groups of a slot, then the slots (more of them than a grid's y may hold)
+	const int ncg = (Nx + nc - 1) / nc, slot = blockIdx.x / ncg, x0 = (blockIdx.x - slot * ncg) * nc, m = min(nc, Nx - x0), gq = slot / 2;
 	const unsigned char* kp = keep + (size_t)gq * Nx + x0;
 	bool any = false;
 	for(int i = 0; i < m; i++) any |= kp[i] != 0;

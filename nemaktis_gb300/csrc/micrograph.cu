@@ -135,16 +135,17 @@ __global__ void k_focus_filter(long long N, int Nl, int Nq, double NA, double a,
 
 // Which Fourier columns of a (wavelength, q) reach the aperture: (kx + px)^2 < (k0 NA)^2, rounded as in
 // k_objective_table, whose |k+p|^2 is not below (kx + px)^2 then either.
-__global__ void k_focus_keep(int Nx, int Nq, double dx, double NA, const double* __restrict__ wl,
+__global__ void k_focus_keep(size_t n, int Nx, int Nq, double dx, double NA, const double* __restrict__ wl,
 		const double* __restrict__ qv, unsigned char* __restrict__ keep) {
-	const int ix = blockIdx.x * blockDim.x + threadIdx.x, lq = blockIdx.y;
-	if(ix >= Nx) return;
+	const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if(t >= n) return;
+	const int ix = (int)(t % Nx), lq = (int)(t / Nx);
 	double tx = __dsub_rn(fmod(__dadd_rn((double)ix, __dmul_rn(0.5, (double)Nx)), (double)Nx), __dmul_rn(0.5, (double)Nx));
 	double kx = __ddiv_rn(__dmul_rn(__dmul_rn(tx, 2.0), PI_NP), __dmul_rn((double)Nx, dx));
 	double k0 = __ddiv_rn(2.0 * PI_NP, wl[lq / Nq]);
 	double ax = __dadd_rn(kx, __dmul_rn(k0, qv[2 * (lq % Nq)]));
 	double kna = __dmul_rn(k0, NA);
-	keep[(size_t)lq * Nx + ix] = __dmul_rn(ax, ax) < __dmul_rn(kna, kna);
+	keep[t] = __dmul_rn(ax, ax) < __dmul_rn(kna, kna);
 }
 
 // One block transforms `lpb` y-lines (adjacent columns x of one plane (l, q, comp)): forward
@@ -484,7 +485,8 @@ struct Microscope {
 		size_t per_line = 2 * (size_t)(Ny + 1) * sizeof(cx<double>);
 		int lpb = (int)std::max<size_t>(1, std::min<size_t>(16, (smem_limit - fft_smem<double>(py, 0)) / per_line));
 		unsigned char* kp = Nx > 1 ? keep.as<unsigned char>() : nullptr;  // one column: no row transforms
-		if(kp) k_focus_keep<<<dim3((unsigned)((Nx + 127) / 128), (unsigned)(Nl * Nq)), 128, 0, st>>>(Nx, Nq, dx, NA, dwl.as<double>(),
+		const size_t nk = (size_t)Nl * Nq * Nx;
+		if(kp) k_focus_keep<<<(unsigned)((nk + 127) / 128), 128, 0, st>>>(nk, Nx, Nq, dx, NA, dwl.as<double>(),
 			dqv.as<double>(), kp);
 		int nlines = Nl * Nq * 4 * Nx;
 		int blocks = (nlines + lpb - 1) / lpb;

@@ -1238,14 +1238,15 @@ struct Plan : PlanBase {
 				const int Nx = h.s.Nx, Ny = h.s.Ny, gq = h.G * h.Nq;
 				unsigned char* keep = h.keep.template as<unsigned char>();
 				launch("screen_keep", (double)Nx * gq, [&] {
-					k_screen_keep<<<dim3((unsigned)((Nx + 127) / 128), (unsigned)gq), 128, 0, cs>>>(h.sp, h.wl.template as<double>(),
+					const size_t nk = (size_t)Nx * gq;
+					k_screen_keep<<<(unsigned)((nk + 127) / 128), 128, 0, cs>>>(h.sp, nk, h.wl.template as<double>(),
 						h.qv.template as<double>(), keep);
 				});
 				fft2(h, F, nplanes, -1, 1);
 				cx<R>* tw = twiddles(Ny);
 				const int threads = std::min(512, std::max(64, (2 * nc * Ny / 4 + 31) / 32 * 32));
 				launch("screen_cols", (double)N * h.slots * 4 * sc, [&] {
-					k_screen_cols<R><<<dim3((unsigned)((Nx + nc - 1) / nc), (unsigned)h.slots), threads, smem, cs>>>(F, h.sp, P, nc, tw,
+					k_screen_cols<R><<<(unsigned)((size_t)((Nx + nc - 1) / nc) * h.slots), threads, smem, cs>>>(F, h.sp, P, nc, tw,
 						h.wl.template as<double>(), h.nout.template as<double>(), h.qv.template as<double>(), keep);
 				});
 				fft2(h, F, nplanes, +1, 1, keep);
