@@ -22,9 +22,9 @@ struct FftPlan1D {
 	int n;
 	int nst;
 	int radix[FFT_MAX_STAGES];
-	// e / d as umulhi(e, m), m = ceil(2^32 / d) (exact while e * d < 2^32), 0 for d = 1: for d = n, the
+	// e / d as umulhi(e, m), m = ceil(2^32 / d) (exact while e * d < 2^32), 0 for d = 1: for d = the
 	// butterflies per line n / radix and the stage's Ns
-	unsigned m_n, m_nb[FFT_MAX_STAGES], m_ns[FFT_MAX_STAGES];
+	unsigned m_nb[FFT_MAX_STAGES], m_ns[FFT_MAX_STAGES];
 	int pmax;  // entries of the shared DFT table of the largest radix above 8; 0: none, or read from tw
 };
 
@@ -44,7 +44,6 @@ inline bool fft_plan_1d(int n, FftPlan1D& P) {
 		while(n % p == 0) { if(!push(p)) return false; n /= p; }
 	if(n > 1 && !push(n)) return false;
 	auto magic = [](int d) { return d == 1 ? 0u : (unsigned)((0x100000000ull + (unsigned)d - 1) / (unsigned)d); };
-	P.m_n = magic(P.n);
 	P.pmax = 0;
 	int Ns = 1;
 	for(int i = 0; i < P.nst; i++) {
