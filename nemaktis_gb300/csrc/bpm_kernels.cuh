@@ -36,8 +36,8 @@ enum { F_A = 0, F_RB, F_W, F_C, F_COR, NFAC };
 // unknown before the chunk adds to point i before the backward sweep. base is 1 on lines of weak coupling,
 // where the difference is rounded to its own, smaller size: in a uniform region every point of every slab repeats
 // the rounding of 1/beta_i, which took 7.7e-8 of the amplitude per slab in FP32 (64 slabs 256x256: 4.9e-6, 0.8e-6
-// so; the solves 324 -> 332 us; FP64, droplets of 128 and 256 points: errors of 2.7e-14, 1.8 and 1.9e-14 so, 2 % of the
-// step). Else 0.
+// so; the solves 324 -> 332 us; FP64, droplets of 128 and 256 points: errors of 2.7e-14, 1.8 and 1.9e-14 so, for at most
+// 2 % of the step). Else 0.
 // It is in the line scalar lsc[line][0].y.
 enum { F_DB = F_RB, F_Z = F_W, F_E = F_COR };
 // Interface coefficients per chunk of those solves (h the chunk's last unknown, g the next chunk's
@@ -45,7 +45,7 @@ enum { F_DB = F_RB, F_Z = F_W, F_E = F_COR };
 // I_PH, I_PG what the previous chunk's h adds to h and g, I_QH, I_QG what the next chunk's g adds. Lines joined
 // by ring_solve (line_join.cuh) hold the node's coefficients in place of those four and after them, and the right-hand
 // sides' coefficients include f2 and d; the line's closing coefficients are the first four entries of I_X.
-enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, I_ETA, I_KAP, I_TAU, I_X, NIF };
+enum { I_HD = 0, I_HY, I_GD, I_GY, I_PH, I_PG, I_QH, I_QG, I_ETA, I_KAP, I_TAU, I_X, I_UNUSED, NIF };
 enum { I_F = I_PH };  // RN_F .. RN_RHO there, RN_ETA .. RN_TAU from I_ETA on
 static_assert(NIF == PART_NIF, "part_plane");
 // Layout of a line's factors: for each point k of a chunk the vectors {F_A, F_Z} of the CH chunks, then
@@ -366,8 +366,7 @@ static __global__ void k_neff_partial(const double* __restrict__ dir, int fd, co
 }
 
 // ---------------------------------------------------------------------------------------
-// Per-slab operator coefficients (FP64 in FP64 mode; in FP32 mode the phase operator stays
-// FP64 and the stencil entries of mu*R are formed in FP32):
+// Per-slab operator coefficients, in the plan's precision (the phase's argument too):
 //  * phase operator exp(i*a*d) (PhaseEvolutionOperator.cpp:34-63)
 //  * mu*R with R = i*W + (D*S^-1 + S^-1*D)/4, D = D0 + D1*K (ParaxialPrimaryEvolution-
 //    Operator.cpp:212-490), written per stencil entry: S^-1 and K at the column point for
@@ -1117,8 +1116,8 @@ template <bool MULTI, typename S>
 __device__ __noinline__ RingNode<S> part_ring_factor(LineThreads T, cx<S> ph, cx<S> pg, cx<S> qh, cx<S> qg, cx<S>* sh) {
 	return ring_factor<MULTI>(T, ph, pg, qh, qg, sh);
 }
-// Registers: 64 in FP64 and 48 in FP32, what the chunks' sweeps take (102 and 63 with those of ring_factor made a
-// 128x128 FP64 step 4 % slower).
+// Registers: 64 in FP64 and 48 in FP32, what the chunks' sweeps take (without the bound ring_factor's make it 102 and
+// 63: a 128x128x64 FP64 step 8.8 -> 10.0 ms).
 template <typename S>
 __global__ void __launch_bounds__(256, sizeof(S) == sizeof(double) ? 4 : 5) k_factor_part(Geom G, int M, const cx<S>* __restrict__ coef,
 		cx<S>* __restrict__ fac, size_t plane, cx<double>* __restrict__ lsc) {
@@ -1354,7 +1353,7 @@ __device__ __forceinline__ void wait_predecessor() {
 // finishes the line, which goes back out coalesced.
 // Bound: L1 wavefronts (73 %) and load latency (issue active 50 %). Partitioning in place of forward,
 // sum and backward maps joined by shuffle scans: 20 instead of 28 multiply-adds per point and slot, 5
-// instead of 7 factor loads, and no scans (5 shuffle steps each over 3 quantities). 256x256, 16
+// instead of 7 factor loads, and no scans (5 shuffle steps each over 3 quantities) but on strongly coupled lines (part_ring). 256x256, 16
 // wavelengths, 13 q, FP32: Woodbury solves 552 -> 490 us, explicit step 499 -> 476 us; the same mesh
 // with 3 wavelengths in FP64 (bound by the FP64 pipe) 1351 -> 962 and 1540 -> 1162 us. With the real
 // entries of the coefficient set (4 x-taps and 10 with one real number each in place of 14 complex
@@ -1948,7 +1947,7 @@ __global__ void __launch_bounds__(128) k_solve_yq(Geom G, int nch, const cx<R>* 
 
 // x-line solve for long lines: one block of W warps per line, 32*W chunks of M points (the
 // partitioned layout with 32*W chunks), solved as in k_solve_xc; neighbouring chunks in different
-// warps exchange their border unknowns through shared memory (2 + K barriers a line).
+// warps exchange their border unknowns through shared memory (2 + K barriers a line, 6 with part_ring).
 // acc_in2 (may be null): a second accumulator input, acc_out = (acc_in + acc_in2) + x. TOUT: the
 // results go out transposed with the components exchanged ((c, iy, e) -> (1 - c, e, iy) of an
 // Ny x Nx plane), as in k_solve_xc.

@@ -118,8 +118,9 @@ struct SolveShape {
 };
 
 // Elements per factor plane of `lines` partitioned lines (part_line_size in bpm_kernels.cuh: 5 factors
-// per point and PART_NIF interface coefficients per chunk).
-constexpr int PART_NIF = 12;
+// per point and PART_NIF interface coefficients per chunk, one of them unused: with 12, lines of 4-point chunks
+// lie a power of two apart; 64x64x32, 8 x 7 waves, FP32 3.24 ms with 12 and 3.14 with 13, 128x128x64 FP64 9.65 and 9.63).
+constexpr int PART_NIF = 13;
 inline size_t part_plane(int lines, int M, int wpl) {
 	return ((size_t)lines * 32 * wpl * (5 * M + PART_NIF) + 4) / 5 + 1;
 }
