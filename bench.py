@@ -269,13 +269,13 @@ def run_ours(args):
     # dram__bytes_write.sum), scaled to this workload's launch by the slots it processes; the
     # capture and its command are summarised under profiles/.
     PROF = "profiles/solve_xp_koehler_256x256x8_fp32.md"
-    WX = 2 * (309.2e6 + 184.7e6 + 527.5e6 + 189.0e6) / 2  # mean of the two Woodbury launches, x2 slots
-    WY = 2 * (309.1e6 + 184.3e6 + 527.6e6 + 188.7e6) / 2
+    WX = 2 * (310.0e6 + 188.6e6 + 527.8e6 + 198.6e6) / 2  # mean of the two Woodbury launches, x2 slots
+    WY = 2 * (309.8e6 + 188.5e6 + 527.8e6 + 198.8e6) / 2
     TRAFFIC = {("koehler", "fp32", "wood_solve_x"): (WX, PROF),
                ("koehler", "fp32", "wood_solve_y"): (WY, PROF),
-               ("koehler", "fp32", "expl_solve_x"): (2 * (322.1e6 + 185.5e6), PROF),
-               ("koehler", "fp32", "expl_solve_y"): (2 * (321.9e6 + 183.4e6), PROF),
-               ("koehler", "fp32", "shift_fused"): (2 * (242.5e6 + 176.1e6), PROF)}
+               ("koehler", "fp32", "expl_solve_x"): (2 * (322.1e6 + 187.9e6), PROF),
+               ("koehler", "fp32", "expl_solve_y"): (2 * (322.1e6 + 188.1e6), PROF),
+               ("koehler", "fp32", "shift_fused"): (2 * (242.5e6 + 179.2e6), PROF)}
     roof = None
     if prof:
         top = max(prof, key=lambda k: prof[k]["ms"])
@@ -300,7 +300,7 @@ def run_ours(args):
         "metric": "voxel-steps/s FP32-batched vs FP64 plain, 1 GB300, <=1e-4 rel err; p50/p99 latency",
         "value": value, "unit": "voxel-steps/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": dev_ms / args.steps, "higher_is_better": True, "scaling": "weak" if world > 1 else "weak",
-        "vs_baseline": None, "dtype": "complex-f32 (f64 phase argument and Sherman-Morrison scalars)"
+        "vs_baseline": None, "dtype": "complex-f32 (f64 nref, aperture test and host-side index expressions)"
         if prec == "fp32" else "complex-f64",
         "data": "synthetic (seeded director fields, no dataset)",
         "config": {"workload": samples[0]["desc"], "precision": prec, "voxel_steps_per_step": vs,
