@@ -186,8 +186,9 @@ __device__ __forceinline__ void ring_solve(const LineThreads& T, const Node& r, 
 	const bool in = T.ci <= T.last;
 	V *sB = s, *sF = s + KS * W, *sL = sF + KS * W;
 	cx<S>* sA = reinterpret_cast<cx<S>*>(sL + KS);
-	// alpha forward
-	cx<S> A = r.get(RN_F);
+	const cx<S> one = mk<S>(1, 0);
+	// alpha forward; the coefficients of threads past the last chunk may never have been written
+	cx<S> A = in ? r.get(RN_F) : one;
 #pragma unroll 1
 	for(int o = 1; o < 32; o <<= 1) {
 		const cx<S> a = shfl_up_c(A, o);
@@ -226,7 +227,7 @@ __device__ __forceinline__ void ring_solve(const LineThreads& T, const Node& r, 
 		const V up = vshfl(h[j], lane - 1);
 		x[j] = in ? vfma(r.get(RN_B1), lane > 0 ? up : c[j], x[j]) : zero;
 	}
-	A = r.get(RN_B2);
+	A = in ? r.get(RN_B2) : one;
 #pragma unroll 1
 	for(int o = 1; o < 32; o <<= 1) {
 		const cx<S> a = shfl_down_c(A, o);

@@ -663,7 +663,6 @@ struct Plan : PlanBase {
 				sc.plane_x = pmax;
 				continue;
 			}
-			if(!zeroed) { zero_workspace(); zeroed = true; }
 			const std::string key = tune_key(h);
 			const size_t semi = forced.find(';');
 			const bool x_forced = !forced.empty() && forced.substr(0, semi) != "auto";
@@ -698,6 +697,7 @@ struct Plan : PlanBase {
 					}
 				}
 			if(!x_known || !y_known) {
+				if(!zeroed) { zero_workspace(); zeroed = true; }
 				const std::string yk = x_known ? ykey() : std::string();
 				tune(h, sc, x_known, y_known, xc, yc, note);
 				if(!x_known) tune_cache_put(xkey, sc.xstr());
