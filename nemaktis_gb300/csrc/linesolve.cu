@@ -123,10 +123,11 @@ __global__ void k_pt_solve(int L, int nlines, long long ls_b, const cx<double>* 
 }
 
 // Largest smaller-than-rounding coupling: ln of 2^-57; Jacobi steps beyond which the chunks are joined by
-// ring_solve, which costs about as much; and the change of a border unknown, relative to itself, that one more
+// ring_solve, which with its factorisation costs about as much (700 lines of 199 unknowns, 8 steps: 56 us, 83 us
+// joined by ring_solve); and the change of a border unknown, relative to itself, that one more
 // step may make.
 constexpr double PT_LN_TOL = -39.5;
-constexpr int PT_KMAX = 6;
+constexpr int PT_KMAX = 24;
 constexpr double PT_CHANGE = 1.0 / (1ll << 50);
 
 __device__ __forceinline__ double pt_l1(cx<double> z) { return l1abs(z); }
@@ -152,7 +153,7 @@ __device__ __forceinline__ cx<double> pt_recip(cx<double> b, bool& ok) {
 // solved again from its inputs by one thread, as k_pt_factor and k_pt_solve do.
 // Bound: the FP64 pipe, about 58 multiply-adds per point plus the reciprocal. 2048 lines of 512: one
 // thread per line with strided loads took 3.02 ms, this kernel 0.18 ms. 2000 lines of 249 unknowns (last chunk of
-// one point, joined by ring_solve): 1.51 ms, 0.20 ms here (2.12 ms where such lines were swept by one thread).
+// one point, some joined by ring_solve): 1.51 ms, 0.19 ms here (2.12 ms where such lines were swept by one thread).
 __global__ void __launch_bounds__(256) k_pt_part(int L, int M, const cx<double>* __restrict__ inf,
 		const cx<double>* __restrict__ mid, const cx<double>* __restrict__ sup, const cx<double>* rhs, cx<double>* x) {
 	extern __shared__ unsigned char smem_raw[];
